@@ -38,26 +38,47 @@ static_assert(kParams == 5252, "parameter count");
 // 11 log(c_S dt / h_j)
 // d = centroid distance (at least h_j/20), h = longest edge, r_min / r_max =
 // the null test's distance bounds d -/+ (h_i + h_j) (r_min at least h_j/20).
-__device__ void lag_features(float f[kF], const TriGeom& Ti, const TriGeom& Tj, int l, double velP, double velS,
-                             double dt) {
+// The features that depend on the pair only, and what the others need of it.
+struct PairFeat {
+    double d, hj, rmin, rmax;
+    float f[kF];            // 7..10 unset
+};
+
+__device__ __forceinline__ void pair_features(PairFeat& q, const TriGeom& Ti, const TriGeom& Tj, double velS, double dt) {
     const double v0 = Ti.ctr[0] - Tj.ctr[0], v1 = Ti.ctr[1] - Tj.ctr[1], v2 = Ti.ctr[2] - Tj.ctr[2];
     const double hj = Tj.maxL, hi = Ti.maxL;
     const double d = fmax(sqrt(v0 * v0 + v1 * v1 + v2 * v2), 0.05 * hj);
     const double gap = (d - hi - hj) / hj;
-    const double rmin = fmax(d - hi - hj, 0.05 * hj), rmax = d + hi + hj;
+    q.d = d;
+    q.hj = hj;
+    q.rmin = fmax(d - hi - hj, 0.05 * hj);
+    q.rmax = d + hi + hj;
+    q.f[0] = (float)log(d / hj);
+    q.f[1] = (float)log(d / hi);
+    q.f[2] = (float)fmin(fmax(gap, -2.0), 20.0) * 0.1f;
+    q.f[3] = (float)log(hi / hj);
+    q.f[4] = (float)fabs(Ti.n[0] * Tj.n[0] + Ti.n[1] * Tj.n[1] + Ti.n[2] * Tj.n[2]);
+    q.f[5] = (float)(fabs(Tj.n[0] * v0 + Tj.n[1] * v1 + Tj.n[2] * v2) / d);
+    q.f[6] = (float)(fabs(Ti.n[0] * v0 + Ti.n[1] * v1 + Ti.n[2] * v2) / d);
+    q.f[11] = (float)log(velS * dt / hj);
+}
+
+__device__ __forceinline__ void time_features(float f[kF], double d, double hj, double rmin, double rmax, int l,
+                                              double velP, double velS, double dt) {
     const double tP = velP * l * dt, tS = velS * l * dt;
-    f[0] = (float)log(d / hj);
-    f[1] = (float)log(d / hi);
-    f[2] = (float)fmin(fmax(gap, -2.0), 20.0) * 0.1f;
-    f[3] = (float)log(hi / hj);
-    f[4] = (float)fabs(Ti.n[0] * Tj.n[0] + Ti.n[1] * Tj.n[1] + Ti.n[2] * Tj.n[2]);
-    f[5] = (float)(fabs(Tj.n[0] * v0 + Tj.n[1] * v1 + Tj.n[2] * v2) / d);
-    f[6] = (float)(fabs(Ti.n[0] * v0 + Ti.n[1] * v1 + Ti.n[2] * v2) / d);
     f[7] = (float)fmin(0.1 * tP / rmin, 3.0);
     f[8] = (float)fmin(0.1 * tS / rmax, 3.0);
     f[9] = (float)fmin(fmax(0.1 * (tP - d) / hj, -3.0), 3.0);
     f[10] = (float)fmin(fmax(0.1 * (tS - d) / hj, -3.0), 3.0);
-    f[11] = (float)log(velS * dt / hj);
+}
+
+__device__ void lag_features(float f[kF], const TriGeom& Ti, const TriGeom& Tj, int l, double velP, double velS,
+                             double dt) {
+    PairFeat q;
+    pair_features(q, Ti, Tj, velS, dt);
+#pragma unroll
+    for (int k = 0; k < kF; k++) f[k] = q.f[k];
+    time_features(f, q.d, q.hj, q.rmin, q.rmax, l, velP, velS, dt);
 }
 
 // Features of explicit samples (source, field, lag): samples[3 q + 0..2].
@@ -94,29 +115,6 @@ __global__ void labels_kernel(const double* __restrict__ blocks, long long n, do
 }
 
 // ---------------------------------------------------------------------------
-// MLP: forward for one sample (weights in shared memory)
-
-__device__ __forceinline__ void mlp_forward(const float* __restrict__ w, const float x[kF], float h1[kH], float h2[kH],
-                                            float z[kC]) {
-    for (int o = 0; o < kH; o++) {
-        float a = w[kOffB1 + o];
-#pragma unroll
-        for (int k = 0; k < kF; k++) a += w[kOffW1 + o * kF + k] * x[k];
-        h1[o] = fmaxf(a, 0.0f);
-    }
-    for (int o = 0; o < kH; o++) {
-        float a = w[kOffB2 + o];
-        for (int k = 0; k < kH; k++) a += w[kOffW2 + o * kH + k] * h1[k];
-        h2[o] = fmaxf(a, 0.0f);
-    }
-#pragma unroll
-    for (int o = 0; o < kC; o++) {
-        float a = w[kOffB3 + o];
-        for (int k = 0; k < kH; k++) a += w[kOffW3 + o * kH + k] * h2[k];
-        z[o] = a;
-    }
-}
-
 // Mini-batch gradient of the mean cross-entropy.  A block takes kB samples:
 // activations and back-propagated errors are staged in shared memory, each
 // weight gradient entry is a contraction over the block's samples, added to
@@ -247,12 +245,20 @@ __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ g, float*
 // the kinks of the front crossing the field triangle and the outer rule
 // converges only algebraically: those lags take the maximal rule whatever
 // the network says.
-EBEM_DI bool front_sweeps(const TriGeom& Ti, const TriGeom& Tj, int l, double velP, double velS, double dt) {
+EBEM_DI void sweep_window(const TriGeom& Ti, const TriGeom& Tj, double& lo, double& hi) {
     const double v0 = Ti.ctr[0] - Tj.ctr[0], v1 = Ti.ctr[1] - Tj.ctr[1], v2 = Ti.ctr[2] - Tj.ctr[2];
     const double d = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-    const double lo = d - Ti.maxL - Tj.maxL, hi = d + Ti.maxL + Tj.maxL;
+    lo = d - Ti.maxL - Tj.maxL;
+    hi = d + Ti.maxL + Tj.maxL;
+}
+EBEM_DI bool window_swept(double lo, double hi, int l, double velP, double velS, double dt) {
     const double t0 = (l - 1) * dt, t1 = (l + 1) * dt;
     return (velP * t1 >= lo && velP * t0 <= hi) || (velS * t1 >= lo && velS * t0 <= hi);
+}
+EBEM_DI bool front_sweeps(const TriGeom& Ti, const TriGeom& Tj, int l, double velP, double velS, double dt) {
+    double lo, hi;
+    sweep_window(Ti, Tj, lo, hi);
+    return window_swept(lo, hi, l, velP, velS, dt);
 }
 
 __global__ void sweep_flags_kernel(const TriGeom* __restrict__ geo, const int* __restrict__ samples, long long n,
@@ -262,54 +268,221 @@ __global__ void sweep_flags_kernel(const TriGeom* __restrict__ geo, const int* _
     out[q] = front_sweeps(geo[samples[3 * q]], geo[samples[3 * q + 1]], samples[3 * q + 2], velP, velS, dt) ? 1 : 0;
 }
 
+// Two FP32 multiply-adds in one instruction, each rounded as fmaf.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+          "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
+// Classes of two samples.  The hidden layers' weights lie in shared memory
+// input by input (w1[k][o], w2[k][o], 16-byte aligned), so that neighbouring
+// units share an instruction, and both samples share the loads (one sample
+// per thread was bound by them); the first hidden layer in registers, the
+// second eight units at a time and added to the outputs at once.  Every
+// unit's sum runs over its inputs in order.
+__device__ __forceinline__ void mlp_class2(const float* __restrict__ w, const float* __restrict__ w1,
+                                           const float* __restrict__ w2, const float x[2][kF], float threshold, int c[2]) {
+    float2 h1[2][kH / 2];
+#pragma unroll
+    for (int o = 0; o < kH / 2; o++) h1[0][o] = h1[1][o] = reinterpret_cast<const float2*>(w + kOffB1)[o];
+#pragma unroll
+    for (int k = 0; k < kF; k++) {
+#pragma unroll
+        for (int o = 0; o < kH / 4; o++) {
+            const float4 v = reinterpret_cast<const float4*>(w1 + k * kH)[o];
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const float2 xk = make_float2(x[t][k], x[t][k]);
+                h1[t][2 * o] = fma2(make_float2(v.x, v.y), xk, h1[t][2 * o]);
+                h1[t][2 * o + 1] = fma2(make_float2(v.z, v.w), xk, h1[t][2 * o + 1]);
+            }
+        }
+    }
+    float z[2][kC];
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+#pragma unroll
+        for (int o = 0; o < kH / 2; o++) h1[t][o] = make_float2(fmaxf(h1[t][o].x, 0.0f), fmaxf(h1[t][o].y, 0.0f));
+#pragma unroll
+        for (int k = 0; k < kC; k++) z[t][k] = w[kOffB3 + k];
+    }
+#pragma unroll 1
+    for (int o = 0; o < kH; o += 8) {
+        float2 a[2][4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) a[0][r] = a[1][r] = reinterpret_cast<const float2*>(w + kOffB2 + o)[r];
+#pragma unroll
+        for (int k = 0; k < kH; k++) {
+            const float4 v = reinterpret_cast<const float4*>(w2 + k * kH + o)[0];
+            const float4 u = reinterpret_cast<const float4*>(w2 + k * kH + o)[1];
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const float hv = (k & 1) ? h1[t][k / 2].y : h1[t][k / 2].x;
+                const float2 h = make_float2(hv, hv);
+                a[t][0] = fma2(make_float2(v.x, v.y), h, a[t][0]);
+                a[t][1] = fma2(make_float2(v.z, v.w), h, a[t][1]);
+                a[t][2] = fma2(make_float2(u.x, u.y), h, a[t][2]);
+                a[t][3] = fma2(make_float2(u.z, u.w), h, a[t][3]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+#pragma unroll
+            for (int k = 0; k < kC; k++) {
+                const float2 v = *reinterpret_cast<const float2*>(w + kOffW3 + k * kH + o + 2 * r);
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+                    z[t][k] += v.x * fmaxf(a[t][r].x, 0.0f);
+                    z[t][k] += v.y * fmaxf(a[t][r].y, 0.0f);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        float m = z[t][0];
+        int arg = 0;
+#pragma unroll
+        for (int o = 1; o < kC; o++)
+            if (z[t][o] > m) { m = z[t][o]; arg = o; }
+        float den = 0.0f;
+#pragma unroll
+        for (int o = 0; o < kC; o++) den += expf(z[t][o] - m);
+        c[t] = (1.0f / den >= threshold) ? arg : kC - 1;
+    }
+}
+
 // Inference for every non-null (pair, lag) of a mesh: cls[(j N + i) nlag + q]
 // for lag l = lag0 + q.  A lag that a front sweeps takes the maximal rule;
 // any other takes the class of the largest probability, or the maximal rule
 // when that probability is below the threshold; 0 outside the pair's
-// non-null lags (nothing to assemble there).  One thread per pair walks its
-// lags; per-class counts of the non-null lags.
-__global__ void __launch_bounds__(128) infer_kernel(const float* __restrict__ params, const TriGeom* __restrict__ geo,
-                                                    int N, double velP, double velS, double dt, int lag0, int nlag,
-                                                    float threshold, unsigned char* __restrict__ cls,
-                                                    unsigned long long* __restrict__ counts) {
-    __shared__ float w[kParams];
+// non-null lags (nothing to assemble there).  A block walks the lags of 128
+// pairs, one thread each, and queues those that need the network; 256 queued
+// lags are evaluated at a time, two per thread.  (One thread evaluating the
+// lags of its own pair kept its hidden layers in local memory and ran with
+// the lanes whose lag a front sweeps idle: 1024-triangle graded screen, 80
+// lags, 9.8 M lags for the network: 19.2 ms, now 3.5 ms, of which 0.7 ms without
+// the network; the network's multiply-adds alone take 1.4 ms of the FP32 pipes.)  Classes are staged in
+// shared memory (stage bytes, a whole number of lags for all pairs) and
+// written in runs.  Per-class counts of the non-null lags.
+static_assert(kOffW1 % 4 == 0 && kOffW2 % 4 == 0 && kOffB1 % 2 == 0 && kOffB2 % 2 == 0 && kOffW3 % 2 == 0 && kH % 8 == 0,
+              "weights are read as float4 and float2");
+constexpr int kInferPairs = 128, kInferQueue = 3 * kInferPairs;
+__global__ void __launch_bounds__(kInferPairs) infer_kernel(const float* __restrict__ params, const TriGeom* __restrict__ geo,
+                                                            int N, double velP, double velS, double dt, int lag0, int nlag,
+                                                            int stage_lags, float threshold,
+                                                            unsigned char* __restrict__ cls,
+                                                            unsigned long long* __restrict__ counts) {
+    extern __shared__ unsigned char stage[];       // [stage_lags][kInferPairs]
+    __shared__ __align__(16) float w[kParams];
     __shared__ unsigned long long cnt[kC];
-    for (int k = threadIdx.x; k < kParams; k += blockDim.x) w[k] = params[k];
-    if (threadIdx.x < kC) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < (long long)N * N) {
-        const int i = (int)(p % N), j = (int)(p / N);
-        int llo = -1, lhi = -2;
-        pair_band(geo[j], geo[i], velP, velS, dt, lag0, nlag, &llo, &lhi);
-        unsigned char* out = cls + p * nlag;
-        unsigned c_loc[kC] = {0, 0, 0, 0};
-        for (int q = 0; q < nlag; q++) {
-            const int l = lag0 + q;
-            int c = 0;
-            if (llo >= 0 && l >= llo && l <= lhi && front_sweeps(geo[i], geo[j], l, velP, velS, dt)) {
-                c = kC - 1;
-                c_loc[c]++;
-            } else if (llo >= 0 && l >= llo && l <= lhi) {
-                float x[kF], h1[kH], h2[kH], z[kC];
-                lag_features(x, geo[i], geo[j], l, velP, velS, dt);
-                mlp_forward(w, x, h1, h2, z);
-                float m = z[0];
-                int arg = 0;
-                for (int o = 1; o < kC; o++)
-                    if (z[o] > m) { m = z[o]; arg = o; }
-                float den = 0.0f;
-                for (int o = 0; o < kC; o++) den += expf(z[o] - m);
-                c = (1.0f / den >= threshold) ? arg : kC - 1;
-                c_loc[c]++;
-            }
-            out[q] = (unsigned char)c;
-        }
-        for (int o = 0; o < kC; o++)
-            if (c_loc[o]) atomicAdd(&cnt[o], (unsigned long long)c_loc[o]);
+    __shared__ int2 queue[kInferQueue];            // (pair of the block, lag offset)
+    __shared__ int queued;
+    __shared__ float pf[kF][kInferPairs];          // the pairs' features, and their d, h_j, r_min, r_max
+    __shared__ double pd[4][kInferPairs];
+    const int tid = (int)threadIdx.x;
+    // the hidden layers' weights transposed, the rest where the parameters have them
+    for (int k = tid; k < kParams; k += kInferPairs) {
+        const float v = params[k];
+        if (k < kOffB1) w[(k % kF) * kH + k / kF] = v;
+        else if (k >= kOffW2 && k < kOffB2) w[kOffW2 + ((k - kOffW2) % kH) * kH + (k - kOffW2) / kH] = v;
+        else w[k] = v;
     }
+    if (tid < kC) cnt[tid] = 0;
+    if (tid == 0) queued = 0;
+    const long long p0 = (long long)blockIdx.x * kInferPairs, p = p0 + tid, NN = (long long)N * N;
+    const int pairs = (int)min((long long)kInferPairs, NN - p0);
+    int llo = -1, lhi = -2;
+    double lo = 0.0, hi = 0.0;                     // the window that a front sweeps (front_sweeps)
+    if (p < NN) {
+        const TriGeom &Ti = geo[p % N], &Tj = geo[p / N];
+        pair_band(Tj, Ti, velP, velS, dt, lag0, nlag, &llo, &lhi);
+        sweep_window(Ti, Tj, lo, hi);
+        PairFeat q;
+        pair_features(q, Ti, Tj, velS, dt);
+#pragma unroll
+        for (int k = 0; k < kF; k++)
+            if (k < 7 || k > 10) pf[k][tid] = q.f[k];
+        pd[0][tid] = q.d;
+        pd[1][tid] = q.hj;
+        pd[2][tid] = q.rmin;
+        pd[3][tid] = q.rmax;
+    }
+    unsigned c_loc[kC] = {0, 0, 0, 0};
+    for (int q0 = 0; q0 < nlag; q0 += stage_lags) {
+        const int nq = min(stage_lags, nlag - q0);
+        __syncthreads();
+        for (int q = 0; q <= nq; q++) {            // a step past the last lag empties the queue
+            const int l = lag0 + q0 + q;
+            bool ask = false;
+            if (q < nq && p < NN) {
+                int c = 0;
+                if (llo >= 0 && l >= llo && l <= lhi) {
+                    if (window_swept(lo, hi, l, velP, velS, dt)) {
+                        c = kC - 1;
+                        c_loc[kC - 1]++;
+                    } else {
+                        ask = true;
+                    }
+                }
+                stage[q * kInferPairs + tid] = (unsigned char)c;
+            }
+            const unsigned asking = __ballot_sync(0xffffffffu, ask);
+            if (asking) {
+                int at = 0;
+                if ((tid & 31) == 0) at = atomicAdd(&queued, __popc(asking));
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(asking & ((1u << (tid & 31)) - 1u));
+                if (ask) queue[at] = make_int2(tid, q);
+            }
+            __syncthreads();
+            int have = queued;
+            __syncthreads();                       // no one queues before everyone has read
+            // at most 255 left over before a step's 128
+            while (have >= 2 * kInferPairs || (q == nq && have > 0)) {
+                const int n = min(have, 2 * kInferPairs);
+                if (tid < n) {
+                    float x[2][kF];
+                    int c[2];
+                    int2 it[2];
+#pragma unroll
+                    for (int t = 0; t < 2; t++) {
+                        it[t] = queue[min(tid + t * kInferPairs, n - 1)];
+                        const int pr = it[t].x;
+#pragma unroll
+                        for (int k = 0; k < kF; k++) x[t][k] = pf[k][pr];
+                        time_features(x[t], pd[0][pr], pd[1][pr], pd[2][pr], pd[3][pr], lag0 + q0 + it[t].y, velP, velS, dt);
+                    }
+                    mlp_class2(w, w + kOffW1, w + kOffW2, x, threshold, c);
+#pragma unroll
+                    for (int t = 0; t < 2; t++) {
+                        if (tid + t * kInferPairs >= n) continue;
+                        stage[it[t].y * kInferPairs + it[t].x] = (unsigned char)c[t];
+#pragma unroll
+                        for (int o = 0; o < kC; o++) c_loc[o] += (c[t] == o);
+                    }
+                }
+                const int2 rest = queue[2 * kInferPairs + tid];
+                __syncthreads();
+                have -= n;
+                if (tid < have) queue[tid] = rest;
+                if (tid == 0) queued = have;
+                __syncthreads();
+            }
+        }
+        for (int k = tid; k < pairs * nq; k += kInferPairs) {
+            const int pr = k / nq, q = k - pr * nq;
+            cls[(p0 + pr) * nlag + q0 + q] = stage[q * kInferPairs + pr];
+        }
+    }
+#pragma unroll
+    for (int o = 0; o < kC; o++)
+        if (c_loc[o]) atomicAdd(&cnt[o], (unsigned long long)c_loc[o]);
     __syncthreads();
-    if (threadIdx.x < kC && cnt[threadIdx.x]) atomicAdd(counts + threadIdx.x, cnt[threadIdx.x]);
+    if (tid < kC && cnt[tid]) atomicAdd(counts + tid, cnt[tid]);
 }
 
 // ---------------------------------------------------------------------------
@@ -420,8 +593,10 @@ int selector_infer(const float* d_params, const MeshData& m, const PhysParams& P
     cudaError_t e = cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * kC, s);
     const long long NN = (long long)m.nt * m.nt;
     if (e == cudaSuccess) {
-        infer_kernel<<<(unsigned)((NN + 127) / 128), 128, 0, s>>>(d_params, m.d_geo, m.nt, P.velP, P.velS, P.dt, lag0,
-                                                                   nlag, threshold, d_cls, d_cnt);
+        // at most 12 KB of staged classes: with the weights, the queue and the features within the default 48 KB
+        const int stage_lags = std::min(nlag, 96);
+        infer_kernel<<<(unsigned)((NN + kInferPairs - 1) / kInferPairs), kInferPairs, (size_t)stage_lags * kInferPairs, s>>>(
+            d_params, m.d_geo, m.nt, P.velP, P.velS, P.dt, lag0, nlag, stage_lags, threshold, d_cls, d_cnt);
         e = cudaGetLastError();
     }
     unsigned long long hc[kC] = {0, 0, 0, 0};
