@@ -85,7 +85,7 @@ def assemble_sa(dmesh: DeviceMesh, prm: ProblemParams, n_gh: int, lag0: int = 0,
     Returns a tensor ``E`` of shape (nlag, 3N, 3N) with ``E[l][row, col]``
     (a transposed view of the column-major C-ABI buffer), and the number of
     non-null pair-lags when ``count`` is set.  ``prec`` selects FP64 or the
-    FP32-bulk / FP64-inner mixed mode.
+    mixed mode (the same FP64 closed form: see ``EBEM_PREC_MIXED``).
     """
     if nlag is None:
         nlag = num_blocks(dmesh, prm) - lag0

@@ -503,8 +503,7 @@ static int assemble_impl(const ebem_mesh* m, const ebem_problem* p, int n_gh, in
     const bool stage = !dev_out || (EBEM_STAGE_DEVICE_OUTPUT && nsrc >= 16 &&
                                     (size_t)ld * n3 * nlag * sizeof(double) >= ((size_t)1 << 30));
     if (!stage) {
-        rc = launch_sa_assemble(md, P, n_gh, lag0, nlag, src0, nsrc, E, (size_t)ld, lag_elems, accumulate, d_count, s, 0,
-                                prec == EBEM_PREC_MIXED);
+        rc = launch_sa_twopass(md, P, n_gh, lag0, nlag, src0, nsrc, E, (size_t)ld, lag_elems, accumulate, d_count, s);
     } else {
         if (!dev_out && ld != 3LL * nsrc) {
             ws_free(d_count, s);
@@ -560,8 +559,8 @@ static int assemble_impl(const ebem_mesh* m, const ebem_problem* p, int n_gh, in
                 e = cudaMemcpy2DAsync(buf[b], ldb * sizeof(double), hE, (size_t)ld * sizeof(double), ldb * sizeof(double),
                                       cols, cudaMemcpyDefault, s);
             if (e != cudaSuccess) { rc = fail(EBEM_ERR_CUDA, "upload failed"); break; }
-            rc = launch_sa_assemble(md, P, n_gh, lag0, nlag, src0 + r0, nr, buf[b], ldb, ldb * n3, accumulate, d_count,
-                                    s, 0, prec == EBEM_PREC_MIXED);
+            rc = launch_sa_twopass(md, P, n_gh, lag0, nlag, src0 + r0, nr, buf[b], ldb, ldb * n3, accumulate, d_count,
+                                    s);
             if (rc) break;
             e = cudaEventRecord(done[b], s);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, done[b], 0);
@@ -583,8 +582,7 @@ static int assemble_impl(const ebem_mesh* m, const ebem_problem* p, int n_gh, in
         if (rc == EBEM_OK && e != cudaSuccess) rc = fail(EBEM_ERR_CUDA, cudaGetErrorString(e));
         // a device output without room for the staging buffers: written in place
         if (!ok && dev_out && rc == EBEM_OK)
-            rc = launch_sa_assemble(md, P, n_gh, lag0, nlag, src0, nsrc, E, (size_t)ld, lag_elems, accumulate, d_count, s,
-                                    0, prec == EBEM_PREC_MIXED);
+            rc = launch_sa_twopass(md, P, n_gh, lag0, nlag, src0, nsrc, E, (size_t)ld, lag_elems, accumulate, d_count, s);
     }
     if (d_count) {
         unsigned long long c = 0;
@@ -623,7 +621,7 @@ int ebem_assemble_ghc(const ebem_mesh* m, const ebem_problem* p, int n_gh, int n
     if (int rc = launch_ghc_assemble(md, P, n_gh, n_sub, n_sing, lag0, nlag, out.d, n3, n3 * n3, s)) return rc;
     if (sa_diagonal) {
         if (int rc = map_nodes(md, n_gh, s)) return rc;
-        if (int rc = launch_sa_assemble(md, P, n_gh, lag0, nlag, 0, md.nt, out.d, n3, n3 * n3, 0, nullptr, s, 1)) return rc;
+        if (int rc = launch_sa_diagonal(md, P, n_gh, lag0, nlag, out.d, n3, n3 * n3, s)) return rc;
     }
     return out.finish(s);
 }
@@ -698,7 +696,7 @@ int ebem_banded_assemble(const ebem_mesh* m, const ebem_problem* p, int n_gh, in
     ebem_banded* b = new ebem_banded();
     b->device = m->d.device;
     int rc = band_structure(md, P, L, &b->op, s);
-    if (!rc) rc = launch_sa_assemble_banded(md, P, n_gh, L, b->op.Eb, b->op.off, b->op.lo, prec == EBEM_PREC_MIXED, s);
+    if (!rc) rc = launch_sa_assemble_banded(md, P, n_gh, L, b->op.Eb, b->op.off, b->op.lo, s);
     if (!rc && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(EBEM_ERR_CUDA, "banded assembly failed");
     if (rc) {
         band_free(&b->op);
@@ -1081,7 +1079,7 @@ int ebem_assemble_sa_noalloc(const ebem_mesh* m, const ebem_problem* p, int n_gh
 }  // extern "C"
 
 struct ebem_batch {
-    int device = 0, n = 0, n_gh = 0, prec = 0;
+    int device = 0, n = 0, n_gh = 0;
     std::vector<const ebem_mesh*> meshes;
     std::vector<int> nlag;
     BatchInst* h_insts = nullptr;          // pinned host copy of the table
@@ -1113,8 +1111,7 @@ int batch_run_twopass(ebem_batch* b, cudaStream_t s) {
         m.d_nodes = const_cast<NodeW*>(I.nodes);
         m.nodes_rule = b->n_gh;
         const size_t n3 = 3 * (size_t)I.N;
-        if (int rc = launch_sa_twopass(m, b->params[k], b->n_gh, 0, I.nlag, 0, I.N, I.E, n3, n3 * n3, 0, nullptr,
-                                       b->prec == EBEM_PREC_MIXED, s))
+        if (int rc = launch_sa_twopass(m, b->params[k], b->n_gh, 0, I.nlag, 0, I.N, I.E, n3, n3 * n3, 0, nullptr, s))
             return rc;
     }
     return EBEM_OK;
@@ -1122,8 +1119,7 @@ int batch_run_twopass(ebem_batch* b, cudaStream_t s) {
 
 int batch_run_direct(ebem_batch* b, int wpb, int chunk, cudaStream_t s) {
     EBEM_CUDA_TRY(cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long), s));
-    return launch_sa_batch(b->d_insts, b->n, b->total, b->n_gh, b->prec == EBEM_PREC_MIXED, wpb, chunk, b->d_next,
-                           b->device, s);
+    return launch_sa_batch(b->d_insts, b->n, b->total, b->n_gh, wpb, chunk, b->d_next, b->device, s);
 }
 
 // Autotuner: time every (warps per block, pairs per grab) candidate once on the
@@ -1226,7 +1222,6 @@ int ebem_batch_create(const ebem_mesh* const* meshes, const ebem_problem* probs,
     b->device = meshes[0]->d.device;
     b->n = n;
     b->n_gh = n_gh;
-    b->prec = prec;
     DeviceGuard dg(b->device);
     auto bail = [&](int rc) { ebem_batch_destroy(b); return rc; };
     if (cudaMallocHost(&b->h_insts, sizeof(BatchInst) * n) != cudaSuccess ||
@@ -1407,7 +1402,7 @@ int ebem_assemble_sa_selected(const ebem_mesh* m, const ebem_problem* p, const i
     if (lag0 < 0 || nlag < 1) return fail(EBEM_ERR_INVALID, "need lag0 >= 0 and nlag >= 1");
     if (prec != EBEM_PREC_FP64 && prec != EBEM_PREC_MIXED) return fail(EBEM_ERR_INVALID, "unknown precision mode");
     DeviceGuard dg(m->d.device);
-    return assemble_selected(const_cast<MeshData&>(m->d), phys_from(p), rules, nclass, cls, lag0, nlag, E, prec, counts,
+    return assemble_selected(const_cast<MeshData&>(m->d), phys_from(p), rules, nclass, cls, lag0, nlag, E, counts,
                              (cudaStream_t)stream);
 }
 

@@ -121,28 +121,32 @@ PhysParams phys_from(const ebem_problem* p);
 
 // SA assembly of source rows [src0, src0+nsrc) into a device buffer
 // (column-major 3 nsrc x 3N per lag, leading dimension ld, lag stride ld_lag).
-int launch_sa_assemble(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc,
-                       double* d_E, size_t ld, size_t ld_lag, int accumulate, unsigned long long* d_count,
-                       cudaStream_t s, int diag_only = 0, int mixed = 0, const int2* pairs = nullptr,
-                       long long npairs = 0);
-// The same assembly in two passes (sa_twopass.cu): F(t_k) of every (pair,
-// level) into a workspace, then the second difference written column by
-// column.  Dense outputs only (no pair list, no diagonal-only mode).
-// With a class array cls (device, cls[(j N + i) nlag + l - lag0] for field j,
-// source i; src0 = 0, nsrc = N) only the lags of class cls_want are written
-// (and the zeros outside the non-null lags when cls_want is 0), with the
-// outer rule in m.d_nodes (n_gh nodes per triangle, composite or not).
+// The diagonal pairs (i, i) only, added to nothing: their blocks overwrite E.
+int launch_sa_diagonal(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, double* d_E, size_t ld,
+                       size_t ld_lag, cudaStream_t s);
+// Outer rules of the classes of a per-(pair, lag) class array (passed to the
+// kernels by value).
+struct ClassTable {
+    int n = 0;
+    int n_gh[256];                  // nodes per triangle
+    const NodeW* nodes[256];
+};
+// The assembly in two passes (sa_twopass.cu): block records, then the dense
+// output written column by column.  With a class array cls (device, cls[(j N
+// + i) nlag + l - lag0] for field j, source i; src0 = 0, nsrc = N) each lag
+// takes the rule of its class; else the rule in m.d_nodes (n_gh nodes per
+// triangle, composite or not).
 int launch_sa_twopass(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc,
-                     double* d_E, size_t ld, size_t ld_lag, int accumulate, unsigned long long* d_count, int mixed,
-                     cudaStream_t s, const unsigned char* cls = nullptr, int cls_want = -1);
+                      double* d_E, size_t ld, size_t ld_lag, int accumulate, unsigned long long* d_count,
+                      cudaStream_t s, const unsigned char* cls = nullptr, const ClassTable* classes = nullptr);
 // Per-pass device times of the two-pass assembly (ebem_profile_enable / _read).
 void profile_enable(int on);
 void profile_read(double ms[2], long long n[2], int reset);
-// Pass 1 of that assembly by the one-warp-per-pair kernel (sa_assemble.cu):
-// F(t_k) and the non-null lags of the pairs of field columns [j0, j0 + nj).
-int launch_sa_fwarp(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc, int j0,
-                    int nj, int kbase, int KL, double* d_F, int2* d_band, unsigned long long* d_count, int mixed,
-                    cudaStream_t s, const unsigned char* cls = nullptr, int cls_want = -1);
+// Pass 1 of that assembly (sa_assemble.cu): the block records and the
+// non-null lags of the pairs of field columns [j0, j0 + nj).
+int launch_sa_records(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc, int j0,
+                      int nj, double* d_rec, int2* d_band, unsigned long long* d_count, cudaStream_t s,
+                      const unsigned char* cls, const ClassTable* classes);
 // Blocks of explicit (source, field) pairs (int2 list, device) at lags
 // [0, nlag) with the rule in m.d_nodes: out[(p nlag + l) 6 + e], 6 symmetric
 // entries per block, zero outside the pair's non-null lags.
@@ -164,7 +168,7 @@ struct BatchInst {
     long long pair_begin;   // first index of this instance in the concatenated pair space
 };
 // Persistent batched assembly over all instances; d_next must be zero.
-int launch_sa_batch(const BatchInst* d_insts, int ninst, long long total, int n_gh, int mixed, int wpb, int chunk,
+int launch_sa_batch(const BatchInst* d_insts, int ninst, long long total, int n_gh, int wpb, int chunk,
                     unsigned long long* d_next, int device, cudaStream_t s);
 int launch_ghc_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_sub, int n_sing, int lag0, int nlag,
                         double* d_E, size_t ld, size_t ld_lag, cudaStream_t s);
@@ -208,7 +212,7 @@ void band_free(BandOp* op);
 int band_to_dense(const BandOp& op, int lag0, int nlag, double* d_E, cudaStream_t s);
 int band_march(const BandOp& op, const double* d_rhs, int nT, double* d_phi, cudaStream_t s);
 int launch_sa_assemble_banded(const MeshData& m, const PhysParams& P, int n_gh, int L, double* d_Eb,
-                              const long long* d_boff, const int* d_blo, int mixed, cudaStream_t s);
+                              const long long* d_boff, const int* d_blo, cudaStream_t s);
 int lu_plan_create(const double* dA, int n, cudaStream_t s, LuPlan* plan, bool pooled = false, bool cholesky = false);
 int lu_plan_solve(LuPlan* plan, double* db, int nrhs, cudaStream_t s);
 void lu_plan_destroy(LuPlan* plan);
@@ -277,7 +281,7 @@ int selector_train(float* d_params, const float* d_feats, const int* d_labels, l
 int selector_infer(const float* d_params, const MeshData& m, const PhysParams& P, float threshold, int lag0, int nlag,
                    unsigned char* d_cls, long long* h_counts, cudaStream_t s);
 int assemble_selected(MeshData& m, const PhysParams& P, const int* h_rules, int nclass, const unsigned char* d_cls,
-                      int lag0, int nlag, double* d_E, int prec, long long* h_counts, cudaStream_t s);
+                      int lag0, int nlag, double* d_E, long long* h_counts, cudaStream_t s);
 void selector_init(float* h_params, unsigned long long seed);
 
 }  // namespace ebem

@@ -13,29 +13,18 @@
 //   children         SA/calcoloMatrice/BEMenerg_coreSA_calcIntgInt_fieldTriangle.m:13-84
 //
 // Work decomposition (B200 design, not the reference's): one warp per
-// (source i, field j) pair walks the pair's time levels t_k = k dt once, in
-// increasing order, with the lanes on the children of the outer nodes
-// (sa_warp.cuh; level_pair below).  F(t_k), the combined kernel integral at
-// one instant, depends on k only, so each level is evaluated once and
-// E_l = F_{l+1} - 2 F_l + F_{l-1} is formed from three levels (the
-// reference evaluates every instant three times, once per lag that uses
-// it).  Dense outputs store the levels and write the blocks in a second,
-// coalesced pass (sa_twopass.cu); the other modes write the blocks directly.
-// A thread-per-pair kernel (sa_assemble_kernel) remains for builds with
-// EBEM_SA_KERNEL=1.
+// (source i, field j) pair.  F(t_k), the combined kernel integral at one
+// instant, depends on k only, so each level is evaluated once and E_l =
+// F_{l+1} - 2 F_l + F_{l-1} is formed from three levels (the reference
+// evaluates every instant three times, once per lag that uses it).  Dense
+// outputs store the levels and write the blocks in a second, coalesced pass
+// (sa_twopass.cu); the other modes write the blocks directly.
 #include "ebem_internal.h"
 
 #include <algorithm>
 #include <mutex>
-#include "sa_pair.cuh"
-#include "sa_warp.cuh"
-
-#ifndef EBEM_SA_KERNEL
-#define EBEM_SA_KERNEL 0    // 0: the warp-per-pair level kernel, 1: thread per pair
-#endif
-#ifndef EBEM_SA_TWOPASS
-#define EBEM_SA_TWOPASS 1   // 1: dense assemblies store F(t_k) and emit the blocks in a second pass (sa_twopass.cu)
-#endif
+#include <type_traits>
+#include "sa_front.cuh"
 
 namespace ebem {
 
@@ -183,113 +172,48 @@ int map_nodes_composite(MeshData& m, int n_gh, int n_sub, cudaStream_t s) {
 // assembly
 
 struct SAArgs {
-    const TriGeom* geo;
-    const NodeW* nodes;
-    int N, n_gh;
-    double velP, velS, dt, c4pirho;
-    int lag0, nlag;
-    int src0, nsrc;         // source rows [src0, src0 + nsrc) of the panel
-    int diag_only;          // 1: only the diagonal pairs (i, i), i in the panel
-    double* E;
-    size_t ld;              // leading dimension (>= 3 nsrc)
-    size_t ld_lag;          // doubles between consecutive lags
-    int accumulate;
-    unsigned long long* count;
-    const int2* pairs;      // optional explicit (source, field) list (npairs entries)
-    long long npairs;
+    const TriGeom* geo = nullptr;
+    const NodeW* nodes = nullptr;
+    int N = 0, n_gh = 0;
+    double velP = 0, velS = 0, dt = 0, ic4 = 0;   // ic4 = 1 / (4 pi rho)
+    int lag0 = 0, nlag = 0;
+    int src0 = 0, nsrc = 0; // source rows [src0, src0 + nsrc) of the panel
+    int j0 = 0, nj = 0;     // field columns [j0, j0 + nj)
+    int diag_only = 0;      // 1: only the diagonal pairs (i, i), i in the panel
+    const int2* pairs = nullptr;   // optional explicit (source, field) list (npairs entries)
+    long long npairs = 0;
+    unsigned long long* count = nullptr;
+    // dense output, column-major 3 nsrc x 3N per lag
+    double* E = nullptr;
+    size_t ld = 0;          // leading dimension (>= 3 nsrc)
+    size_t ld_lag = 0;      // doubles between consecutive lags
+    int accumulate = 0;
+    int zeros_written = 0;  // the buffer is zeroed already: only the band's blocks are written
     // banded output (instead of E): pair p = (i - src0) N + j owns the blocks
     // [boff[p], boff[p+1]) of Eb, one per lag of its band starting at blo[p],
     // 6 symmetric entries (11,12,13,22,23,33) each
     double* Eb = nullptr;
     const long long* boff = nullptr;
     const int* blo = nullptr;
-    // level output (instead of E): field columns [j0, j0 + nj) of the panel;
-    // F(t_k) of pair (i, j) at Fout[(((j - j0) KL + k - kbase) nsrc + i - src0) 6 + e]
-    // for every level it needs, its non-null lags (llo, lhi) at band[(j - j0) nsrc + i - src0]
-    double* Fout = nullptr;
+    // block records (instead of E), written at the non-null lags only: the 6
+    // entries of lag l of pair (i, j) at Lout[(((j - j0) nlag + l - lag0) nsrc
+    // + i - src0) 6], of pair p of a list at Lout[(p nlag + l - lag0) 6]; the
+    // non-null lags (llo, lhi) at band[(j - j0) nsrc + i - src0] when asked for
+    double* Lout = nullptr;
     int2* band = nullptr;
-    int j0 = 0, nj = 0, kbase = 0, KL = 0;
-    // level output restricted to one class of a per-(pair, lag) class array:
-    // cls[(j N + i) nlag + l - lag0] (fields j, sources i); only the levels
-    // that lags of class cls_want use are computed, only those lags counted
+    // classes of a per-(pair, lag) class array: cls[(j N + i) nlag + l - lag0]
     const unsigned char* cls = nullptr;
-    int cls_want = -1;
-    // direct dense output into a buffer already zeroed: only the band's blocks are written
-    int zeros_written = 0;
+    // derived (sa_args_derive)
+    double k1 = 0, ks = 0, icP = 0, icS = 0;   // 1 / c_P^2, 1 / c_S^2, 1 / (c_P dt), 1 / (c_S dt)
 };
 
-__device__ __forceinline__ void store_block(const SAArgs& A, int q, int i, int j, const double b[6]) {
-    // symmetric entries (11,12,13,22,23,33) -> column-major 3x3 at (3(i - src0), 3j)
-    const size_t n3 = A.ld;
-    double* base = A.E + (size_t)q * A.ld_lag + (3 * (size_t)j) * n3 + 3 * (size_t)(i - A.src0);
-    const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};   // (r, c) column-major -> sym index
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            double v = b[map[3 * c + r]];
-            if (A.accumulate) base[c * n3 + r] += v;
-            else base[c * n3 + r] = v;
-        }
-}
+constexpr int kGroupNodes = 10;  // outer nodes per group: 30 children on 32 lanes
 
-__global__ void __launch_bounds__(128) sa_assemble_kernel(SAArgs A) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long NN = A.diag_only ? (long long)A.nsrc : (long long)A.nsrc * A.N;
-    const bool valid = p < NN;
-    const int i = valid ? A.src0 + (int)(p % A.nsrc) : A.src0;   // source (row block)
-    const int j = A.diag_only ? i : (valid ? (int)(p / A.nsrc) : 0);   // field (column block)
-    const TriGeom& F = A.geo[j];
-    const TriGeom& Sg = A.geo[i];
-    double v0 = F.ctr[0] - Sg.ctr[0], v1 = F.ctr[1] - Sg.ctr[1], v2 = F.ctr[2] - Sg.ctr[2];
-    double d = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-    double distMin = d - F.maxL - Sg.maxL;
-    double distMax = d + F.maxL + Sg.maxL;
-    // contiguous range of non-null lags inside [lag0, lag0 + nlag)
-    int llo = -1, lhi = -2;
-    for (int q = 0; q < A.nlag; q++) {
-        int l = A.lag0 + q;
-        if (lag_nonnull(l, A.velP, A.velS, A.dt, distMin, distMax)) {
-            if (llo < 0) llo = l;
-            lhi = l;
-        }
-    }
-    if (A.count) {
-        unsigned cnt = (valid && llo >= 0) ? (unsigned)(lhi - llo + 1) : 0u;
-        unsigned tot = __reduce_add_sync(0xffffffffu, cnt);
-        if ((threadIdx.x & 31) == 0 && tot) atomicAdd(A.count, (unsigned long long)tot);
-    }
-    if (!valid) return;
-    const double zero[6] = {0, 0, 0, 0, 0, 0};
-    if (llo < 0) {
-        if (!A.accumulate)
-            for (int q = 0; q < A.nlag; q++) store_block(A, q, i, j, zero);
-        return;
-    }
-    if (!A.accumulate) {
-        for (int l = A.lag0; l < llo; l++) store_block(A, l - A.lag0, i, j, zero);
-        for (int l = lhi + 1; l < A.lag0 + A.nlag; l++) store_block(A, l - A.lag0, i, j, zero);
-    }
-    const int klo = max(1, llo - 1), khi = lhi + 1;
-    // sliding window F_{k-2}, F_{k-1}, F_k; F_k = 0 for k <= 0
-    double Fm2[6] = {0, 0, 0, 0, 0, 0}, Fm1[6] = {0, 0, 0, 0, 0, 0}, Fk[6];
-    const double c4 = A.c4pirho;
-    for (int k = klo; k <= khi; k++) {
-        level_value(Fk, k, A.velP, A.velS, A.dt, F, A.nodes + (size_t)i * A.n_gh, A.n_gh);
-        const int l = k - 1;                     // lag completed by F_k
-        if (l >= llo && l <= lhi) {
-            double b[6];
-#pragma unroll
-            for (int e = 0; e < 6; e++) {
-                double prev = (l - 1 >= 1) ? Fm2[e] : 0.0;
-                double v = ((Fk[e] + (-2.0) * Fm1[e]) + prev) / c4;
-                b[e] = (fabs(v) < 1.0e-14) ? 0.0 : v;
-            }
-            store_block(A, l - A.lag0, i, j, b);
-        }
-#pragma unroll
-        for (int e = 0; e < 6; e++) { Fm2[e] = Fm1[e]; Fm1[e] = Fk[e]; }
-    }
+EBEM_HDI void sa_args_derive(SAArgs& A) {
+    A.k1 = 1.0 / (A.velP * A.velP);
+    A.ks = 1.0 / (A.velS * A.velS);
+    A.icP = 1.0 / (A.velP * A.dt);
+    A.icS = 1.0 / (A.velS * A.dt);
 }
 
 __device__ __forceinline__ void store_entry(const SAArgs& A, int q, int i, int j, int e, double v) {
@@ -302,70 +226,131 @@ __device__ __forceinline__ void store_entry(const SAArgs& A, int q, int i, int j
 
 
 // ---------------------------------------------------------------------------
-// Level pass of the two-pass assembly, outer nodes in groups.
+// Level kernel: F(t_k) of one (source, field) pair per warp, from the closed
+// form of sa_front.cuh.
 //
-// One warp per (source, field) pair walks the pair's time levels with the
-// schedule of sa_warp.cuh (lane = child of one outer node; per level the
-// per-child decision phase, the whole-range moments, the warp-wide list of
-// Gauss-Legendre nodes and one warp reduction), for the children of at most
-// 10 outer nodes at a time, so composite outer rules of any size
-// (GaussHammerComposite.m) run group after group with each group's per-level
-// sums added in shared memory.  After the levels of a chunk, one lane per
-// level forms F(t_k) (the rotation to global axes) and stores it for the
-// emission pass.  With a per-(pair, lag) class array only the levels used by
-// lags of the wanted class are walked.
+// * Lane = child of an outer node: level-independent data of the child
+//   (fields in shared memory, one column per child) and the two level ranges
+//   of each front, [kA, kN): from the first level at which the front meets
+//   the side to the first at which it has passed the node's whole triangle.
+// * Item = (level, front, child) with the level in that range: the children's
+//   ranges become two bit masks per level (ballots), the masks' population
+//   counts number the items level by level, and the 32 lanes take 32 items
+//   at a time whatever their level, front or child, all on one path
+//   (front_item).  On the sphere of 1280 triangles a pair has some 130
+//   items, where the lanes of one level's children would be a third busy.
+// * The items' seven values go through shared memory into per-level sums,
+//   lane = (level, entry), always in item order: a level's sum does not
+//   depend on where the 32-item rounds fall, so any lag window or row panel
+//   gives the same bits.
+// * Lane = level: the nodes a front has passed wholly add a + t^2 b, summed
+//   over the node's children beforehand; nodes that project inside the field
+//   triangle add V(rho) x (angle); then the rotation to global axes.
+// Outer rules with more than 10 nodes run in equal groups of at most 10; levels
+// in chunks of 32.
 //
-// Two alternative schedules were measured and not kept.  Compacted (child,
-// level) items, 32 per round, each lane on its own item: sphere of 1280
-// triangles 224 ms per step against 186 ms (ncu: 9 % fewer warp
-// instructions, but more instruction-fetch stalls, the items of a round
-// taking more distinct branches than the children of one level).  Groups
-// of 10 consecutive outer nodes of up to three pairs of one field column
-// (30 lanes busy instead of 21 with the 7-node rule, per-pair level sums):
-// 165.9 ms against 167.2 ms with the 7-node rule, 104.7 against 135.4 ms
-// with the 3-node rule; the children of different pairs take more distinct
-// branches per pass than those of one pair, which cancels most of the lanes
-// gained, and the results then depend on how pairs fall into groups (a
-// source-row sub-panel no longer reproduces the full assembly bit for bit).
+// Bound: FP64 issue (an item's two logarithms, two arctangents, two square
+// roots and one division, sa_math.cuh).  Sphere of 320 triangles, L = 40,
+// GH7 (ncu): issue active 57 %, FP64 pipe 40 %, stalls per issued
+// instruction 1.8 on fixed latencies and 0.3 on instruction fetch.  Per
+// assembly, against the kernel that integrated the edge pieces by
+// Gauss-Legendre and decided each child's pieces at each level (lane = child,
+// FP64 pipe 22 %, 3 to 4 stalls on instruction fetch): sphere of 1280
+// triangles 159.4 -> 10.8 ms, of 320 12.8 -> 0.93 ms, prism of 252 with GH12
+// 8.9 -> 0.69 ms.  On the way (1280 triangles): closed form with the library's
+// functions out of line 24.6 ms, inlined 29.4; sa_math.cuh, one division per
+// evaluation and 32-bit pair indices 13.0; blocks as records that stay in L2
+// (sa_twopass.cu) 11.1; the level masks by a bit transpose 10.8.  The IEEE
+// divisions of the second difference alone cost 2.0 ms (their slow path's
+// code), hence ic4.  Launch shape: 8 warps, 2 blocks per SM (128 registers);
+// 4 x 4 13.3 against 13.0 ms, 4 x 3 13.5, 16 x 1 13.2, 12 x 1 13.1.
+constexpr int kLevelChunk = 32;  // levels per chunk: one lane per level
+constexpr int kSlots = 3 * kGroupNodes;
 
-// Levels per chunk (per-level sums in shared memory).  24 rather than 48:
-// the 4 warps' sums take 5.4 KB less shared memory per block, which leaves
-// the 3 blocks per SM a larger L1 for the kernel's stack and loads (sphere
-// N=1280, L=40: 163.5 -> 160.2 ms per step, two A/B rounds on one box; 16
-// levels gave 163.2 ms: the chunks' set-up then costs what L1 gains).
-#ifndef EBEM_LEVEL_KC
-#define EBEM_LEVEL_KC 24
-#endif
 #ifndef EBEM_LEVEL_WPB
-#define EBEM_LEVEL_WPB 4
+#define EBEM_LEVEL_WPB 8
 #endif
 #ifndef EBEM_LEVEL_MINB
-#define EBEM_LEVEL_MINB 3
+#define EBEM_LEVEL_MINB 2
 #endif
-#ifndef EBEM_LEVEL_SKIP_IDLE
-#define EBEM_LEVEL_SKIP_IDLE 1   // 1: levels at which no child works skip the decision and node phases
-#endif
-constexpr int kGroupNodes = 10;  // outer nodes per group: 30 children on 32 lanes
 
 struct LevelShared {
-    WarpShared<1> W;
-    double acc[7][EBEM_LEVEL_KC];
-    double carry[2][6];          // direct output: F of the two levels before the chunk
+    double f[FC_N * kSlots];                 // children, field-major
+    double full[kGroupNodes][14];            // a, b of the node's whole triangle (plane frame, weighted)
+    double ang[kGroupNodes][6];              // its angle moments around the node
+    double zeta[kGroupNodes], zs[kGroupNodes], dmin[kGroupNodes];
+    double res[32][7];                       // the round's items
+    double acc[kLevelChunk][7];              // per-level sums
+    unsigned long long mask[kLevelChunk];    // items of a level: P children, S children << 32
+    double carry[2][6];                      // direct output: F of the two levels before the chunk
+    int kP[kGroupNodes], kS[kGroupNodes];    // first level at which the front has passed the whole triangle
+    int off[kLevelChunk + 1];                // first item of each level
 };
 
-// Whether level k is used by a lag of the wanted class (lags k-1, k, k+1 of
-// the pair's non-null range [llo, lhi]).
-EBEM_DI bool level_wanted(const SAArgs& A, const unsigned char* cls, int k, int llo, int lhi) {
-    if (!cls) return true;
+// Position of the n-th set bit (n counted from 0) of m.
+EBEM_DI int nth_bit(unsigned m, int n) {
+    int pos = 0;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) {
+        const int c = __popc(m & ((1u << h) - 1u));
+        if (n >= c) {
+            n -= c;
+            pos += h;
+            m >>= h;
+        }
+    }
+    return pos;
+}
+
+// pair_band by a warp, one lag per lane.
+EBEM_DI void pair_band_warp(const TriGeom& F, const TriGeom& S, double velP, double velS, double dt, int lag0, int nlag,
+                            int lane, int* llo, int* lhi) {
+    const double v0 = F.ctr[0] - S.ctr[0], v1 = F.ctr[1] - S.ctr[1], v2 = F.ctr[2] - S.ctr[2];
+    const double d = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
+    const double distMin = d - F.maxL - S.maxL;
+    const double distMax = d + F.maxL + S.maxL;
+    *llo = -1;
+    *lhi = -2;
+    for (int q0 = 0; q0 < nlag; q0 += 32) {
+        const int l = lag0 + q0 + lane;
+        const unsigned on = __ballot_sync(0xffffffffu, q0 + lane < nlag && lag_nonnull(l, velP, velS, dt, distMin, distMax));
+        if (on) {
+            if (*llo < 0) *llo = lag0 + q0 + __ffs(on) - 1;
+            *lhi = lag0 + q0 + 31 - __clz(on);
+        }
+    }
+}
+
+// Bits [max(lo, 0), min(hi, 32)).
+EBEM_DI unsigned level_bits(int lo, int hi) {
+    lo = max(lo, 0);
+    hi = min(hi, 32);
+    return hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
+}
+
+// 32 x 32 bit transpose over a warp: bit k of lane i becomes bit i of lane k.
+EBEM_DI unsigned transpose32(unsigned x, int lane) {
+    unsigned m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1, m ^= m << j) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
+    }
+    return x;
+}
+
+EBEM_DI double shfl3_sum(double v, int lane) {
+    return v + __shfl_sync(0xffffffffu, v, lane + 1) + __shfl_sync(0xffffffffu, v, lane + 2);
+}
+
+// Whether level k is used by a lag of class c (lags k-1, k, k+1 of the pair's
+// non-null range [llo, lhi]).
+EBEM_DI bool level_wanted(const SAArgs& A, const unsigned char* cls, int c, int k, int llo, int lhi) {
     for (int l = max(k - 1, llo); l <= min(k + 1, lhi); l++)
-        if (cls[l - A.lag0] == A.cls_want) return true;
+        if (cls[l - A.lag0] == c) return true;
     return false;
 }
 
-// Pair p of the launch: (source i, field j); its record in A.band and its
-// levels in A.Fout (record rec, level k at (rec + (k - kbase) kstride) 6):
-// field columns of a panel (rec = (j - j0) KL nsrc + i - src0, kstride =
-// nsrc) or an explicit pair list (rec = p KL, kstride = 1).
 // The dynamic shared memory opt-in of a kernel, before every launch that is
 // not being captured: it belongs to the context, which a caller may have
 // reset since the last call; a captured launch relies on the uncaptured one
@@ -378,15 +363,20 @@ static int opt_in_smem(K kernel, size_t smem, cudaStream_t s) {
     return EBEM_OK;
 }
 
-template <bool MIXED>
-__device__ __forceinline__ void level_pair(const SAArgs& A, LevelShared& Ls, const double* glx, const double* glw,
-                                           long long p, int i, int j, int lane, unsigned long long& my_count) {
-    WarpShared<1>& W = Ls.W;
+// Pair p of the launch: (source i, field j).  With classes (CLS) the pair's
+// levels are walked once for each class its lags have, with that class's
+// rule.
+// Output of a launch: dense blocks, the banded layout, or block records.
+enum : int { OUT_DENSE, OUT_BANDED, OUT_RECORDS };
+
+template <int OUT, bool CLS>
+__device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T, LevelShared& Ls, long long p, int i, int j,
+                                           int lane, unsigned long long& my_count) {
     const TriGeom& F = A.geo[j];
     const TriGeom& Sg = A.geo[i];
     int llo = -1, lhi = -2;
     long long bbase = 0;
-    if (A.Eb) {
+    if (OUT == OUT_BANDED) {
         // banded output: the band comes from the structure pass, so writes stay in the pair's blocks
         const long long pb = (long long)(i - A.src0) * A.N + j;
         bbase = A.boff[pb];
@@ -396,348 +386,339 @@ __device__ __forceinline__ void level_pair(const SAArgs& A, LevelShared& Ls, con
             lhi = llo + nb - 1;
         }
     } else {
-        pair_band(F, Sg, A.velP, A.velS, A.dt, A.lag0, A.nlag, &llo, &lhi);
+        pair_band_warp(F, Sg, A.velP, A.velS, A.dt, A.lag0, A.nlag, lane, &llo, &lhi);
     }
-    const long long brec = A.pairs ? p : (long long)(j - A.j0) * A.nsrc + (i - A.src0);
-    const long long frec = A.pairs ? p * A.KL : (long long)(j - A.j0) * A.KL * A.nsrc + (i - A.src0);
-    const long long kstride = A.pairs ? 1 : A.nsrc;
-    if (A.band && lane == 0) A.band[brec] = make_int2(llo, lhi);
+    if (OUT == OUT_RECORDS && A.band && lane == 0)
+        A.band[(long long)(j - A.j0) * A.nsrc + (i - A.src0)] = make_int2(llo, lhi);
     // direct dense output: the zeros of the window's lags outside the band
-    const bool dense = !A.Fout && !A.Eb;
-    if (dense && !A.accumulate && !A.zeros_written) {
+    if (OUT == OUT_DENSE && !A.accumulate && !A.zeros_written) {
         for (int idx = lane; idx < A.nlag * 9; idx += 32) {
             const int q = idx / 9, e = idx - 9 * q, l = A.lag0 + q;
             if (llo < 0 || l < llo || l > lhi) store_entry(A, q, i, j, e, 0.0);
         }
     }
     if (llo < 0) return;
-    if (!A.Fout && lane < 12) (&Ls.carry[0][0])[lane] = 0.0;
-    const unsigned char* cls = A.cls ? A.cls + ((long long)j * A.N + i) * A.nlag : nullptr;
-    if (cls) {
-        int n = 0;
-        for (int l = llo; l <= lhi; l++) n += (cls[l - A.lag0] == A.cls_want);
-        if (lane == 0) my_count += (unsigned long long)n;
-        if (n == 0) return;
-    } else if (lane == 0) {
-        my_count += (unsigned long long)(lhi - llo + 1);
+    if (lane == 0) my_count += (unsigned long long)(lhi - llo + 1);
+    const long long rec = A.pairs ? p * A.nlag : (long long)(j - A.j0) * A.nlag * A.nsrc + (i - A.src0);
+    const long long rstride = A.pairs ? 1 : A.nsrc;
+    const unsigned char* cls = CLS ? A.cls + ((long long)j * A.N + i) * A.nlag : nullptr;
+    const double k1 = A.k1, ks = A.ks;
+    int klo = max(1, llo - 1), khi = lhi + 1;
+    const int ncls = CLS ? T->n : 1;
+    unsigned present = 1u;                     // classes of the pair's lags, class 31 and above in bit 31
+    if (CLS) {
+        present = 0u;
+        for (int l = llo + lane; l <= lhi; l += 32) present |= 1u << min((int)cls[l - A.lag0], 31);
+        present = __reduce_or_sync(0xffffffffu, present);
     }
-    const double vp2 = A.velP * A.velP, vs2 = A.velS * A.velS, den = vp2 * vs2;
-    const double k1 = 1.0 / vp2, k5 = (vp2 + vs2) / den, k6 = (vp2 - vs2) / den;
-    const int ngroups = (A.n_gh + kGroupNodes - 1) / kGroupNodes;
-    const int klo = max(1, llo - 1), khi = lhi + 1;
-    const int slot = lane;
-    LaneChild Cu;
-    bool hasmom = false, is_stat = false;
-    for (int kc0 = klo; kc0 <= khi; kc0 += EBEM_LEVEL_KC) {
-        const int kc1 = min(khi, kc0 + EBEM_LEVEL_KC - 1), nk = kc1 - kc0 + 1;
-        for (int x = lane; x < 7 * EBEM_LEVEL_KC; x += 32) (&Ls.acc[0][0])[x] = 0.0;
-        for (int grp = 0; grp < ngroups; grp++) {
-            const int g0 = kGroupNodes * grp, gn = min(kGroupNodes, A.n_gh - g0);
-            if (ngroups > 1 || kc0 == klo) {
-                // children of outer nodes [g0, g0 + gn): slot = 3 (g - g0) + child
-                __syncwarp();
-                Cu.live = false;
-                Cu.zeta = 0.0; Cu.sigma = 0.0; Cu.dMIN = 0.0; Cu.w = 0.0;
-                hasmom = false;
-                is_stat = false;
-                const int g = g0 + slot / 3, c = slot - 3 * (slot / 3);
-                if (slot < 3 * gn) {
-                    NodeW sp = A.nodes[(size_t)i * A.n_gh + g];
-                    NodeGeo G;
-                    node_geo(G, sp, F);
-                    Cu.zeta = G.zeta;
-                    Cu.sigma = G.sigma;
-                    Cu.dMIN = G.dMIN;
-                    Cu.w = sp.w;
-                    if (node_child_e(Cu.g, G, c)) {
-                        Cu.live = true;
-                        m_sincos(Cu.g.gamma, &Cu.sg, &Cu.cg);
-                    }
-                }
-                if (Cu.live) {
-                    const ChildE& gg = Cu.g;
-                    LevelCtx L0;
-                    L0.k5 = k5;
-                    L0.k6 = k6;
-                    const W4 w0 = origin_weights(Cu.zeta, L0);
-                    W.w0[0][slot] = w0.sc;
-                    W.w0[1][slot] = w0.in;
-                    W.w0[2][slot] = w0.mx;
-                    W.w0[3][slot] = w0.zz;
-                    W.amax[slot] = gg.amax;
-                    W.F[slot] = gg.F;
-                    W.cbp[slot] = gg.cb * gg.ct + gg.sb * gg.st;     // cos(beta - theta_V1)
-                    W.sbp[slot] = gg.sb * gg.ct - gg.cb * gg.st;     // sin(beta - theta_V1)
-                    W.zeta[slot] = Cu.zeta;
-                    W.zs[slot] = Cu.zeta * Cu.sigma;
-                    W.scale[slot] = Cu.w * gg.sgnC;
-                    if (MIXED) {
-                        W.Ff[slot] = (float)W.F[slot];
-                        W.cbpf[slot] = (float)W.cbp[slot];
-                        W.sbpf[slot] = (float)W.sbp[slot];
-                        W.zetaf[slot] = (float)W.zeta[slot];
-                        W.zsf[slot] = (float)W.zs[slot];
-                        W.scalef[slot] = (float)W.scale[slot];
-                    }
+    for (int ic = 0; ic < ncls; ic++) {
+        const NodeW* nodes = A.nodes;
+        int n_gh = A.n_gh;
+        if (CLS) {
+            if (!((present >> min(ic, 31)) & 1u)) continue;
+            // the class's first and last lag bound its levels
+            int first = -1, last = -1;
+            for (int l0 = llo; l0 <= lhi; l0 += 32) {
+                const unsigned on = __ballot_sync(0xffffffffu, l0 + lane <= lhi && cls[min(l0 + lane, lhi) - A.lag0] == ic);
+                if (on) {
+                    if (first < 0) first = l0 + __ffs(on) - 1;
+                    last = l0 + 31 - __clz(on);
                 }
             }
-            __syncwarp();
-            for (int k = kc0; k <= kc1; k++) {
-                if (!level_wanted(A, cls, k, llo, lhi)) continue;
-                const double t = k * A.dt;
-                LevelCtx L;
-                L.t2 = t * t;
-                L.RP = A.velP * t;
-                L.RS = A.velS * t;
-                L.k1 = k1;
-                L.k5 = k5;
-                L.k6 = k6;
-                double S = 0.0, T[6] = {0, 0, 0, 0, 0, 0};
-                Piece pc[3];
-                int np = 0, nsubs[3], ngs[3];
-                double hs[3];
-                int nn = 0;
-                // decision phase (per child)
-                int type = T_NONE;
-                double rhoP = -1.0, rhoS = -1.0;
-                if (Cu.live && !is_stat) type = classify(Cu.zeta, L.RP, L.RS, Cu.dMIN, rhoP, rhoS);
-                // no child at work at this level (about half the levels of a pair's
-                // band: the null test's distance bounds are conservative): F is the
-                // sum of the static children, zero when there are none
-                if (EBEM_LEVEL_SKIP_IDLE && __ballot_sync(0xffffffffu, type != T_NONE) == 0u) {
-                    if (__ballot_sync(0xffffffffu, is_stat) != 0u) {
-                        double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                        if (is_stat) {
-#pragma unroll
-                            for (int e = 0; e < 7; e++) v[e] = W.sv[e][slot];
-                        }
-                        const double tot = warp_reduce_scatter8(v, lane);
-                        const int e = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-                        if ((lane & 3) == 0 && e < 7) Ls.acc[e][k - kc0] += tot;
-                    }
-                    continue;
-                }
-                AccE Ac = {0, 0, 0, 0, 0, 0, 0};
-                int full = 0;
-                if (type != T_NONE) {
-                    W4 w0;
-                    w0.sc = W.w0[0][slot];
-                    w0.in = W.w0[1][slot];
-                    w0.mx = W.w0[2][slot];
-                    w0.zz = W.w0[3][slot];
-                    child_decide(Ac, pc, np, full, Cu, L, rhoP, rhoS, type, w0, W.amax[slot]);
-                }
-                // whole-range moments, computed by the whole warp once per child
-                const bool need = full && !hasmom;
-                unsigned mm = __ballot_sync(0xffffffffu, need);
-                while (mm) {
-                    const int b = __ffs(mm) - 1;
-                    mm &= mm - 1;
-                    const double Fb = __shfl_sync(0xffffffffu, Cu.g.F, b), cbb = __shfl_sync(0xffffffffu, Cu.g.cb, b);
-                    const double sbb = __shfl_sync(0xffffffffu, Cu.g.sb, b), zb = __shfl_sync(0xffffffffu, Cu.zeta, b);
-                    const double s1b = __shfl_sync(0xffffffffu, Cu.g.s1, b), s0b = __shfl_sync(0xffffffffu, Cu.g.s0, b);
-                    double m[16];
-                    moment_share(m, Fb, cbb, sbb, zb, s1b, s0b, lane, glx, glw);
-                    m[14] = 0.0;
-                    m[15] = 0.0;
-                    const double tot = warp_reduce_scatter16(m, lane);
-                    const int e = scatter16_index(lane);
-                    if (!(lane & 1) && e < 14) W.mom[e][b] = tot;
-                }
-                __syncwarp();
-                if (need) hasmom = true;
-                const double zs = Cu.zeta * Cu.sigma;
-                if (full & 1) apply_moments(Ac, W, slot, true, L, zs);
-                if (full & 2) apply_moments(Ac, W, slot, false, L, zs);
-                if (type != T_NONE) {
-                    double Sc = 0.0, Tc[6] = {0, 0, 0, 0, 0, 0};
-                    child_to_plane(Sc, Tc, Ac, Cu.g, Cu.w * Cu.g.sgnC);
-                    S += Sc;
-#pragma unroll
-                    for (int e = 0; e < 6; e++) T[e] += Tc[e];
-                    // inside the S front with its whole edge (only the full S piece):
-                    // level-independent from now on (the fronts only grow)
-                    if (type == T_SP_SP && full == 2 && np == 0) {
-                        W.sv[0][slot] = Sc;
-#pragma unroll
-                        for (int e = 0; e < 6; e++) W.sv[1 + e][slot] = Tc[e];
-                        is_stat = true;
-                    }
-                } else if (is_stat) {
-                    S += W.sv[0][slot];
-#pragma unroll
-                    for (int e = 0; e < 6; e++) T[e] += W.sv[1 + e][slot];
-                }
-#pragma unroll
-                for (int q = 0; q < 3; q++) {
-                    nsubs[q] = 0;
-                    ngs[q] = 10;
-                    hs[q] = 0.0;
-                    if (q < np) {
-                        double len = pc[q].shi - pc[q].slo;
-                        int ns = (int)ceil(len * (1.0 / EBEM_EDGE_H));
-                        ns = max(1, min(ns, 4096));
-                        // nodes per sub-piece: 6 up to length 1/4, 8 up to 1/2 (gl6_x)
-                        if (EBEM_GL_ADAPT && ns == 1) ngs[q] = len <= 0.25 ? 6 : (len <= 0.5 ? 8 : 10);
-                        nsubs[q] = ns;
-                        hs[q] = len / ns;
-                        nn += ngs[q] * ns;
-                    }
-                }
-                // partial edge pieces of all children -> per-warp list
-                int totp, totn;
-                int pb = warp_excl_scan(np, lane, totp);
-                int o = warp_excl_scan(nn, lane, totn);
-#pragma unroll
-                for (int q = 0; q < 3; q++) {
-                    if (q < np) {
-                        W.slo[pb] = pc[q].slo;
-                        W.h[pb] = hs[q];
-                        W.off[pb] = o;
-                        W.who[pb] = slot | (pc[q].pterm ? 64 : 0) | (((ngs[q] - 6) >> 1) << 7);
-                        o += ngs[q] * nsubs[q];
-                        pb++;
-                    }
-                }
-                if (lane == 31) W.off[totp] = totn;
-                __syncwarp();
-                // all lanes: Gauss-Legendre nodes of the list, plane frame
-                int pp = 0;
-                if (MIXED) {
-                    float Sf = 0.0f, Tf[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-                    const float fk1 = (float)L.k1, ft2 = (float)L.t2, fk5 = (float)L.k5, fk6 = (float)L.k6;
-                    for (int idx = lane; idx < totn; idx += 32) {
-                        while (idx >= W.off[pp + 1]) pp++;
-                        const int who = W.who[pp], cl = who & 63, code = who >> 7;
-                        const int u = idx - W.off[pp], sub = code == 2 ? u / 10 : 0;
-                        const int q = u - (6 + 2 * code) * sub + (code == 0 ? 0 : (code == 1 ? 6 : 14));
-                        const double h = W.h[pp];
-                        const double s = W.slo[pp] + (sub + 0.5) * h + 0.5 * h * glx[q];
-                        edge_node_f32(Sf, Tf, s, (float)(0.5 * h * glw[q]), W.Ff[cl], W.cbpf[cl], W.sbpf[cl],
-                                      W.zetaf[cl], W.zsf[cl], W.scalef[cl], (who & 64) != 0, fk1, ft2, fk5, fk6);
-                    }
-                    S += (double)Sf;
-#pragma unroll
-                    for (int e = 0; e < 6; e++) T[e] += (double)Tf[e];
-                    totn = 0;    // the FP64 loop below has nothing left to do
-                }
-                for (int idx = lane; idx < totn; idx += 32) {
-                    while (idx >= W.off[pp + 1]) pp++;
-                    const int who = W.who[pp], cl = who & 63, code = who >> 7;
-                    const int u = idx - W.off[pp], sub = code == 2 ? u / 10 : 0;
-                    const int q = u - (6 + 2 * code) * sub + (code == 0 ? 0 : (code == 1 ? 6 : 14));
-                    const double h = W.h[pp];
-                    const double s = W.slo[pp] + (sub + 0.5) * h + 0.5 * h * glx[q];
-                    double sech, th;
-                    Rad v;
-                    edge_point(s, W.F[cl], W.zeta[cl], sech, th, v);
-                    const double cbq = W.cbp[cl], sbq = W.sbp[cl];
-                    const double cq = th * cbq + sech * sbq, sq = sech * cbq - th * sbq;
-                    W4 w = weigh(v, (who & 64) != 0, L);
-                    const double f = 0.5 * h * glw[q] * sech * W.scale[cl];
-                    const double fin = f * w.in, fmx = -W.zs[cl] * f * w.mx;
-                    S += f * w.sc;
-                    T[0] += fin * cq * cq;
-                    T[1] += fin * sq * cq;
-                    T[2] += fin * sq * sq;
-                    T[3] += fmx * cq;
-                    T[4] += fmx * sq;
-                    T[5] += f * w.zz;
-                }
-                __syncwarp();
-                // warp sums; lane scatter8_lane(e) holds entry e (S, T11, T12, T22, T13, T23, T33)
-                double v[8] = {S, T[0], T[1], T[2], T[3], T[4], T[5], 0.0};
-                const double tot = warp_reduce_scatter8(v, lane);
-                const int e = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-                if ((lane & 3) == 0 && e < 7) Ls.acc[e][k - kc0] += tot;
-            }
-            __syncwarp();
-        }
-        // F(t_k) = (S I + C^T M C) / 2 in global axes, one lane per level
-        for (int kl = lane; kl < nk; kl += 32) {
-            const int k = kc0 + kl;
-            if (!level_wanted(A, cls, k, llo, lhi)) continue;
-            const double S = Ls.acc[0][kl];
-            double T[6];
-#pragma unroll
-            for (int e = 0; e < 6; e++) T[e] = Ls.acc[1 + e][kl];
-            double M[3][3] = {{T[0], T[1], T[3]}, {T[1], T[2], T[4]}, {T[3], T[4], T[5]}};
-            const double* Cm = F.C;
-            double MC[3][3];
-#pragma unroll
-            for (int r = 0; r < 3; r++)
-#pragma unroll
-                for (int cc = 0; cc < 3; cc++)
-                    MC[r][cc] = M[r][0] * Cm[cc] + M[r][1] * Cm[3 + cc] + M[r][2] * Cm[6 + cc];
-            double Rm[3][3];
-#pragma unroll
-            for (int r = 0; r < 3; r++)
-#pragma unroll
-                for (int cc = r; cc < 3; cc++)
-                    Rm[r][cc] = Cm[r] * MC[0][cc] + Cm[3 + r] * MC[1][cc] + Cm[6 + r] * MC[2][cc];
-            const double Fk[6] = {0.5 * (S + Rm[0][0]), 0.5 * Rm[0][1], 0.5 * Rm[0][2],
-                                  0.5 * (S + Rm[1][1]), 0.5 * Rm[1][2], 0.5 * (S + Rm[2][2])};
-            if (A.Fout) {
-                double2* dst = reinterpret_cast<double2*>(A.Fout + (frec + (k - A.kbase) * kstride) * 6);
-                dst[0] = make_double2(Fk[0], Fk[1]);
-                dst[1] = make_double2(Fk[2], Fk[3]);
-                dst[2] = make_double2(Fk[4], Fk[5]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 6; e++) Ls.acc[e][kl] = Fk[e];     // this lane's level only
-            }
+            if (first < 0) continue;
+            klo = max(1, first - 1);
+            khi = last + 1;
+            nodes = T->nodes[ic];
+            n_gh = T->n_gh[ic];
         }
         __syncwarp();
-        if (!A.Fout) {
-            // direct output: E_l = (F_{l+1} - 2 F_l + F_{l-1}) / (4 pi rho) for the
-            // lags l = k - 1 completed by the chunk's levels k, clean-up |x| < 1e-14
+        if (lane < 12) (&Ls.carry[0][0])[lane] = 0.0;
+        const int ngroups = (n_gh + kGroupNodes - 1) / kGroupNodes, gsize = (n_gh + ngroups - 1) / ngroups;
+        const FrontView view{Ls.f + (lane < kSlots ? lane : 0), kSlots};
+        // this lane's child: level ranges of its items, zeta; circ: nodes with an angle (bit 3 g)
+        int kaP = 0, knP = 0, kaS = 0, knS = 0;
+        double zeta = 0.0;
+        bool work = false;
+        unsigned circ = 0;
+        for (int kc0 = klo; kc0 <= khi; kc0 += kLevelChunk) {
+            const int nk = min(khi - kc0 + 1, kLevelChunk);
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < 7; e++) Ls.acc[lane][e] = 0.0;
+            const bool wanted = lane < nk && (!CLS || level_wanted(A, cls, ic, kc0 + lane, llo, lhi));
+            for (int grp = 0; grp < ngroups; grp++) {
+                const int g0 = gsize * grp, gn = min(gsize, n_gh - g0);
+                if (ngroups > 1 || kc0 == klo) {
+                    __syncwarp();
+                    FrontSide s;
+                    NodeGeo G;
+                    bool live = false;
+                    double w = 0.0, all = 0.0, tau = 0.0;
+                    const int g = lane / 3, c = lane - 3 * g;
+                    const bool child = g < gn;
+                    G.zeta = G.sigma = G.dMIN = 0.0;
+                    G.inside = false;
+                    if (child) {
+                        const NodeW sp = nodes[(size_t)i * n_gh + g0 + g];
+                        node_project(G, sp, F);
+                        live = front_side(s, G, c);
+                        w = sp.w;
+                    }
+                    zeta = G.zeta;
+                    const double z2 = G.zeta * G.zeta;
+                    if (live) {
+                        const double F2 = s.F * s.F + 1.0e-6;
+                        const bool foot = s.x1 >= 0 && s.x2 < 0;
+                        all = fmax(fmax(s.R1s, s.R2s), F2);
+                        tau = foot ? F2 : fmax(F2, fmin(s.R1s, s.R2s));
+                    }
+                    // the whole triangle is passed when every live child is
+                    const int b3 = 3 * g;
+                    const double a1 = __shfl_sync(0xffffffffu, all, b3), a2 = __shfl_sync(0xffffffffu, all, b3 + 1);
+                    const double a3 = __shfl_sync(0xffffffffu, all, (b3 + 2) & 31);
+                    all = q_sqrt(fmax(a1, fmax(a2, a3)) + z2);
+                    tau = q_sqrt(tau + z2);
+                    kaP = live ? front_level(tau, A.icP, khi + 1) : khi + 1;
+                    kaS = live ? front_level(tau, A.icS, khi + 1) : khi + 1;
+                    knP = front_level(all, A.icP, khi + 1);
+                    knS = front_level(all, A.icS, khi + 1);
+                    // a node can have an angle only inside the triangle or next to a skipped child
+                    const bool maybe = child && (G.inside || !live);
+                    if (maybe && !G.inside) G.dMIN = edge_distance(G.tri);
+                    const int k0 = maybe ? front_level(q_sqrt(G.dMIN * G.dMIN + z2), A.icP, khi + 1) : kaP;
+                    work = __ballot_sync(0xffffffffu, child && min(k0, kaP) <= khi) != 0u;
+                    if (work) {
+                        if (live) front_fields(Ls.f + lane, kSlots, s, G.zeta, G.sigma, w * s.sgnC);
+                        // angle of the triangle around the node
+                        double ag[6] = {0, 0, 0, 0, 0, 0};
+                        const bool some = __ballot_sync(0xffffffffu, maybe) != 0u;
+                        circ = 0;
+                        if (some) {
+                            if (live) front_angles(ag, view);
+                            double a0 = live ? s.sgnC * ag[0] : 0.0;
+                            a0 = shfl3_sum(a0, lane);
+                            circ = __ballot_sync(0xffffffffu, child && c == 0 && fabs(a0) > 1.0e-12);
+                            // d_min of the node is known to the lanes that asked for it
+                            if (maybe) Ls.dmin[g] = G.dMIN;
+                            if (circ) {
+                                double T[7] = {0, 0, 0, 0, 0, 0, 0};
+                                if (live) {
+                                    const double h[7] = {ag[0], ag[1], ag[2], ag[3], ag[4], ag[5], 0.0};
+                                    front_to_plane(T, h, s.ux, s.uy, -1.0, w * s.sgnC, w * s.sgnC);
+                                }
+#pragma unroll
+                                for (int e = 0; e < 6; e++) {
+                                    const double v = shfl3_sum(T[e], lane);
+                                    if (child && c == 0) Ls.ang[g][e] = v;
+                                }
+                            }
+                        }
+                        // whole triangle: a + t^2 b
+                        double a[7] = {0, 0, 0, 0, 0, 0, 0}, b[7] = {0, 0, 0, 0, 0, 0, 0};
+                        if (live) {
+                            double fa[7], fb[7];
+                            front_full(fa, fb, view);
+                            const double ws = w * s.sgnC, zs = G.zeta * G.sigma;
+                            front_to_plane(a, fa, s.ux, s.uy, zs, ws, ws);
+                            front_to_plane(b, fb, s.ux, s.uy, zs, ws, ws);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 7; e++) {
+                            const double va = shfl3_sum(a[e], lane), vb = shfl3_sum(b[e], lane);
+                            if (child && c == 0) {
+                                Ls.full[g][e] = va;
+                                Ls.full[g][7 + e] = vb;
+                            }
+                        }
+                        if (child && c == 0) {
+                            Ls.kP[g] = knP;
+                            Ls.kS[g] = knS;
+                            Ls.zeta[g] = G.zeta;
+                            Ls.zs[g] = G.zeta * G.sigma;
+                        }
+                    }
+                }
+                if (!work) continue;
+                // items of each level: this child's levels, transposed to the level's children
+                unsigned mP = level_bits(kaP - kc0, knP - kc0), mS = level_bits(kaS - kc0, knS - kc0);
+                if (zeta != 0.0) {
+                    // c_S t == zeta: no front
+                    const int kd = (int)rint(zeta * A.icS), b = kd - kc0;
+                    if (b >= 0 && b < 32 && A.velS * (kd * A.dt) == zeta) mP &= ~(1u << b);
+                }
+                mP = transpose32(mP, lane);
+                mS = transpose32(mS, lane);
+                if (!wanted) mP = mS = 0;
+                const int n = __popc(mP) + __popc(mS);
+                int incl = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int total = __shfl_sync(0xffffffffu, incl, 31);
+                Ls.mask[lane] = (unsigned long long)mP | ((unsigned long long)mS << 32);
+                Ls.off[lane] = incl - n;
+                if (lane == 31) Ls.off[32] = total;
+                __syncwarp();
+                for (int base = 0; base < total; base += 32) {
+                    const int idx = min(base + lane, total - 1);
+                    int lev = 0;                                       // last level with off <= idx that has items
+#pragma unroll
+                    for (int h = 16; h > 0; h >>= 1)
+                        if (Ls.off[lev + h] <= idx) lev += h;
+                    const unsigned long long m = Ls.mask[lev];
+                    int r = idx - Ls.off[lev];
+                    const int np = __popc((unsigned)m);
+                    const bool isP = r < np;
+                    const int slot = nth_bit(isP ? (unsigned)m : (unsigned)(m >> 32), isP ? r : r - np);
+                    {
+                        const FrontView C{Ls.f + slot, kSlots};
+                        const double kk = isP ? k1 : ks, t = (kc0 + lev) * A.dt, w = kk * C(FC_W);
+                        double H[7], T[7] = {0, 0, 0, 0, 0, 0, 0};
+                        front_item(H, C, (isP ? A.velP : A.velS) * t, isP);
+                        front_to_plane(T, H, C(FC_UX), C(FC_UY), C(FC_ZS), w, isP ? -w : w);
+#pragma unroll
+                        for (int e = 0; e < 7; e++) Ls.res[lane][e] = T[e];
+                    }
+                    const int l0 = __shfl_sync(0xffffffffu, lev, 0), l1 = __shfl_sync(0xffffffffu, lev, 31);
+                    __syncwarp();
+                    const int e = lane & 7;
+                    for (int lv = l0 + (lane >> 3); lv <= l1; lv += 4) {
+                        const int i0 = max(Ls.off[lv] - base, 0), i1 = min(Ls.off[lv + 1] - base, 32);
+                        if (e < 7 && i0 < i1) {
+                            double v = Ls.acc[lv][e];
+                            for (int q = i0; q < i1; q++) v += Ls.res[q][e];
+                            Ls.acc[lv][e] = v;
+                        }
+                    }
+                    __syncwarp();
+                }
+                // nodes the fronts have passed wholly, nodes with an angle: lane = level
+                if (wanted) {
+                    const int k = kc0 + lane;
+                    const double t = k * A.dt, t2 = t * t, rP = A.velP * t, rS = A.velS * t;
+                    double T[7];
+#pragma unroll
+                    for (int e = 0; e < 7; e++) T[e] = Ls.acc[lane][e];
+                    for (int g = 0; g < gn; g++) {
+                        const double zg = Ls.zeta[g];
+                        const bool cP = k >= Ls.kP[g] && (zg == 0.0 || zg != rS), cS = k >= Ls.kS[g];
+                        if (cP) {
+                            const double ca = cS ? ks - k1 : -k1, cb = cS ? 0.0 : t2, c0 = cS ? ks + k1 : k1;
+                            const double* fu = Ls.full[g];
+                            T[0] += c0 * fu[0] + cb * fu[7];
+#pragma unroll
+                            for (int e = 1; e < 7; e++) T[e] += ca * fu[e] - cb * fu[7 + e];
+                        }
+                        if ((circ >> (3 * g)) & 1u) {
+                            double rhoP, rhoS;
+                            const int type = classify(zg, rP, rS, Ls.dmin[g], rhoP, rhoS);
+                            if (type != T_NONE)
+                                front_node_terms(T, Ls.ang[g], zg, Ls.zs[g], type, rP, rS, rhoP, rhoS, !cP, !cS, t2, k1, ks);
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 7; e++) Ls.acc[lane][e] = T[e];
+                }
+            }
+            // F(t_k) = (S I + C^T M C) / 2 in global axes, one lane per level
+            double Fk[6] = {0, 0, 0, 0, 0, 0};
+            if (wanted) {
+                const double S = Ls.acc[lane][0];
+                double T[6];
+#pragma unroll
+                for (int e = 0; e < 6; e++) T[e] = Ls.acc[lane][1 + e];
+                double M[3][3] = {{T[0], T[1], T[3]}, {T[1], T[2], T[4]}, {T[3], T[4], T[5]}};
+                const double* Cm = F.C;
+                double MC[3][3];
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+#pragma unroll
+                    for (int cc = 0; cc < 3; cc++)
+                        MC[r][cc] = M[r][0] * Cm[cc] + M[r][1] * Cm[3 + cc] + M[r][2] * Cm[6 + cc];
+                double Rm[3][3];
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+#pragma unroll
+                    for (int cc = r; cc < 3; cc++)
+                        Rm[r][cc] = Cm[r] * MC[0][cc] + Cm[3 + r] * MC[1][cc] + Cm[6 + r] * MC[2][cc];
+                Fk[0] = 0.5 * (S + Rm[0][0]);
+                Fk[1] = 0.5 * Rm[0][1];
+                Fk[2] = 0.5 * Rm[0][2];
+                Fk[3] = 0.5 * (S + Rm[1][1]);
+                Fk[4] = 0.5 * Rm[1][2];
+                Fk[5] = 0.5 * (S + Rm[2][2]);
+            }
+            // E_l = (F_{l+1} - 2 F_l + F_{l-1}) / (4 pi rho) for the lags l = k - 1
+            // completed by the chunk's levels k, clean-up |x| < 1e-14
             // (calcMatrixSubBlock.m:15,23,111; calcMatrixBlock.m:77); F_0 = 0
             const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-            for (int kl = lane; kl < nk; kl += 32) {
-                const int k = kc0 + kl, l = k - 1;
-                if (l < llo || l > lhi) continue;
-                double b[6];
+            const int l = kc0 + lane - 1;
+            double b[6];
 #pragma unroll
-                for (int e = 0; e < 6; e++) {
-                    const double f1 = Ls.acc[e][kl];
-                    const double f0 = (k - 1 < 1) ? 0.0 : (kl >= 1 ? Ls.acc[e][kl - 1] : Ls.carry[1][e]);
-                    const double fm = (k - 2 < 1) ? 0.0 : (kl >= 2 ? Ls.acc[e][kl - 2] : Ls.carry[kl][e]);
-                    const double v = ((f1 + (-2.0) * f0) + fm) / A.c4pirho;
-                    b[e] = (fabs(v) < 1.0e-14) ? 0.0 : v;
-                }
-                if (A.Eb) {
+            for (int e = 0; e < 6; e++) Ls.acc[lane][e] = Fk[e];
+            __syncwarp();
+            // rows -2 and -1: the two levels before the chunk
+            const double* r1 = lane >= 1 ? Ls.acc[lane - 1] : Ls.carry[1];
+            const double* r2 = lane >= 2 ? Ls.acc[lane - 2] : Ls.carry[lane];
 #pragma unroll
-                    for (int e = 0; e < 6; e++) A.Eb[(bbase + (l - llo)) * 6 + e] = b[e];
+            for (int e = 0; e < 6; e++) {
+                const double v = ((Fk[e] + (-2.0) * r1[e]) + r2[e]) * A.ic4;
+                b[e] = (fabs(v) < 1.0e-14) ? 0.0 : v;
+            }
+            __syncwarp();
+            if (lane >= 30) {
+                // a further chunk follows a full one only
+#pragma unroll
+                for (int e = 0; e < 6; e++) Ls.carry[lane - 30][e] = Fk[e];
+            }
+            if (lane < nk && l >= llo && l <= lhi && (!CLS || cls[l - A.lag0] == ic)) {
+                if (OUT != OUT_DENSE) {
+                    double* dst = OUT == OUT_RECORDS ? A.Lout + (rec + (long long)(l - A.lag0) * rstride) * 6 : A.Eb + (bbase + (l - llo)) * 6;
+                    if ((reinterpret_cast<size_t>(dst) & 15) == 0) {
+                        double2* d2 = reinterpret_cast<double2*>(dst);
+                        d2[0] = make_double2(b[0], b[1]);
+                        d2[1] = make_double2(b[2], b[3]);
+                        d2[2] = make_double2(b[4], b[5]);
+                    } else {
+                        // a caller's buffer off a 16-byte boundary
+#pragma unroll
+                        for (int e = 0; e < 6; e++) dst[e] = b[e];
+                    }
                 } else {
 #pragma unroll
                     for (int e9 = 0; e9 < 9; e9++) store_entry(A, l - A.lag0, i, j, e9, b[map[e9]]);
                 }
             }
             __syncwarp();
-            if (lane < 6) {
-                const double c1 = Ls.carry[1][lane];
-                Ls.carry[0][lane] = (nk >= 2) ? Ls.acc[lane][nk - 2] : c1;
-                Ls.carry[1][lane] = Ls.acc[lane][nk - 1];
-            }
-            __syncwarp();
         }
     }
+    // a class without a rule: the block is zero
+    if (CLS)
+        for (int l = llo + lane; l <= lhi; l += 32)
+            if (cls[l - A.lag0] >= ncls)
+                for (int e = 0; e < 6; e++) A.Lout[(rec + (long long)(l - A.lag0) * rstride) * 6 + e] = 0.0;
 }
 
-template <int WPB, int MINB, bool MIXED>
-__global__ void __launch_bounds__(32 * WPB, MINB) sa_level_kernel(SAArgs A) {
+// Table: ClassTable, or NoClasses for the one rule of the arguments.
+struct NoClasses {};
+EBEM_DI const ClassTable* class_table(const ClassTable& T) { return &T; }
+EBEM_DI const ClassTable* class_table(const NoClasses&) { return nullptr; }
+
+template <int WPB, int MINB, int OUT, class Table>
+__global__ void __launch_bounds__(32 * WPB, MINB) sa_level_kernel(SAArgs A, const __grid_constant__ Table T) {
     extern __shared__ __align__(16) unsigned char level_smem[];
     LevelShared* Lsh = reinterpret_cast<LevelShared*>(level_smem);
-    __shared__ double gt[48];          // Gauss-Legendre nodes and weights (gl_table_entry)
     __shared__ unsigned long long blk_count;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     LevelShared& Ls = Lsh[wib];
-    if (threadIdx.x < 24) gl_table_entry(threadIdx.x, gt[threadIdx.x], gt[24 + threadIdx.x]);
     if (threadIdx.x == 0) blk_count = 0;
     __syncthreads();
     const long long NP = A.pairs ? A.npairs : A.diag_only ? (long long)A.nsrc : (long long)A.nsrc * A.nj;
     const long long nwarps = (long long)gridDim.x * WPB;
     unsigned long long my_count = 0;
+    const bool small = NP <= 0xffffffffLL;
     for (long long p = (long long)blockIdx.x * WPB + wib; p < NP; p += nwarps) {
         int i, j;
         if (A.pairs) {
@@ -745,10 +726,11 @@ __global__ void __launch_bounds__(32 * WPB, MINB) sa_level_kernel(SAArgs A) {
             i = pj.x;
             j = pj.y;
         } else {
-            i = A.src0 + (int)(p % A.nsrc);
-            j = A.diag_only ? i : A.j0 + (int)(p / A.nsrc);
+            const long long q = A.diag_only ? 0 : small ? (long long)((unsigned)p / (unsigned)A.nsrc) : p / A.nsrc;
+            i = A.src0 + (int)(p - q * A.nsrc);
+            j = A.diag_only ? i : A.j0 + (int)q;
         }
-        level_pair<MIXED>(A, Ls, gt, gt + 24, p, i, j, lane, my_count);
+        level_pair<OUT, std::is_same<Table, ClassTable>::value>(A, class_table(T), Ls, p, i, j, lane, my_count);
     }
     if (A.count) {
         if (lane == 0 && my_count) atomicAdd(&blk_count, my_count);
@@ -757,68 +739,26 @@ __global__ void __launch_bounds__(32 * WPB, MINB) sa_level_kernel(SAArgs A) {
     }
 }
 
-template <int WPB, int MINB, bool MIXED>
-static int launch_level(const SAArgs& A, long long NN, int device, cudaStream_t s) {
+template <int OUT, class Table>
+static int launch_level(SAArgs A, const Table& T, long long NN, int device, cudaStream_t s) {
+    constexpr int WPB = EBEM_LEVEL_WPB, MINB = EBEM_LEVEL_MINB;
+    sa_args_derive(A);
     const size_t smem = sizeof(LevelShared) * WPB;
-    if (int rc = opt_in_smem(sa_level_kernel<WPB, MINB, MIXED>, smem, s)) return rc;
+    if (int rc = opt_in_smem(sa_level_kernel<WPB, MINB, OUT, Table>, smem, s)) return rc;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     long long want = (NN + WPB - 1) / WPB;
     long long cap = (long long)sms * MINB * 16;
     unsigned blocks = (unsigned)(want < cap ? want : cap);
     if (blocks == 0) blocks = 1;
-    sa_level_kernel<WPB, MINB, MIXED><<<blocks, 32 * WPB, smem, s>>>(A);
-    EBEM_CUDA_TRY(cudaGetLastError());
-    return EBEM_OK;
-}
-int launch_sa_assemble(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc,
-                       double* d_E, size_t ld, size_t ld_lag, int accumulate, unsigned long long* d_count,
-                       cudaStream_t s, int diag_only, int mixed, const int2* pairs, long long npairs) {
-    if (EBEM_SA_TWOPASS && EBEM_SA_KERNEL == 0 && !diag_only && !pairs)
-        return launch_sa_twopass(m, P, n_gh, lag0, nlag, src0, nsrc, d_E, ld, ld_lag, accumulate, d_count, mixed, s);
-    SAArgs A;
-    A.geo = m.d_geo;
-    A.nodes = m.d_nodes;
-    A.N = m.nt;
-    A.n_gh = n_gh;
-    A.velP = P.velP;
-    A.velS = P.velS;
-    A.dt = P.dt;
-    A.c4pirho = 4 * kPi * P.rho;
-    A.lag0 = lag0;
-    A.nlag = nlag;
-    A.src0 = src0;
-    A.nsrc = nsrc;
-    A.diag_only = diag_only;
-    A.E = d_E;
-    A.ld = ld;
-    A.ld_lag = ld_lag;
-    A.accumulate = accumulate;
-    A.count = d_count;
-    A.pairs = pairs;
-    A.npairs = npairs;
-    A.j0 = 0;
-    A.nj = m.nt;
-    long long NN = diag_only ? (long long)nsrc : (long long)nsrc * m.nt;
-    if (pairs) NN = npairs;
-    if (EBEM_SA_KERNEL == 0)
-        return mixed ? launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, true>(A, NN, m.device, s)
-                     : launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, false>(A, NN, m.device, s);
-    if (pairs || mixed) return fail(EBEM_ERR_INVALID, "pair lists and mixed precision need the warp kernel");
-    int threads = 128;
-    long long blocks = (NN + threads - 1) / threads;
-    if (blocks > 0x7fffffffLL) return fail(EBEM_ERR_INVALID, "mesh too large for one launch");
-    sa_assemble_kernel<<<(unsigned)blocks, threads, 0, s>>>(A);
+    sa_level_kernel<WPB, MINB, OUT, Table><<<blocks, 32 * WPB, smem, s>>>(A, T);
     EBEM_CUDA_TRY(cudaGetLastError());
     return EBEM_OK;
 }
 
-// Level output for the two-pass assembly (sa_twopass.cu): F(t_k) of the pairs
-// (sources [src0, src0 + nsrc), fields [j0, j0 + nj)) at every level their
-// non-null lags in [lag0, lag0 + nlag) need, and those lags.
-int launch_sa_fwarp(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc, int j0,
-                    int nj, int kbase, int KL, double* d_F, int2* d_band, unsigned long long* d_count, int mixed,
-                    cudaStream_t s, const unsigned char* cls, int cls_want) {
+// All source rows and field columns of a mesh at lags [lag0, lag0 + nlag); the
+// caller picks the output.
+static SAArgs sa_args(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag) {
     SAArgs A;
     A.geo = m.d_geo;
     A.nodes = m.d_nodes;
@@ -827,145 +767,65 @@ int launch_sa_fwarp(const MeshData& m, const PhysParams& P, int n_gh, int lag0, 
     A.velP = P.velP;
     A.velS = P.velS;
     A.dt = P.dt;
-    A.c4pirho = 4 * kPi * P.rho;
+    A.ic4 = 1.0 / (4 * kPi * P.rho);
     A.lag0 = lag0;
     A.nlag = nlag;
+    A.nsrc = m.nt;
+    A.nj = m.nt;
+    return A;
+}
+
+int launch_sa_diagonal(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, double* d_E, size_t ld,
+                       size_t ld_lag, cudaStream_t s) {
+    SAArgs A = sa_args(m, P, n_gh, lag0, nlag);
+    A.diag_only = 1;
+    A.E = d_E;
+    A.ld = ld;
+    A.ld_lag = ld_lag;
+    return launch_level<OUT_DENSE>(A, NoClasses(), m.nt, m.device, s);
+}
+
+int launch_sa_records(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, int src0, int nsrc, int j0,
+                      int nj, double* d_rec, int2* d_band, unsigned long long* d_count, cudaStream_t s,
+                      const unsigned char* cls, const ClassTable* classes) {
+    SAArgs A = sa_args(m, P, n_gh, lag0, nlag);
     A.src0 = src0;
     A.nsrc = nsrc;
-    A.diag_only = 0;
-    A.E = nullptr;
-    A.ld = 0;
-    A.ld_lag = 0;
-    A.accumulate = 0;
-    A.count = d_count;
-    A.pairs = nullptr;
-    A.npairs = 0;
-    A.Fout = d_F;
-    A.band = d_band;
     A.j0 = j0;
     A.nj = nj;
-    A.kbase = kbase;
-    A.KL = KL;
+    A.count = d_count;
+    A.Lout = d_rec;
+    A.band = d_band;
     A.cls = cls;
-    A.cls_want = cls_want;
     const long long NN = (long long)nsrc * nj;
-    return mixed ? launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, true>(A, NN, m.device, s)
-                 : launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, false>(A, NN, m.device, s);
+    return classes ? launch_level<OUT_RECORDS>(A, *classes, NN, m.device, s)
+                   : launch_level<OUT_RECORDS>(A, NoClasses(), NN, m.device, s);
 }
 
 // Blocks of an explicit list of (source, field) pairs at every lag [0, nlag)
 // with the outer rule in m.d_nodes (n_gh nodes per triangle, composite or
 // not): out[(p nlag + l) 6 + e], the 6 symmetric entries (11, 12, 13, 22, 23,
 // 33) of E_l, zero outside the pair's non-null lags.
-__global__ void pair_emit_kernel(const double* __restrict__ Fb, const int2* __restrict__ band, long long np, int nlag,
-                                 int KL, double c4, double* __restrict__ out) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= np * nlag) return;
-    const long long p = t / nlag;
-    const int l = (int)(t - p * nlag);
-    const int2 b = band[p];
-    double v[6] = {0, 0, 0, 0, 0, 0};
-    if (b.x >= 0 && l >= b.x && l <= b.y) {
-        // level k of pair p at (p KL + k - 1) 6 (kbase = 1); F_0 = 0
-        const double* rec = Fb + p * KL * 6;
-#pragma unroll
-        for (int e = 0; e < 6; e++) {
-            const double a1 = rec[l * 6 + e];
-            const double a0 = (l >= 1) ? rec[(l - 1) * 6 + e] : 0.0;
-            const double am = (l >= 2) ? rec[(l - 2) * 6 + e] : 0.0;
-            const double x = ((a1 + (-2.0) * a0) + am) / c4;
-            v[e] = (fabs(x) < 1.0e-14) ? 0.0 : x;
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < 6; e++) out[t * 6 + e] = v[e];
-}
-
 int launch_sa_pair_blocks(const MeshData& m, const PhysParams& P, int n_gh, const int2* d_pairs, long long npairs,
                           int nlag, double* d_out, cudaStream_t s) {
     if (npairs <= 0) return EBEM_OK;
-    const int KL = nlag;                          // levels 1 .. nlag
-    const long long chunk = std::max<long long>(1, ((long long)256 << 20) / ((long long)KL * 48 + 8));
-    const long long np0 = std::min(npairs, chunk);
-    double* Fb = nullptr;
-    if (ws_malloc(&Fb, (size_t)np0 * KL * 48 + (size_t)np0 * sizeof(int2), s) != cudaSuccess)
-        return fail(EBEM_ERR_NOMEM, "pair-block workspace allocation failed");
-    int2* band = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(Fb) + (size_t)np0 * KL * 48);
-    int rc = EBEM_OK;
-    for (long long q0 = 0; q0 < npairs && rc == EBEM_OK; q0 += np0) {
-        const long long nq = std::min(np0, npairs - q0);
-        SAArgs A;
-        A.geo = m.d_geo;
-        A.nodes = m.d_nodes;
-        A.N = m.nt;
-        A.n_gh = n_gh;
-        A.velP = P.velP;
-        A.velS = P.velS;
-        A.dt = P.dt;
-        A.c4pirho = 4 * kPi * P.rho;
-        A.lag0 = 0;
-        A.nlag = nlag;
-        A.src0 = 0;
-        A.nsrc = m.nt;
-        A.diag_only = 0;
-        A.E = nullptr;
-        A.ld = 0;
-        A.ld_lag = 0;
-        A.accumulate = 0;
-        A.count = nullptr;
-        A.pairs = d_pairs + q0;
-        A.npairs = nq;
-        A.Fout = Fb;
-        A.band = band;
-        A.j0 = 0;
-        A.nj = 0;
-        A.kbase = 1;
-        A.KL = KL;
-        rc = launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, false>(A, nq, m.device, s);
-        if (rc) break;
-        const long long nt = nq * nlag;
-        pair_emit_kernel<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(Fb, band, nq, nlag, KL, 4 * kPi * P.rho,
-                                                                     d_out + q0 * nlag * 6);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(EBEM_ERR_CUDA, std::string("pair blocks: ") + cudaGetErrorString(e));
-    }
-    ws_free(Fb, s);
-    return rc;
+    EBEM_CUDA_TRY(cudaMemsetAsync(d_out, 0, (size_t)npairs * nlag * 6 * sizeof(double), s));
+    SAArgs A = sa_args(m, P, n_gh, 0, nlag);
+    A.pairs = d_pairs;
+    A.npairs = npairs;
+    A.Lout = d_out;
+    return launch_level<OUT_RECORDS>(A, NoClasses(), npairs, m.device, s);
 }
 
 // Banded output: all lags [0, L) of every pair, written into the band
-// layout that band_structure() built (only the warp kernel has this mode).
+// layout that band_structure() built.
 int launch_sa_assemble_banded(const MeshData& m, const PhysParams& P, int n_gh, int L, double* d_Eb,
-                              const long long* d_boff, const int* d_blo, int mixed, cudaStream_t s) {
-    SAArgs A;
-    A.geo = m.d_geo;
-    A.nodes = m.d_nodes;
-    A.N = m.nt;
-    A.n_gh = n_gh;
-    A.velP = P.velP;
-    A.velS = P.velS;
-    A.dt = P.dt;
-    A.c4pirho = 4 * kPi * P.rho;
-    A.lag0 = 0;
-    A.nlag = L;
-    A.src0 = 0;
-    A.nsrc = m.nt;
-    A.diag_only = 0;
-    A.E = nullptr;
-    A.ld = 0;
-    A.ld_lag = 0;
-    A.accumulate = 0;
-    A.count = nullptr;
-    A.pairs = nullptr;
-    A.npairs = 0;
+                              const long long* d_boff, const int* d_blo, cudaStream_t s) {
+    SAArgs A = sa_args(m, P, n_gh, 0, L);
     A.Eb = d_Eb;
     A.boff = d_boff;
     A.blo = d_blo;
-    A.j0 = 0;
-    A.nj = m.nt;
-    const long long NN = (long long)m.nt * m.nt;
-    return mixed ? launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, true>(A, NN, m.device, s)
-                 : launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, false>(A, NN, m.device, s);
+    return launch_level<OUT_BANDED>(A, NoClasses(), (long long)m.nt * m.nt, m.device, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1056,31 +916,14 @@ int launch_sa_assemble_noalloc(const MeshData& m, const PhysParams& P, int n_gh,
     map_nodes_param_kernel<<<(total + 127) / 128, 128, 0, s>>>(m.d_coords, m.d_tris, m.nt, m.d_geo, rule, n_gh, d_nodes);
     EBEM_CUDA_TRY(cudaGetLastError());
     if (count) EBEM_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), s));
-    SAArgs A;
-    A.geo = m.d_geo;
+    SAArgs A = sa_args(m, P, n_gh, lag0, nlag);
     A.nodes = d_nodes;
-    A.N = m.nt;
-    A.n_gh = n_gh;
-    A.velP = P.velP;
-    A.velS = P.velS;
-    A.dt = P.dt;
-    A.c4pirho = 4 * kPi * P.rho;
-    A.lag0 = lag0;
-    A.nlag = nlag;
-    A.src0 = 0;
-    A.nsrc = m.nt;
-    A.diag_only = 0;
     A.E = d_E;
     A.ld = 3 * (size_t)m.nt;
     A.ld_lag = A.ld * A.ld;
     A.accumulate = accumulate;
     A.count = count ? d_count : nullptr;
-    A.pairs = nullptr;
-    A.npairs = 0;
-    A.j0 = 0;
-    A.nj = m.nt;
-    const long long NN = (long long)m.nt * m.nt;
-    int rc = launch_level<EBEM_LEVEL_WPB, EBEM_LEVEL_MINB, false>(A, NN, m.device, s);
+    int rc = launch_level<OUT_DENSE>(A, NoClasses(), (long long)m.nt * m.nt, m.device, s);
     if (rc) return rc;
     if (count) {
         EBEM_CUDA_TRY(cudaMemcpyAsync(host_count, d_count, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
@@ -1097,16 +940,14 @@ int launch_sa_assemble_noalloc(const MeshData& m, const PhysParams& P, int n_gh,
 // so a batch result equals the single-mesh results to rounding: per pair the
 // per-level sums of level_pair, one lane per level forming F(t_k) and writing
 // the blocks of the lags it completes.
-template <int WPB, int MINB, bool MIXED>
+template <int WPB, int MINB>
 __global__ void __launch_bounds__(32 * WPB, MINB)
 sa_batch_level_kernel(const BatchInst* __restrict__ insts, int ninst, long long total, int n_gh, int chunk,
                       unsigned long long* next) {
     extern __shared__ __align__(16) unsigned char batch_smem[];
     LevelShared* Lsh = reinterpret_cast<LevelShared*>(batch_smem);
-    __shared__ double gt[48];          // Gauss-Legendre nodes and weights (gl_table_entry)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     LevelShared& Ls = Lsh[wib];
-    if (threadIdx.x < 24) gl_table_entry(threadIdx.x, gt[threadIdx.x], gt[24 + threadIdx.x]);
     __syncthreads();
     unsigned long long unused = 0;
     while (true) {
@@ -1131,37 +972,30 @@ sa_batch_level_kernel(const BatchInst* __restrict__ insts, int ninst, long long 
             A.velP = I.velP;
             A.velS = I.velS;
             A.dt = I.dt;
-            A.c4pirho = I.c4pirho;
-            A.lag0 = 0;
+            A.ic4 = 1.0 / I.c4pirho;
             A.nlag = I.nlag;
-            A.src0 = 0;
             A.nsrc = I.N;
-            A.diag_only = 0;
+            A.nj = I.N;
             A.E = I.E;
             A.ld = 3 * (size_t)I.N;
             A.ld_lag = A.ld * A.ld;
-            A.accumulate = 0;
-            A.count = nullptr;
-            A.pairs = nullptr;
-            A.npairs = 0;
-            A.j0 = 0;
-            A.nj = I.N;
             A.zeros_written = 1;
+            sa_args_derive(A);
             const long long q = p - I.pair_begin;
-            level_pair<MIXED>(A, Ls, gt, gt + 24, q, (int)(q % I.N), (int)(q / I.N), lane, unused);
+            level_pair<OUT_DENSE, false>(A, nullptr, Ls, q, (int)(q % I.N), (int)(q / I.N), lane, unused);
         }
     }
 }
 
-template <int WPB, int MINB, bool MIXED>
+template <int WPB, int MINB>
 static int launch_batch_level(const BatchInst* d_insts, int ninst, long long total, int n_gh, int chunk,
                               unsigned long long* d_next, int device, cudaStream_t s) {
     const size_t smem = sizeof(LevelShared) * WPB;
-    if (int rc = opt_in_smem(sa_batch_level_kernel<WPB, MINB, MIXED>, smem, s)) return rc;
+    if (int rc = opt_in_smem(sa_batch_level_kernel<WPB, MINB>, smem, s)) return rc;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const unsigned blocks = (unsigned)(sms * MINB);       // one resident wave: persistent
-    sa_batch_level_kernel<WPB, MINB, MIXED><<<blocks, 32 * WPB, smem, s>>>(d_insts, ninst, total, n_gh, chunk, d_next);
+    sa_batch_level_kernel<WPB, MINB><<<blocks, 32 * WPB, smem, s>>>(d_insts, ninst, total, n_gh, chunk, d_next);
     EBEM_CUDA_TRY(cudaGetLastError());
     return EBEM_OK;
 }
@@ -1186,17 +1020,14 @@ __global__ void batch_zero_kernel(const BatchInst* __restrict__ insts) {
     }
 }
 
-int launch_sa_batch(const BatchInst* d_insts, int ninst, long long total, int n_gh, int mixed, int wpb, int chunk,
+int launch_sa_batch(const BatchInst* d_insts, int ninst, long long total, int n_gh, int wpb, int chunk,
                     unsigned long long* d_next, int device, cudaStream_t s) {
     (void)n_gh;
     if (ninst > 65535) return fail(EBEM_ERR_INVALID, "too many batch instances for one launch");
     batch_zero_kernel<<<dim3(148, (unsigned)ninst), 256, 0, s>>>(d_insts);
     EBEM_CUDA_TRY(cudaGetLastError());
-    if (wpb == 2)
-        return mixed ? launch_batch_level<2, 6, true>(d_insts, ninst, total, n_gh, chunk, d_next, device, s)
-                     : launch_batch_level<2, 6, false>(d_insts, ninst, total, n_gh, chunk, d_next, device, s);
-    return mixed ? launch_batch_level<4, 3, true>(d_insts, ninst, total, n_gh, chunk, d_next, device, s)
-                 : launch_batch_level<4, 3, false>(d_insts, ninst, total, n_gh, chunk, d_next, device, s);
+    if (wpb == 2) return launch_batch_level<2, 8>(d_insts, ninst, total, n_gh, chunk, d_next, device, s);
+    return launch_batch_level<4, 4>(d_insts, ninst, total, n_gh, chunk, d_next, device, s);
 }
 
 }  // namespace ebem

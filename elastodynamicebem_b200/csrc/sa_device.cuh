@@ -72,6 +72,7 @@ EBEM_MFN double m_exp(double x) { return exp(x); }
 EBEM_MFN double m_acos(double x) { return acos(x); }
 EBEM_MFN double m_asin(double x) { return asin(x); }
 EBEM_MFN double m_atan2(double y, double x) { return atan2(y, x); }
+EBEM_MFN double m_atan(double x) { return atan(x); }
 
 enum : int { T_NONE = 0, T_SP_SP = 1, T_SP_P = 2, T_P = 3 };
 

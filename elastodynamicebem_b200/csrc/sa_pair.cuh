@@ -111,11 +111,13 @@ EBEM_DI void tri_geom(const double V[3][3], TriGeom& g) {
 
 // Node-level geometry: the projection of preparazioneTriangolo.m — the field
 // triangle in the plane frame centred at the projected node, the signed
-// doubled areas of the three children, zeta, the side of the node and d_min.
+// doubled areas of the three children, zeta, the side of the node, whether it
+// projects inside the triangle (node_project) and d_min (node_geo).
 struct NodeGeo {
     double zeta, sigma, dMIN;
     double tri[3][2];
     double c[3];
+    bool inside;
 };
 
 EBEM_DI double edge_distance(const double tri[3][2]) {
@@ -144,7 +146,7 @@ EBEM_DI double edge_distance(const double tri[3][2]) {
     return (best == INFINITY) ? 0.0 : best;
 }
 
-EBEM_DI void node_geo(NodeGeo& G, const NodeW& sp, const TriGeom& F) {
+EBEM_DI void node_project(NodeGeo& G, const NodeW& sp, const TriGeom& F) {
     double ds0 = sp.x - F.P1[0], ds1 = sp.y - F.P1[1], ds2 = sp.z - F.P1[2];
     double param_s = F.n[0] * ds0 + F.n[1] * ds1 + F.n[2] * ds2;
     double pp0 = sp.x - param_s * F.n[0], pp1 = sp.y - param_s * F.n[1], pp2 = sp.z - param_s * F.n[2];
@@ -169,7 +171,12 @@ EBEM_DI void node_geo(NodeGeo& G, const NodeW& sp, const TriGeom& F) {
     double eta2 = c[2] / Ad, eta3 = c[0] / Ad, eta1 = 1 - eta2 - eta3;
     bool inside = (-1.0e-6 <= eta1) && (-1.0e-6 <= eta2) && (-1.0e-6 <= eta3) && (eta1 <= 1) && (eta2 <= 1) &&
                   (eta3 <= 1);
-    G.dMIN = inside ? 0.0 : edge_distance(tri);
+    G.inside = inside;
+}
+
+EBEM_DI void node_geo(NodeGeo& G, const NodeW& sp, const TriGeom& F) {
+    node_project(G, sp, F);
+    G.dMIN = G.inside ? 0.0 : edge_distance(G.tri);
 }
 
 // Child k = (O, P_k, P_k+1) of a projected node, oriented counter-clockwise

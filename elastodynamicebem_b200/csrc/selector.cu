@@ -610,8 +610,36 @@ int selector_infer(const float* d_params, const MeshData& m, const PhysParams& P
     return rc;
 }
 
+// Non-null lags of each class: one thread per pair, block sums in shared memory.
+__global__ void __launch_bounds__(256) class_lags_kernel(const TriGeom* __restrict__ geo, int N, double velP, double velS,
+                                                         double dt, int lag0, int nlag,
+                                                         const unsigned char* __restrict__ cls, int nclass,
+                                                         unsigned long long* __restrict__ cnt) {
+    __shared__ unsigned bin[256];
+    bin[threadIdx.x] = 0;
+    __syncthreads();
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < (long long)N * N) {
+        int llo, lhi;
+        pair_band(geo[p / N], geo[p % N], velP, velS, dt, lag0, nlag, &llo, &lhi);
+        const unsigned char* c = cls + p * nlag - lag0;
+        int run = 0, last = -1;                          // one addition per run of equal classes
+        for (int l = llo; l >= 0 && l <= lhi; l++) {
+            if (c[l] != last) {
+                if (run) atomicAdd(bin + last, (unsigned)run);
+                last = c[l];
+                run = 0;
+            }
+            run++;
+        }
+        if (run) atomicAdd(bin + last, (unsigned)run);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nclass && bin[threadIdx.x]) atomicAdd(cnt + threadIdx.x, (unsigned long long)bin[threadIdx.x]);
+}
+
 int assemble_selected(MeshData& m, const PhysParams& P, const int* h_rules, int nclass, const unsigned char* d_cls,
-                      int lag0, int nlag, double* d_E, int prec, long long* h_counts, cudaStream_t s) {
+                      int lag0, int nlag, double* d_E, long long* h_counts, cudaStream_t s) {
     unsigned long long* d_cnt = nullptr;
     if (ws_malloc(&d_cnt, sizeof(unsigned long long) * nclass, s) != cudaSuccess)
         return fail(EBEM_ERR_NOMEM, "assembly workspace allocation failed");
@@ -619,13 +647,21 @@ int assemble_selected(MeshData& m, const PhysParams& P, const int* h_rules, int 
     if (cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * nclass, s) != cudaSuccess)
         rc = fail(EBEM_ERR_CUDA, "counter reset failed");
     const size_t n3 = 3 * (size_t)m.nt;
-    // class 0 also writes the zeros outside every pair's non-null lags
+    if (!rc && h_counts) {
+        const long long NN = (long long)m.nt * m.nt;
+        class_lags_kernel<<<(unsigned)((NN + 255) / 256), 256, 0, s>>>(m.d_geo, m.nt, P.velP, P.velS, P.dt, lag0, nlag, d_cls,
+                                                                       nclass, d_cnt);
+        if (cudaGetLastError() != cudaSuccess) rc = fail(EBEM_ERR_CUDA, "class count failed");
+    }
+    // one level pass and one emission for all classes
+    ClassTable T;
     for (int c = 0; c < nclass && rc == EBEM_OK; c++) {
         rc = map_nodes_composite(m, h_rules[2 * c], h_rules[2 * c + 1], s);
-        if (!rc)
-            rc = launch_sa_twopass(m, P, h_rules[2 * c] * h_rules[2 * c + 1], lag0, nlag, 0, m.nt, d_E, n3, n3 * n3, 0,
-                                   d_cnt + c, prec, s, d_cls, c);
+        T.n_gh[c] = h_rules[2 * c] * h_rules[2 * c + 1];
+        T.nodes[c] = m.d_nodes;
     }
+    T.n = nclass;
+    if (!rc) rc = launch_sa_twopass(m, P, 0, lag0, nlag, 0, m.nt, d_E, n3, n3 * n3, 0, nullptr, s, d_cls, &T);
     std::vector<unsigned long long> hc(nclass, 0ull);
     if (rc == EBEM_OK && h_counts) {
         cudaError_t e = cudaMemcpyAsync(hc.data(), d_cnt, sizeof(unsigned long long) * nclass, cudaMemcpyDeviceToHost, s);

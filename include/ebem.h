@@ -161,14 +161,11 @@ int ebem_assemble_sa_panel(const ebem_mesh* mesh, const ebem_problem* prob, int 
                            long long* nonnull);
 
 /* Precision of the semi-analytic assembly.  EBEM_PREC_FP64 is the reference's
- * arithmetic.  EBEM_PREC_MIXED evaluates the bulk quadrature, the Gauss-
- * Legendre nodes of the edge-bounded pieces (after the node position e^s,
- * which stays FP64), in FP32 with FP32 per-lane accumulation, and keeps FP64
- * for the closed-form pieces at the wavefronts and the singularity (crossing
- * angles, logarithmic terms), the whole-edge moments, the level combination
- * F_{l+1} - 2 F_l + F_{l-1}, the E_0 factorisation and the time-marching
- * right-hand side.  No counterpart in the reference (the mixed-precision form
- * of the assembly). */
+ * arithmetic.  EBEM_PREC_MIXED lets the assembly evaluate a bulk
+ * quadrature in FP32 (front-bounded pieces, the level combination, the E_0
+ * factorisation and the marching always FP64).  The closed-form inner
+ * integral has no such quadrature left, so both modes give the FP64 blocks.
+ * No counterpart in the reference. */
 #define EBEM_PREC_FP64 0
 #define EBEM_PREC_MIXED 1
 
