@@ -9,7 +9,7 @@
 //   post-processing   functions/BEMenerg_indir/BEMenerg_postProc/BEMenerg_postProcA/
 //                     BEMenerg_postProcA_singlePoint.m:21-61, _calcMatrix.m, _calcMatrixBlock.m
 #include "ebem_internal.h"
-#include "sa_pair.cuh"
+#include "sa_group.cuh"
 
 #include <cublas_v2.h>
 #include <cusolverDn.h>
@@ -548,20 +548,7 @@ void lu_plan_destroy(LuPlan* plan) {
 // - M(t - k dt)) phi_k + M(t - nHat dt) phi_{nHat+1}, nHat = ceil(t/dt) - 1,
 // M(tau) the single-point combined kernel integral over each triangle
 // (BEMenerg_postProcA_singlePoint.m:21-61), divided by 4 pi rho and cleaned
-// below 1e-14 (BEMenerg_postProcA_calcMatrix.m:103).  One thread per
-// (triangle, point, time); consecutive lanes take consecutive triangles of
-// one (point, time), reduce over the warp and add to u with one atomic per
-// component.
-__device__ __forceinline__ void pp_block(double M[6], const TriGeom& F, const NodeW& x, double tau, double velP,
-                                         double velS, double c4) {
-    level_value(M, 1, velP, velS, tau, F, &x, 1);
-#pragma unroll
-    for (int e = 0; e < 6; e++) {
-        double v = M[e] / c4;
-        M[e] = (fabs(v) < 1.0e-14) ? 0.0 : v;
-    }
-}
-
+// below 1e-14 (BEMenerg_postProcA_calcMatrix.m:103).
 __device__ __forceinline__ void sym_mv_add(double acc[3], const double M[6], const double* ph, double sgn) {
     acc[0] += sgn * (M[0] * ph[0] + M[1] * ph[1] + M[2] * ph[2]);
     acc[1] += sgn * (M[1] * ph[0] + M[3] * ph[1] + M[4] * ph[2]);
@@ -593,155 +580,149 @@ __device__ __forceinline__ bool pp_before_front(double reach, double velP, doubl
     return __dmul_rn(velP, tau) < reach;
 }
 
-// pp_block, or zero at an instant before the P front reaches the triangle.
-__device__ __forceinline__ void pp_block_or_zero(double M[6], const TriGeom& F, const NodeW& x, double reach,
-                                                 double tau, double velP, double velS, double c4) {
-    if (pp_before_front(reach, velP, tau)) {
-#pragma unroll
-        for (int e = 0; e < 6; e++) M[e] = 0.0;
-    } else {
-        pp_block(M, F, x, tau, velP, velS, c4);
-    }
-}
-
-// At most 128 registers (4 blocks of 128 threads per SM; 254 without the
-// cap): 40 scattered times at 256 points on the 1280-triangle sphere 37.1 ->
-// 27.6 ms.
-__global__ void __launch_bounds__(128, 4) pp_sa_kernel(const TriGeom* __restrict__ geo, int N, const double* __restrict__ pts,
-                                                    int npts, const double* __restrict__ times, int ntimes,
-                                                    const double* __restrict__ phi, int nT, double velP, double velS,
-                                                    double dt, double c4, double* __restrict__ u) {
-    // one thread per (triangle j, point p, time q), j fastest: a warp shares
-    // (p, q) unless it straddles two of them
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long NP = (long long)N * npts;
-    const bool valid = idx < NP * ntimes;
-    const int q = valid ? (int)(idx / NP) : 0;
-    const long long r = valid ? idx - (long long)q * NP : 0;
-    const int j = (int)(r % N), p = (int)(r / N);
-    NodeW x;
-    x.x = pts[3 * p]; x.y = pts[3 * p + 1]; x.z = pts[3 * p + 2]; x.w = 1.0;
-    const TriGeom& F = geo[j];
-    const size_t n3 = 3 * (size_t)N;
-    const double t = times[q];
-    double acc[3] = {0, 0, 0};
-    if (valid && t > 0) {
-        int nHat = (int)ceil(t / dt) - 1;
-        if (nHat > nT - 1) nHat = nT - 1;
-        double Mc[6], Mn[6];
-        const double reach = pp_reach(F, x);
-        pp_block_or_zero(Mc, F, x, reach, t, velP, velS, c4);
-        for (int k = 1; k <= nHat; k++) {
-            pp_block_or_zero(Mn, F, x, reach, __dsub_rn(t, __dmul_rn((double)k, dt)), velP, velS, c4);   // no fused multiply-add
-            const double* ph = phi + (size_t)(k - 1) * n3 + 3 * (size_t)j;
-            double D[6];
-#pragma unroll
-            for (int e = 0; e < 6; e++) { D[e] = Mc[e] - Mn[e]; Mc[e] = Mn[e]; }
-            sym_mv_add(acc, D, ph, 1.0);
-        }
-        sym_mv_add(acc, Mc, phi + (size_t)nHat * n3 + 3 * (size_t)j, 1.0);
-    }
-    double sum[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        double v = acc[c];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        sum[c] = v;
-    }
-    // a warp may straddle two (point, time) outputs: then every lane adds its own value
-    const long long o_me = (long long)q * npts + p;
-    const long long o_first = __shfl_sync(0xffffffffu, o_me, 0), o_last = __shfl_sync(0xffffffffu, o_me, 31);
-    const int v_last = __shfl_sync(0xffffffffu, valid ? 1 : 0, 31);
-    if (o_first == o_last && v_last) {
-        if ((threadIdx.x & 31) == 0)
-            for (int c = 0; c < 3; c++) atomicAdd(u + o_me * 3 + c, sum[c]);
-    } else if (valid) {
-        for (int c = 0; c < 3; c++) atomicAdd(u + o_me * 3 + c, acc[c]);
-    }
-}
-
-// Shared instants.  By parts the sum above is
+// By parts the sum above is
 //   u(x, t_q) = M(t_q) phi_0 + sum_{k=1}^{nHat} M(t_q - k dt) (phi_k - phi_{k-1}),
 // and for output times on the time grid the instants t_q - k dt of different
-// (q, k) coincide.  The instants are formed on the host exactly as the
-// per-time kernel forms them (k dt rounded, then subtracted from t_q, no
-// fused multiply-add: the closed form's case selection is discontinuous
-// where a front radius equals the point's distance from the plane, so an
-// instant one unit in the last place off can change M there), deduplicated
-// by value; pp_inst_count_kernel finds, per (point, triangle) row, the first
-// instant that the P front reaches (the instants are sorted, so the skipped
-// ones come first), a prefix sum numbers the evaluated items, and
-// pp_inst_level_kernel evaluates M once per (triangle, point, distinct
-// evaluated instant); pp_inst_sum_kernel contracts, one block per (time,
-// point).
-__global__ void __launch_bounds__(128) pp_inst_count_kernel(const TriGeom* __restrict__ geo, int N,
-                                                            const double* __restrict__ pts, int p0, int np, int nu,
-                                                            const double* __restrict__ taus, double velP,
-                                                            long long* __restrict__ cnt, int* __restrict__ first) {
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long rows = (long long)N * np;
-    if (r == 0) cnt[rows] = 0;            // becomes the total after the exclusive scan
-    if (r >= rows) return;
-    const int pl = (int)(r / N), j = (int)(r - (long long)pl * N);
-    const int p = p0 + pl;
-    NodeW x;
-    x.x = pts[3 * p]; x.y = pts[3 * p + 1]; x.z = pts[3 * p + 2]; x.w = 1.0;
-    const double reach = pp_reach(geo[j], x);
-    // the skip test is monotone in the sorted instants: first instant not skipped
-    int lo = 0, hi = nu;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (pp_before_front(reach, velP, taus[mid])) lo = mid + 1;
-        else hi = mid;
+// (q, k) coincide.  The instants are formed on the host as k dt rounded, then
+// subtracted from t_q (no fused multiply-add: the closed form's case
+// selection is discontinuous where a front radius equals the point's distance
+// from the plane, so an instant one unit in the last place off can change M
+// there) and deduplicated by value; pp_front_kernel evaluates M once per
+// (triangle, point, distinct instant that the P front has reached);
+// pp_inst_sum_kernel contracts, one block per (time, point).
+//
+// pp_front_kernel: one warp per (point, 10 consecutive triangles), their 30
+// children on the lanes (sa_group.cuh), so that what does not depend on the
+// instant is formed once.  Then per triangle the instants run over the lanes:
+// those at which no side is partly covered (zero, or the whole triangle: a +
+// tau^2 b) are finished at once; the others, (triangle, instant) cells with
+// one to six (front, child) items, are queued and evaluated 32 at a time, a
+// lane walking its cell's items.  1280 triangles, 256 points, 40 grid times:
+// 0.47 ms, against 9.4 ms for one thread per (triangle, point, instant) with
+// the edge pieces by Gauss-Legendre (the whole call 9.9 -> 1.2 ms).
+struct PPShared {
+    FrontGroup W;
+    double C[kGroupNodes][9];
+    double near[kSlots], all[kGroupNodes];
+    int first[kGroupNodes];
+    int2 queue[64];                // (triangle of the group, instant)
+};
+
+// M of the cell, cleaned, to the buffer.
+__device__ __forceinline__ void pp_store(double* dst, const double T[7], const double* C, double ic4) {
+    double Fk[6];
+    front_rotate(Fk, T, C);
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+        const double v = Fk[e] * ic4;
+        Fk[e] = (fabs(v) < 1.0e-14) ? 0.0 : v;
     }
-    first[r] = lo;
-    cnt[r] = nu - lo;
+    double2* d2 = reinterpret_cast<double2*>(dst);
+    d2[0] = make_double2(Fk[0], Fk[1]);
+    d2[1] = make_double2(Fk[2], Fk[3]);
+    d2[2] = make_double2(Fk[4], Fk[5]);
 }
 
-__global__ void __launch_bounds__(128, 6) pp_inst_level_kernel(const TriGeom* __restrict__ geo, int N,
-                                                            const double* __restrict__ pts, int p0, int np, int nu,
-                                                            const double* __restrict__ taus, double velP, double velS,
-                                                            double c4, const long long* __restrict__ off,
-                                                            const int* __restrict__ first, long long total,
-                                                            double* __restrict__ Mbuf) {
-    // Items numbered row by row ((point, triangle) rows, triangles fastest),
-    // the evaluated instants of a row consecutive: the lanes of a warp take
-    // neighbouring instants of one (triangle, point), which mostly meet the
-    // fronts in the same way, and 32 evaluations whatever the skipped
-    // instants (97 % of them on the 1280-triangle sphere with 256 points;
-    // warps over all the instants of a row mixed skipped and evaluated lanes:
-    // 4.6 ms there).  Triangles fastest over all instants took more distinct
-    // branches (1.34 against 0.97 ms for 64 points x 40 grid times on 320
-    // triangles before the skip); a buffer ordered (point, triangle,
-    // instant), which makes the stores contiguous, made the contraction's
-    // loads strided (1.8 -> 5.8 ms on 1280).  At most 80 registers (6 blocks
-    // of 128 threads per SM): with 200 registers 2 blocks fitted, 1.5 warps
-    // per scheduler waited on the FP64 dependencies of one evaluation, and
-    // the spills this cap adds cost less than the occupancy gains (11.7 ->
-    // 7.0 ms on 1280 triangles before the skip; 128 registers: 7.4 ms).
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total) return;
-    // the row: last r with off[r] <= idx (off: exclusive prefix sums of the
-    // rows' counts, off[rows] = total; an empty row shares its offset with
-    // the next one)
-    const long long rows = (long long)N * np;
-    long long lo = 0, hi = rows;
-    while (hi - lo > 1) {
-        const long long mid = (lo + hi) >> 1;
-        if (off[mid] <= idx) lo = mid;
-        else hi = mid;
-    }
-    const long long r = lo;
-    const int ui = first[r] + (int)(idx - off[r]);
-    const int pl = (int)(r / N), j = (int)(r - (long long)pl * N);
-    const int p = p0 + pl;
-    NodeW x;
-    x.x = pts[3 * p]; x.y = pts[3 * p + 1]; x.z = pts[3 * p + 2]; x.w = 1.0;
-    double M[6];
-    pp_block(M, geo[j], x, taus[ui], velP, velS, c4);
-    double* dst = Mbuf + (((size_t)pl * nu + ui) * N + j) * 6;
+constexpr int kPPWarps = 4;
+__global__ void __launch_bounds__(32 * kPPWarps, 4) pp_front_kernel(const TriGeom* __restrict__ geo, int N,
+                                                                    const double* __restrict__ pts, int p0, int np, int nu,
+                                                                    const double* __restrict__ taus, double velP,
+                                                                    double velS, double ic4, double* __restrict__ Mbuf) {
+    extern __shared__ __align__(16) unsigned char pp_smem[];
+    const int lane = threadIdx.x & 31;
+    PPShared& S = reinterpret_cast<PPShared*>(pp_smem)[threadIdx.x >> 5];
+    const int groups = (N + kGroupNodes - 1) / kGroupNodes;
+    const long long tasks = (long long)groups * np, nwarps = (long long)gridDim.x * kPPWarps;
+    const double k1 = 1.0 / (velP * velP), ks = 1.0 / (velS * velS);
+    const int g = lane / 3, c = lane - 3 * g;
+    for (long long t = (long long)blockIdx.x * kPPWarps + (threadIdx.x >> 5); t < tasks; t += nwarps) {
+        const int pl = (int)(t / groups), j0 = (int)(t - (long long)pl * groups) * kGroupNodes;
+        const int gn = min(kGroupNodes, N - j0), p = p0 + pl;
+        NodeW x;
+        x.x = pts[3 * p]; x.y = pts[3 * p + 1]; x.z = pts[3 * p + 2]; x.w = 1.0;
+        const TriGeom* F = geo + j0 + min(g, gn - 1);
+        __syncwarp();
+        int first = nu;
+        if (g < gn) {
+            // the skip test is monotone in the sorted instants: first instant not skipped
+            const double reach = pp_reach(*F, x);
+            int lo = 0, hi = nu;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (pp_before_front(reach, velP, taus[mid])) lo = mid + 1;
+                else hi = mid;
+            }
+            first = lo;
+        }
+        if (__ballot_sync(0xffffffffu, first < nu) == 0u) continue;
+        FrontLane L;
+        group_geometry(L, g < gn, &x, F, lane);
+        const unsigned circ = group_fields(S.W, L, lane);
+        if (L.child) {
+            S.near[lane] = L.live ? L.near : INFINITY;
+            if (c == 0) {
+                S.all[g] = L.all;
+                S.first[g] = first;
+            }
 #pragma unroll
-    for (int e = 0; e < 6; e++) dst[e] = M[e];
+            for (int e = 0; e < 3; e++) S.C[g][3 * c + e] = F->C[3 * c + e];
+        }
+        __syncwarp();
+        int queued = 0;
+        for (int gg = 0; gg <= gn; gg++) {
+            const int u0 = gg < gn ? S.first[gg] : nu - 1;          // one step past the last triangle empties the queue
+            for (int ub = u0; ub < nu; ub += 32) {
+                const int ui = ub + lane;
+                bool ask = false;
+                if (gg < gn && ui < nu) {
+                    const double tau = taus[ui], rP = velP * tau, rS = velS * tau, z = S.W.zeta[gg], all = S.all[gg];
+                    const bool front = z == 0.0 || z != rS;        // c_S tau == zeta: no front
+                    const bool cP = front && rP > all, cS = front && rS > all;
+                    if (front)
+#pragma unroll
+                        for (int k = 0; k < 3; k++)
+                            ask = ask || (!cP && rP > S.near[3 * gg + k]) || (!cS && rS > S.near[3 * gg + k]);
+                    if (!ask) {
+                        double T[7] = {0, 0, 0, 0, 0, 0, 0};
+                        group_node(T, S.W, gg, cP, cS, (circ >> (3 * gg)) & 1u, rP, rS, tau * tau, k1, ks);
+                        pp_store(Mbuf + (((size_t)pl * nu + ui) * N + j0 + gg) * 6, T, S.C[gg], ic4);
+                    }
+                }
+                const unsigned asking = __ballot_sync(0xffffffffu, ask);
+                if (ask) S.queue[queued + __popc(asking & ((1u << lane) - 1u))] = make_int2(gg, ui);
+                queued += __popc(asking);
+                __syncwarp();
+                if (queued >= 32 || (gg == gn && queued > 0)) {
+                    const int n = min(queued, 32);
+                    if (lane < n) {
+                        const int2 cell = S.queue[lane];
+                        const double tau = taus[cell.y], rP = velP * tau, rS = velS * tau, all = S.all[cell.x];
+                        const bool cP = rP > all, cS = rS > all;
+                        unsigned m = 0;
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            if (!cP && rP > S.near[3 * cell.x + k]) m |= 1u << k;
+                            if (!cS && rS > S.near[3 * cell.x + k]) m |= 8u << k;
+                        }
+                        double T[7] = {0, 0, 0, 0, 0, 0, 0};
+                        group_node(T, S.W, cell.x, cP, cS, (circ >> (3 * cell.x)) & 1u, rP, rS, tau * tau, k1, ks);
+                        while (m) {
+                            const int k = __ffs(m) - 1;
+                            m &= m - 1;
+                            const bool isP = k < 3;
+                            group_item(T, S.W, 3 * cell.x + (isP ? k : k - 3), isP, isP ? rP : rS, isP ? k1 : ks);
+                        }
+                        pp_store(Mbuf + (((size_t)pl * nu + cell.y) * N + j0 + cell.x) * 6, T, S.C[cell.x], ic4);
+                    }
+                    const int2 rest = S.queue[32 + lane];
+                    __syncwarp();
+                    queued -= n;
+                    if (lane < queued) S.queue[lane] = rest;
+                    __syncwarp();
+                }
+            }
+        }
+    }
 }
 
 // Blocks of 128 threads, or of 1024 when there are too few (time, point)
@@ -763,7 +744,7 @@ __global__ void __launch_bounds__(1024) pp_inst_sum_kernel(const double* __restr
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
         const double reach = pp_reach(geo[j], x);
         for (int k = 0; k <= nh; k++) {
-            if (pp_before_front(reach, velP, taus[tq[k]])) continue;    // M = 0, not stored
+            if (pp_before_front(reach, velP, taus[tq[k]])) break;       // M = 0 from here on (instants fall with k), not stored
             const double* Mv = Mbuf + (((size_t)pl * nu + tq[k]) * N + j) * 6;
             const double* pk = phi + (size_t)k * n3 + 3 * (size_t)j;
             double d[3] = {pk[0], pk[1], pk[2]};
@@ -794,14 +775,10 @@ __global__ void __launch_bounds__(1024) pp_inst_sum_kernel(const double* __restr
     }
 }
 
-// The shared-instant path of launch_pp_sa; returns 1 (nothing done) when the
-// instants barely repeat (times off the grid), where the per-time kernel
-// does the same work without the buffer.
-static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const double* d_phi, const double* d_pts,
-                               int npts, const double* h_times, int ntimes, double* d_u, cudaStream_t s) {
+int launch_pp_sa(const MeshData& m, const PhysParams& P, const double* d_phi, const double* d_pts, int npts,
+                       const double* h_times, int ntimes, double* d_u, cudaStream_t s) {
     std::vector<int> nh(ntimes);
     int kmax = 1;
-    long long terms = 0;
     std::vector<double> taus;
     for (int q = 0; q < ntimes; q++) {
         const double t = h_times[q];
@@ -812,7 +789,6 @@ static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const dou
         }
         nh[q] = n;
         kmax = std::max(kmax, n + 1);
-        terms += n + 1;
         for (int k = 0; k <= n; k++) {
             volatile double a = (double)k * P.dt;      // rounded product, then the difference
             taus.push_back(t - a);
@@ -822,7 +798,11 @@ static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const dou
     std::sort(uniq.begin(), uniq.end());
     uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
     const int nu = (int)uniq.size();
-    if (nu == 0 || 2LL * nu > terms) return 1;
+    if (nu == 0) {
+        // no instant: u = 0
+        EBEM_CUDA_TRY(cudaMemsetAsync(d_u, 0, sizeof(double) * 3 * (size_t)npts * ntimes, s));
+        return EBEM_OK;
+    }
     std::vector<int> tab((size_t)ntimes * kmax, 0);
     {
         size_t c = 0;
@@ -831,6 +811,15 @@ static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const dou
                 tab[(size_t)q * kmax + k] = (int)(std::lower_bound(uniq.begin(), uniq.end(), taus[c++]) - uniq.begin());
     }
     const size_t per_point = (size_t)nu * m.nt * 6 * sizeof(double);
+    if (per_point > ((size_t)1 << 30) && ntimes > 1) {
+        // times off the grid have their own instants each: in two halves
+        const int half = ntimes / 2;
+        if (int rc = launch_pp_sa(m, P, d_phi, d_pts, npts, h_times, half, d_u, s)) return rc;
+        return launch_pp_sa(m, P, d_phi, d_pts, npts, h_times + half, ntimes - half, d_u + 3 * (size_t)npts * half, s);
+    }
+    // up to 1 GiB of M at a time.  1280 triangles, 256 points, 40 grid times (114
+    // distinct instants, 7 MB a point): 1.18 ms; 512 MB 1.35, 192 MB 1.88, 96 MB
+    // 2.98 (a chunk of 14 points has fewer warps than the GPU holds).
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)npts, ((size_t)1 << 30) / per_point));
     // the tables in one upload: instants, index table, nHat
     HostPack pk;
@@ -838,17 +827,10 @@ static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const dou
     const size_t o_tab = pk.add(tab.data(), tab.size() * sizeof(int));
     const size_t o_nh = pk.add(nh.data(), ntimes * sizeof(int));
     unsigned char* d_pack = nullptr;
-    int* d_first = nullptr;
     double* Mbuf = nullptr;
-    long long* d_cnt = nullptr;
-    const long long rows_max = (long long)m.nt * chunk;
-    if (pk.upload(&d_pack, s) != cudaSuccess ||
-        ws_malloc(&d_cnt, (rows_max + 1) * sizeof(long long), s) != cudaSuccess ||
-        ws_malloc(&d_first, rows_max * sizeof(int), s) != cudaSuccess || ws_malloc(&Mbuf, per_point * chunk, s) != cudaSuccess) {
+    if (pk.upload(&d_pack, s) != cudaSuccess || ws_malloc(&Mbuf, per_point * chunk, s) != cudaSuccess) {
         cudaGetLastError();
         ws_free(d_pack, s);
-        ws_free(d_cnt, s);
-        ws_free(d_first, s);
         return fail(EBEM_ERR_NOMEM, "post-processing workspace allocation failed");
     }
     const double* d_taus = reinterpret_cast<const double*>(d_pack + o_taus);
@@ -856,24 +838,14 @@ static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const dou
     const int* d_nh = reinterpret_cast<const int*>(d_pack + o_nh);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device);
-    cudaError_t e = cudaSuccess;
-    int rc = EBEM_OK;
-    for (int p0 = 0; p0 < npts && e == cudaSuccess && rc == EBEM_OK; p0 += chunk) {
+    const size_t smem = sizeof(PPShared) * kPPWarps;
+    cudaError_t e = cudaFuncSetAttribute(pp_front_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (int p0 = 0; p0 < npts && e == cudaSuccess; p0 += chunk) {
         const int np = std::min(chunk, npts - p0);
-        const long long rows = (long long)m.nt * np;
-        pp_inst_count_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(m.d_geo, m.nt, d_pts, p0, np, nu, d_taus,
-                                                                           P.velP, d_cnt, d_first);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) break;
-        rc = exclusive_scan(d_cnt, rows + 1, s);
-        if (rc) break;
-        long long total = 0;
-        e = cudaMemcpyAsync(&total, d_cnt + rows, sizeof(long long), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) break;
-        if (total > 0)
-            pp_inst_level_kernel<<<(unsigned)((total + 127) / 128), 128, 0, s>>>(
-                m.d_geo, m.nt, d_pts, p0, np, nu, d_taus, P.velP, P.velS, 4 * kPi * P.rho, d_cnt, d_first, total, Mbuf);
+        const long long tasks = (long long)((m.nt + kGroupNodes - 1) / kGroupNodes) * np;
+        const long long want = (tasks + kPPWarps - 1) / kPPWarps, cap = 64LL * sms;
+        pp_front_kernel<<<(unsigned)std::min(want, cap), 32 * kPPWarps, smem, s>>>(
+            m.d_geo, m.nt, d_pts, p0, np, nu, d_taus, P.velP, P.velS, 1.0 / (4 * kPi * P.rho), Mbuf);
         const int sum_threads = ((long long)ntimes * np < 2LL * sms) ? 1024 : 128;
         pp_inst_sum_kernel<<<(unsigned)((long long)ntimes * np), sum_threads, 0, s>>>(
             Mbuf, m.d_geo, m.nt, d_pts, p0, np, nu, d_taus, P.velP, d_tab, kmax, d_nh, npts, d_phi, d_u);
@@ -881,38 +853,8 @@ static int launch_pp_sa_shared(const MeshData& m, const PhysParams& P, const dou
     }
     ws_free(Mbuf, s);
     ws_free(d_pack, s);
-    ws_free(d_cnt, s);
-    ws_free(d_first, s);
-    if (rc) return rc;
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(EBEM_ERR_CUDA, std::string("post-processing kernels: ") + cudaGetErrorString(e));
-    return EBEM_OK;
-}
-
-int launch_pp_sa(const MeshData& m, const PhysParams& P, const double* d_phi, const double* d_pts, int npts,
-                 const double* h_times, int ntimes, double* d_u, cudaStream_t s) {
-    {
-        const int rc = launch_pp_sa_shared(m, P, d_phi, d_pts, npts, h_times, ntimes, d_u, s);
-        if (rc != 1) return rc;                         // done (or failed); 1: instants barely repeat
-    }
-    long long total = (long long)m.nt * npts * ntimes;
-    int threads = 128;
-    if ((total + threads - 1) / threads > 0x7fffffffLL)
-        return fail(EBEM_ERR_INVALID, "too many (triangle, point, time) triples for one launch");
-    double* d_times = nullptr;
-    EBEM_CUDA_TRY(ws_malloc(&d_times, sizeof(double) * ntimes, s));
-    cudaError_t e = cudaMemcpyAsync(d_times, h_times, sizeof(double) * ntimes, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_u, 0, sizeof(double) * 3 * (size_t)npts * ntimes, s);
-    if (e != cudaSuccess) {
-        ws_free(d_times, s);
-        return fail(EBEM_ERR_CUDA, std::string("post-processing set-up: ") + cudaGetErrorString(e));
-    }
-    pp_sa_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, s>>>(
-        m.d_geo, m.nt, d_pts, npts, d_times, ntimes, d_phi, P.nT, P.velP, P.velS, P.dt, 4 * kPi * P.rho, d_u);
-    e = cudaGetLastError();
-    ws_free(d_times, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return fail(EBEM_ERR_CUDA, std::string("post-processing kernel: ") + cudaGetErrorString(e));
     return EBEM_OK;
 }
 

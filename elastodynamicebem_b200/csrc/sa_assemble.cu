@@ -24,7 +24,7 @@
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
-#include "sa_front.cuh"
+#include "sa_group.cuh"
 
 namespace ebem {
 
@@ -207,8 +207,6 @@ struct SAArgs {
     double k1 = 0, ks = 0, icP = 0, icS = 0;   // 1 / c_P^2, 1 / c_S^2, 1 / (c_P dt), 1 / (c_S dt)
 };
 
-constexpr int kGroupNodes = 10;  // outer nodes per group: 30 children on 32 lanes
-
 EBEM_HDI void sa_args_derive(SAArgs& A) {
     A.k1 = 1.0 / (A.velP * A.velP);
     A.ks = 1.0 / (A.velS * A.velS);
@@ -265,7 +263,6 @@ __device__ __forceinline__ void store_entry(const SAArgs& A, int q, int i, int j
 // code), hence ic4.  Launch shape: 8 warps, 2 blocks per SM (128 registers);
 // 4 x 4 13.3 against 13.0 ms, 4 x 3 13.5, 16 x 1 13.2, 12 x 1 13.1.
 constexpr int kLevelChunk = 32;  // levels per chunk: one lane per level
-constexpr int kSlots = 3 * kGroupNodes;
 
 #ifndef EBEM_LEVEL_WPB
 #define EBEM_LEVEL_WPB 8
@@ -275,10 +272,7 @@ constexpr int kSlots = 3 * kGroupNodes;
 #endif
 
 struct LevelShared {
-    double f[FC_N * kSlots];                 // children, field-major
-    double full[kGroupNodes][14];            // a, b of the node's whole triangle (plane frame, weighted)
-    double ang[kGroupNodes][6];              // its angle moments around the node
-    double zeta[kGroupNodes], zs[kGroupNodes], dmin[kGroupNodes];
+    FrontGroup W;
     double res[32][7];                       // the round's items
     double acc[kLevelChunk][7];              // per-level sums
     unsigned long long mask[kLevelChunk];    // items of a level: P children, S children << 32
@@ -339,10 +333,6 @@ EBEM_DI unsigned transpose32(unsigned x, int lane) {
     return x;
 }
 
-EBEM_DI double shfl3_sum(double v, int lane) {
-    return v + __shfl_sync(0xffffffffu, v, lane + 1) + __shfl_sync(0xffffffffu, v, lane + 2);
-}
-
 // Whether level k is used by a lag of class c (lags k-1, k, k+1 of the pair's
 // non-null range [llo, lhi]).
 EBEM_DI bool level_wanted(const SAArgs& A, const unsigned char* cls, int c, int k, int llo, int lhi) {
@@ -363,12 +353,12 @@ static int opt_in_smem(K kernel, size_t smem, cudaStream_t s) {
     return EBEM_OK;
 }
 
-// Pair p of the launch: (source i, field j).  With classes (CLS) the pair's
-// levels are walked once for each class its lags have, with that class's
-// rule.
 // Output of a launch: dense blocks, the banded layout, or block records.
 enum : int { OUT_DENSE, OUT_BANDED, OUT_RECORDS };
 
+// Pair p of the launch: (source i, field j).  With classes (CLS) the pair's
+// levels are walked once for each class its lags have, with that class's
+// rule.
 template <int OUT, bool CLS>
 __device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T, LevelShared& Ls, long long p, int i, int j,
                                            int lane, unsigned long long& my_count) {
@@ -434,7 +424,6 @@ __device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T,
         __syncwarp();
         if (lane < 12) (&Ls.carry[0][0])[lane] = 0.0;
         const int ngroups = (n_gh + kGroupNodes - 1) / kGroupNodes, gsize = (n_gh + ngroups - 1) / ngroups;
-        const FrontView view{Ls.f + (lane < kSlots ? lane : 0), kSlots};
         // this lane's child: level ranges of its items, zeta; circ: nodes with an angle (bit 3 g)
         int kaP = 0, knP = 0, kaS = 0, knS = 0;
         double zeta = 0.0;
@@ -450,91 +439,21 @@ __device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T,
                 const int g0 = gsize * grp, gn = min(gsize, n_gh - g0);
                 if (ngroups > 1 || kc0 == klo) {
                     __syncwarp();
-                    FrontSide s;
-                    NodeGeo G;
-                    bool live = false;
-                    double w = 0.0, all = 0.0, tau = 0.0;
+                    FrontLane C;
                     const int g = lane / 3, c = lane - 3 * g;
-                    const bool child = g < gn;
-                    G.zeta = G.sigma = G.dMIN = 0.0;
-                    G.inside = false;
-                    if (child) {
-                        const NodeW sp = nodes[(size_t)i * n_gh + g0 + g];
-                        node_project(G, sp, F);
-                        live = front_side(s, G, c);
-                        w = sp.w;
-                    }
-                    zeta = G.zeta;
-                    const double z2 = G.zeta * G.zeta;
-                    if (live) {
-                        const double F2 = s.F * s.F + 1.0e-6;
-                        const bool foot = s.x1 >= 0 && s.x2 < 0;
-                        all = fmax(fmax(s.R1s, s.R2s), F2);
-                        tau = foot ? F2 : fmax(F2, fmin(s.R1s, s.R2s));
-                    }
-                    // the whole triangle is passed when every live child is
-                    const int b3 = 3 * g;
-                    const double a1 = __shfl_sync(0xffffffffu, all, b3), a2 = __shfl_sync(0xffffffffu, all, b3 + 1);
-                    const double a3 = __shfl_sync(0xffffffffu, all, (b3 + 2) & 31);
-                    all = q_sqrt(fmax(a1, fmax(a2, a3)) + z2);
-                    tau = q_sqrt(tau + z2);
-                    kaP = live ? front_level(tau, A.icP, khi + 1) : khi + 1;
-                    kaS = live ? front_level(tau, A.icS, khi + 1) : khi + 1;
-                    knP = front_level(all, A.icP, khi + 1);
-                    knS = front_level(all, A.icS, khi + 1);
-                    // a node can have an angle only inside the triangle or next to a skipped child
-                    const bool maybe = child && (G.inside || !live);
-                    if (maybe && !G.inside) G.dMIN = edge_distance(G.tri);
-                    const int k0 = maybe ? front_level(q_sqrt(G.dMIN * G.dMIN + z2), A.icP, khi + 1) : kaP;
-                    work = __ballot_sync(0xffffffffu, child && min(k0, kaP) <= khi) != 0u;
+                    group_geometry(C, g < gn, nodes + (size_t)i * n_gh + g0 + min(g, gn - 1), &F, lane);
+                    zeta = C.G.zeta;
+                    kaP = C.live ? front_level(C.near, A.icP, khi + 1) : khi + 1;
+                    kaS = C.live ? front_level(C.near, A.icS, khi + 1) : khi + 1;
+                    knP = front_level(C.all, A.icP, khi + 1);
+                    knS = front_level(C.all, A.icS, khi + 1);
+                    const int k0 = C.maybe ? front_level(q_sqrt(C.G.dMIN * C.G.dMIN + zeta * zeta), A.icP, khi + 1) : kaP;
+                    work = __ballot_sync(0xffffffffu, C.child && min(k0, kaP) <= khi) != 0u;
                     if (work) {
-                        if (live) front_fields(Ls.f + lane, kSlots, s, G.zeta, G.sigma, w * s.sgnC);
-                        // angle of the triangle around the node
-                        double ag[6] = {0, 0, 0, 0, 0, 0};
-                        const bool some = __ballot_sync(0xffffffffu, maybe) != 0u;
-                        circ = 0;
-                        if (some) {
-                            if (live) front_angles(ag, view);
-                            double a0 = live ? s.sgnC * ag[0] : 0.0;
-                            a0 = shfl3_sum(a0, lane);
-                            circ = __ballot_sync(0xffffffffu, child && c == 0 && fabs(a0) > 1.0e-12);
-                            // d_min of the node is known to the lanes that asked for it
-                            if (maybe) Ls.dmin[g] = G.dMIN;
-                            if (circ) {
-                                double T[7] = {0, 0, 0, 0, 0, 0, 0};
-                                if (live) {
-                                    const double h[7] = {ag[0], ag[1], ag[2], ag[3], ag[4], ag[5], 0.0};
-                                    front_to_plane(T, h, s.ux, s.uy, -1.0, w * s.sgnC, w * s.sgnC);
-                                }
-#pragma unroll
-                                for (int e = 0; e < 6; e++) {
-                                    const double v = shfl3_sum(T[e], lane);
-                                    if (child && c == 0) Ls.ang[g][e] = v;
-                                }
-                            }
-                        }
-                        // whole triangle: a + t^2 b
-                        double a[7] = {0, 0, 0, 0, 0, 0, 0}, b[7] = {0, 0, 0, 0, 0, 0, 0};
-                        if (live) {
-                            double fa[7], fb[7];
-                            front_full(fa, fb, view);
-                            const double ws = w * s.sgnC, zs = G.zeta * G.sigma;
-                            front_to_plane(a, fa, s.ux, s.uy, zs, ws, ws);
-                            front_to_plane(b, fb, s.ux, s.uy, zs, ws, ws);
-                        }
-#pragma unroll
-                        for (int e = 0; e < 7; e++) {
-                            const double va = shfl3_sum(a[e], lane), vb = shfl3_sum(b[e], lane);
-                            if (child && c == 0) {
-                                Ls.full[g][e] = va;
-                                Ls.full[g][7 + e] = vb;
-                            }
-                        }
-                        if (child && c == 0) {
+                        circ = group_fields(Ls.W, C, lane);
+                        if (C.child && c == 0) {
                             Ls.kP[g] = knP;
                             Ls.kS[g] = knS;
-                            Ls.zeta[g] = G.zeta;
-                            Ls.zs[g] = G.zeta * G.sigma;
                         }
                     }
                 }
@@ -573,11 +492,9 @@ __device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T,
                     const bool isP = r < np;
                     const int slot = nth_bit(isP ? (unsigned)m : (unsigned)(m >> 32), isP ? r : r - np);
                     {
-                        const FrontView C{Ls.f + slot, kSlots};
-                        const double kk = isP ? k1 : ks, t = (kc0 + lev) * A.dt, w = kk * C(FC_W);
-                        double H[7], T[7] = {0, 0, 0, 0, 0, 0, 0};
-                        front_item(H, C, (isP ? A.velP : A.velS) * t, isP);
-                        front_to_plane(T, H, C(FC_UX), C(FC_UY), C(FC_ZS), w, isP ? -w : w);
+                        const double t = (kc0 + lev) * A.dt;
+                        double T[7] = {0, 0, 0, 0, 0, 0, 0};
+                        group_item(T, Ls.W, slot, isP, (isP ? A.velP : A.velS) * t, isP ? k1 : ks);
 #pragma unroll
                         for (int e = 0; e < 7; e++) Ls.res[lane][e] = T[e];
                     }
@@ -602,21 +519,9 @@ __device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T,
 #pragma unroll
                     for (int e = 0; e < 7; e++) T[e] = Ls.acc[lane][e];
                     for (int g = 0; g < gn; g++) {
-                        const double zg = Ls.zeta[g];
-                        const bool cP = k >= Ls.kP[g] && (zg == 0.0 || zg != rS), cS = k >= Ls.kS[g];
-                        if (cP) {
-                            const double ca = cS ? ks - k1 : -k1, cb = cS ? 0.0 : t2, c0 = cS ? ks + k1 : k1;
-                            const double* fu = Ls.full[g];
-                            T[0] += c0 * fu[0] + cb * fu[7];
-#pragma unroll
-                            for (int e = 1; e < 7; e++) T[e] += ca * fu[e] - cb * fu[7 + e];
-                        }
-                        if ((circ >> (3 * g)) & 1u) {
-                            double rhoP, rhoS;
-                            const int type = classify(zg, rP, rS, Ls.dmin[g], rhoP, rhoS);
-                            if (type != T_NONE)
-                                front_node_terms(T, Ls.ang[g], zg, Ls.zs[g], type, rP, rS, rhoP, rhoS, !cP, !cS, t2, k1, ks);
-                        }
+                        const double zg = Ls.W.zeta[g];
+                        const bool cP = k >= Ls.kP[g] && (zg == 0.0 || zg != rS);
+                        group_node(T, Ls.W, g, cP, k >= Ls.kS[g], (circ >> (3 * g)) & 1u, rP, rS, t2, k1, ks);
                     }
 #pragma unroll
                     for (int e = 0; e < 7; e++) Ls.acc[lane][e] = T[e];
@@ -625,30 +530,10 @@ __device__ __forceinline__ void level_pair(const SAArgs& A, const ClassTable* T,
             // F(t_k) = (S I + C^T M C) / 2 in global axes, one lane per level
             double Fk[6] = {0, 0, 0, 0, 0, 0};
             if (wanted) {
-                const double S = Ls.acc[lane][0];
-                double T[6];
+                double T[7];
 #pragma unroll
-                for (int e = 0; e < 6; e++) T[e] = Ls.acc[lane][1 + e];
-                double M[3][3] = {{T[0], T[1], T[3]}, {T[1], T[2], T[4]}, {T[3], T[4], T[5]}};
-                const double* Cm = F.C;
-                double MC[3][3];
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-#pragma unroll
-                    for (int cc = 0; cc < 3; cc++)
-                        MC[r][cc] = M[r][0] * Cm[cc] + M[r][1] * Cm[3 + cc] + M[r][2] * Cm[6 + cc];
-                double Rm[3][3];
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-#pragma unroll
-                    for (int cc = r; cc < 3; cc++)
-                        Rm[r][cc] = Cm[r] * MC[0][cc] + Cm[3 + r] * MC[1][cc] + Cm[6 + r] * MC[2][cc];
-                Fk[0] = 0.5 * (S + Rm[0][0]);
-                Fk[1] = 0.5 * Rm[0][1];
-                Fk[2] = 0.5 * Rm[0][2];
-                Fk[3] = 0.5 * (S + Rm[1][1]);
-                Fk[4] = 0.5 * Rm[1][2];
-                Fk[5] = 0.5 * (S + Rm[2][2]);
+                for (int e = 0; e < 7; e++) T[e] = Ls.acc[lane][e];
+                front_rotate(Fk, T, F.C);
             }
             // E_l = (F_{l+1} - 2 F_l + F_{l-1}) / (4 pi rho) for the lags l = k - 1
             // completed by the chunk's levels k, clean-up |x| < 1e-14

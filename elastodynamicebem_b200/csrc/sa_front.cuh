@@ -1,11 +1,19 @@
 // Closed form of the semi-analytic inner integral, one front at a time.
 //
-// The quantity is the one of sa_edge.cuh (the reference's SA/calcoloMatrice/
+// The quantity is the reference's (SA/calcoloMatrice/
 // BEMenerg_coreSA_calcIntgInt_childTriangle.m with the region integrals of
 // f/BEMenerg_analiticIntg/*.m and the weights of
-// BEMenerg_coreSA_calcMatrixSubBlock.m:101-104); sa_edge.cuh integrates the
-// edge-bounded pieces by Gauss-Legendre, here every piece has its
-// antiderivative, and the P and the S front separate.
+// BEMenerg_coreSA_calcMatrixSubBlock.m:101-104); the evaluation is not: every
+// piece has its antiderivative in a coordinate along the side, free of the
+// skew basis of coeffB.m whose 1/sin^2 factors amplify rounding by 1e6 on
+// thin children, and the P and the S front separate.
+//
+// Radial antiderivatives in r = sqrt(rho^2 + zeta^2):
+//   A1 = r, A3 = -1/r                     (1/r, 1/r^3 times rho d rho)
+//   B2 = r + zeta^2/r, C2 = ln(rho + r) - rho/r, D2 = -zeta^2/r
+//                                         (in-plane, mixed, normal parts of r_i r_j / r^3)
+//   B4 = -1/r + zeta^2/(3 r^3), C4 = -(r^2 + r rho + rho^2)/(3 (r + rho) r^3),
+//   D4 = -zeta^2/(3 r^3)                  (the same of r_i r_j / r^5)
 //
 // Separation.  A field triangle seen from the projection O of an outer node
 // is a signed sum of children (O, V1, V2).  Along the ray at polar angle
@@ -292,6 +300,32 @@ struct FrontView {
     EBEM_DI double operator()(int f) const { return p[f * stride]; }
 };
 
+// Radial antiderivatives at in-plane radius rho (r = sqrt(rho^2+zeta^2)
+// supplied by the caller).  The mixed (C) and normal (D) parts are only used
+// for zeta > 0.
+struct Rad { double A1, A3, B2, C2, D2, B4, C4, D4; };
+
+EBEM_DI Rad radial_at(double rho, double r, double zeta) {
+    Rad v;
+    // one reciprocal gives both 1/r and 1/(r + rho)
+    const double q = 1.0 / (r * (r + rho));
+    const double ir = (r + rho) * q, ir3 = ir * ir * ir, z2 = zeta * zeta;
+    v.A1 = r;
+    v.A3 = -ir;
+    v.B2 = r + z2 * ir;
+    v.D2 = -z2 * ir;
+    v.B4 = -ir + z2 * ir3 * (1.0 / 3.0);
+    v.D4 = -z2 * ir3 * (1.0 / 3.0);
+    if (zeta > 0) {
+        v.C2 = q_log(rho + r) - rho * ir;
+        v.C4 = -(r * r + r * rho + rho * rho) * ir3 * (r * q) * (1.0 / 3.0);
+    } else {
+        v.C2 = 0.0;
+        v.C4 = 0.0;
+    }
+    return v;
+}
+
 // Terms of a node whose field triangle fills the angle moments g (1, cc, sc,
 // ss, c, s; plane frame, signed and weighted) around it: V at the fronts that
 // have not passed the whole triangle (inP, inS) and at O.  zs = zeta sigma.
@@ -301,11 +335,11 @@ EBEM_DI void front_node_terms(double T[7], const double g[6], double zeta, doubl
     if (inP) {
         sc += 2 * k1 * rP;
         in -= 4 * k1 * rP;
-        if (zeta > 0) mx -= k1 * (m_log(rhoP + rP) + rP / (rP + rhoP));
+        if (zeta > 0) mx -= k1 * (q_log(rhoP + rP) + rP / (rP + rhoP));
     }
     if (type == T_P) {
         const double v = k1 * zeta + t2 / zeta;
-        const double lz = m_log(zeta);
+        const double lz = q_log(zeta);
         sc -= v;
         in += 2 * v;
         mx += k1 * lz + t2 / (zeta * zeta);
@@ -319,13 +353,13 @@ EBEM_DI void front_node_terms(double T[7], const double g[6], double zeta, doubl
     } else {
         if (inS) {
             in += 4 * ks * rS;
-            if (zeta > 0) mx += ks * (m_log(rhoS + rS) + rS / (rS + rhoS));
+            if (zeta > 0) mx += ks * (q_log(rhoS + rS) + rS / (rS + rhoS));
         }
         if (zeta > 0) {
             const double k5 = ks + k1, k6 = ks - k1;
             sc -= k5 * zeta;
             in -= 2 * k6 * zeta;
-            mx -= k6 * m_log(zeta);
+            mx -= k6 * q_log(zeta);
             zz += k6 * zeta;
         }
     }

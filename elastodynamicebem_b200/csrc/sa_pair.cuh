@@ -1,7 +1,7 @@
 // Per-pair algebra of the semi-analytic assembly shared by the CUDA kernels
 // (and compilable as host code): the per-triangle preparation, the
-// projection of an outer node on the field plane, the case split, the null
-// test and the combined kernel integral F(t_k) of one (source, field) pair.
+// projection of an outer node on the field plane, the case split and the null
+// test of one (source, field) pair.
 //
 // Reference ("SA/" = functions/BEMenerg_indir/BEMenerg_core/BEMenerg_coreSA/):
 //   frame            SA/calcoloMatrice/operazioniGeometriche/calcoloSistemaRiferimento.m
@@ -14,13 +14,6 @@
 #pragma once
 
 #include "sa_device.cuh"
-#include "sa_edge.cuh"
-
-// 1: child integrals in the edge variable (stable; default); 0: the
-// reference's closed-form region formulas (for comparison)
-#ifndef EBEM_SA_FORM
-#define EBEM_SA_FORM 1
-#endif
 
 namespace ebem {
 
@@ -179,28 +172,6 @@ EBEM_DI void node_geo(NodeGeo& G, const NodeW& sp, const TriGeom& F) {
     G.dMIN = G.inside ? 0.0 : edge_distance(G.tri);
 }
 
-// Child k = (O, P_k, P_k+1) of a projected node, oriented counter-clockwise
-// (fieldTriangle.m:22-33); false when the child is degenerate (|c| < 1e-6).
-EBEM_DI bool node_child(ChildGeo& g, const NodeGeo& G, int k) {
-    const int k1 = (k == 2) ? 0 : k + 1;
-    double C = G.c[k];
-    if (fabs(C) < 1.0e-06) return false;
-    double v1x = G.tri[k][0], v1y = G.tri[k][1], v2x = G.tri[k1][0], v2y = G.tri[k1][1];
-    if (C < 0) { double tx = v1x, ty = v1y; v1x = v2x; v1y = v2y; v2x = tx; v2y = ty; }
-    child_geo(g, v1x, v1y, v2x, v2y, sgn(C));
-    return true;
-}
-
-EBEM_DI bool node_child_e(ChildE& g, const NodeGeo& G, int k) {
-    const int k1 = (k == 2) ? 0 : k + 1;
-    double C = G.c[k];
-    if (fabs(C) < 1.0e-06) return false;
-    double v1x = G.tri[k][0], v1y = G.tri[k][1], v2x = G.tri[k1][0], v2y = G.tri[k1][1];
-    if (C < 0) { double tx = v1x, ty = v1y; v1x = v2x; v1y = v2y; v2x = tx; v2y = ty; }
-    child_geo_e(g, v1x, v1y, v2x, v2y, sgn(C));
-    return true;
-}
-
 // rho_P / rho_S and the case split (BEMenerg_coreSA_calcMatrixSubBlock.m:58-81)
 EBEM_DI int classify(double zeta, double rP, double rS, double dMIN, double& rhoP, double& rhoS) {
     if (zeta == 0) { rhoP = rP; rhoS = rS; }
@@ -237,67 +208,5 @@ EBEM_DI void pair_band(const TriGeom& F, const TriGeom& S, double velP, double v
         }
     }
 }
-
-// F(t_k) for one pair: sum over the outer nodes of the source triangle of the
-// weighted closed-form inner integrals, combined (calcMatrixSubBlock.m:101-104)
-// and rotated back to global axes; 6 symmetric entries (11,12,13,22,23,33).
-EBEM_DI void level_value(double Fk[6], int k, double velP, double velS, double dt, const TriGeom& F,
-                         const NodeW* __restrict__ nodes, int n_gh) {
-    const double t = k * dt;
-    LevelCtx L;
-    L.t2 = t * t;
-    L.RP = velP * t;
-    L.RS = velS * t;
-    double vp2 = velP * velP, vs2 = velS * velS, den = (velP * velS) * (velP * velS);
-    L.k1 = 1.0 / vp2;
-    L.k5 = (vp2 + vs2) / den;
-    L.k6 = (vp2 - vs2) / den;
-    double S = 0.0, T[6] = {0, 0, 0, 0, 0, 0};
-    for (int g = 0; g < n_gh; g++) {
-        NodeW sp = nodes[g];
-        NodeGeo G;
-        node_geo(G, sp, F);
-        double rhoP, rhoS;
-        int type = classify(G.zeta, L.RP, L.RS, G.dMIN, rhoP, rhoS);
-        if (type == T_NONE) continue;
-        double s = 0.0, tt[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll 1
-        for (int c = 0; c < 3; c++) {
-#if EBEM_SA_FORM == 1
-            ChildE cg;
-            if (!node_child_e(cg, G, c)) continue;
-            child_level_e(s, tt, cg, L, G.zeta, G.sigma, rhoP, rhoS, type);
-#else
-            ChildGeo cg;
-            if (!node_child(cg, G, c)) continue;
-            child_level(s, tt, cg, L, G.zeta, G.sigma, rhoP, rhoS, type);
-#endif
-        }
-        S += sp.w * s;
-#pragma unroll
-        for (int e = 0; e < 6; e++) T[e] += sp.w * tt[e];
-    }
-    // local tensor (child-frame order 11,12,22,13,23,33) -> full symmetric
-    double M[3][3] = {{T[0], T[1], T[3]}, {T[1], T[2], T[4]}, {T[3], T[4], T[5]}};
-    const double* C = F.C;
-    // R = C^T M C
-    double MC[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) MC[r][c] = M[r][0] * C[c] + M[r][1] * C[3 + c] + M[r][2] * C[6 + c];
-    double R[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int c = r; c < 3; c++) R[r][c] = C[r] * MC[0][c] + C[3 + r] * MC[1][c] + C[6 + r] * MC[2][c];
-    Fk[0] = 0.5 * (S + R[0][0]);
-    Fk[1] = 0.5 * R[0][1];
-    Fk[2] = 0.5 * R[0][2];
-    Fk[3] = 0.5 * (S + R[1][1]);
-    Fk[4] = 0.5 * R[1][2];
-    Fk[5] = 0.5 * (S + R[2][2]);
-}
-
 
 }  // namespace ebem

@@ -1,4 +1,6 @@
-// Child-triangle integral of the semi-analytic method in the edge variable.
+// Child-triangle integral of the semi-analytic method in the edge variable,
+// the edge-bounded pieces by Gauss-Legendre: the reference of the closed form
+// of sa_front.cuh in test_front_cpu.py, on the host.
 //
 // The quantity is the reference's (SA/calcoloMatrice/
 // BEMenerg_coreSA_calcIntgInt_childTriangle.m with the region integrals of
@@ -37,21 +39,22 @@
 // (DeltaP, DeltaS <= 1e-6 means "no crossing", childTriangle.m:62,75).
 #pragma once
 
-#include "sa_device.cuh"
+#include <cmath>
+
+#include "sa_front.cuh"
 
 #ifndef EBEM_EDGE_H
 #define EBEM_EDGE_H 1.0
 #endif
-#ifndef EBEM_EDGE_NOINLINE
-#define EBEM_EDGE_NOINLINE 1
-#endif
-#if EBEM_EDGE_NOINLINE && defined(__CUDACC__)
-#define EBEM_EFN static __device__ __noinline__
-#else
-#define EBEM_EFN EBEM_DI
-#endif
 
 namespace ebem {
+
+// Time-level constants shared by every node and child.
+struct LevelCtx {
+    double t2;                  // t^2
+    double RP, RS;              // c_P t, c_S t
+    double k1, k5, k6;          // 1/c_P^2, (c_P^2+c_S^2)/(c_P c_S)^2, (c_P^2-c_S^2)/(c_P c_S)^2
+};
 
 // 10-point Gauss-Legendre on [-1, 1] (positive half; symmetric)
 #define EBEM_GL_N2 5
@@ -66,40 +69,6 @@ EBEM_HDI double gl_w(int k) {
     return w[k];
 }
 
-// 6- and 8-point Gauss-Legendre on [-1, 1] (positive halves), for edge
-// pieces shorter than 1/4 and 1/2 in s: the integrands are analytic in the
-// strip |Im s| < pi/2, so on a piece of half-length h the n-point rule errs
-// by about rho^(-2n), rho = (pi/2)/h + sqrt(((pi/2)/h)^2 + 1): 1.5e-17 for
-// n = 6, h = 1/8; 2.3e-18 for n = 8, h = 1/4; 6.7e-17 for n = 10, h = 1/2.
-EBEM_HDI double gl6_x(int k) {
-    const double x[3] = {0.2386191860831969, 0.6612093864662645, 0.9324695142031519};
-    return x[k];
-}
-EBEM_HDI double gl6_w(int k) {
-    const double w[3] = {0.46791393457269104, 0.3607615730481387, 0.17132449237917027};
-    return w[k];
-}
-EBEM_HDI double gl8_x(int k) {
-    const double x[4] = {0.18343464249564978, 0.525532409916329, 0.7966664774136267, 0.9602898564975362};
-    return x[k];
-}
-EBEM_HDI double gl8_w(int k) {
-    const double w[4] = {0.36268378337836166, 0.3137066458778869, 0.22238103445337443, 0.10122853629037706};
-    return w[k];
-}
-
-// The three rules in one table: nodes gt[0..23] (6-point at 0, 8-point at 6,
-// 10-point at 14; each as -x then +x), weights gt[24..47] in the same order.
-EBEM_HDI void gl_table_entry(int t, double& x, double& w) {
-    int n = 10, j = t - 14;
-    if (t < 6) { n = 6; j = t; }
-    else if (t < 14) { n = 8; j = t - 6; }
-    const int half = n / 2, k = j < half ? j : j - half;
-    const double xk = n == 6 ? gl6_x(k) : n == 8 ? gl8_x(k) : gl_x(k);
-    w = n == 6 ? gl6_w(k) : n == 8 ? gl8_w(k) : gl_w(k);
-    x = j < half ? -xk : xk;
-}
-
 // Level-independent data of a child in the edge variable.
 struct ChildE {
     double a, bm;            // |V1| and a*vt_x of the reference (for its DeltaP/DeltaS tests)
@@ -111,32 +80,6 @@ struct ChildE {
     double sgnC;
     double amax;             // max(|V1|, |V2|): a front of larger radius covers the whole edge
 };
-
-// Radial antiderivatives at in-plane radius rho (r = sqrt(rho^2+zeta^2)
-// supplied by the caller).  The mixed (C) and normal (D) parts are only used
-// for zeta > 0.
-struct Rad { double A1, A3, B2, C2, D2, B4, C4, D4; };
-
-EBEM_DI Rad radial_at(double rho, double r, double zeta) {
-    Rad v;
-    // one reciprocal gives both 1/r and 1/(r + rho)
-    const double q = 1.0 / (r * (r + rho));
-    const double ir = (r + rho) * q, ir3 = ir * ir * ir, z2 = zeta * zeta;
-    v.A1 = r;
-    v.A3 = -ir;
-    v.B2 = r + z2 * ir;
-    v.D2 = -z2 * ir;
-    v.B4 = -ir + z2 * ir3 * (1.0 / 3.0);
-    v.D4 = -z2 * ir3 * (1.0 / 3.0);
-    if (zeta > 0) {
-        v.C2 = m_log(rho + r) - rho * ir;
-        v.C4 = -(r * r + r * rho + rho * rho) * ir3 * (r * q) * (1.0 / 3.0);
-    } else {
-        v.C2 = 0.0;
-        v.C4 = 0.0;
-    }
-    return v;
-}
 
 EBEM_DI Rad rad_sub(const Rad& x, const Rad& y) {
     Rad v;
@@ -170,7 +113,7 @@ struct AccE { double S, t11, t12, t22, t13, t23, t33; };
 
 // cos/sin of the polar angle theta (from V1) at edge variable s.
 EBEM_DI void theta_cs(const ChildE& g, double s, double& c, double& sn) {
-    double e = m_exp(s), ie = 1.0 / e;
+    double e = std::exp(s), ie = 1.0 / e;
     double ch = 0.5 * (e + ie);
     double sech = 1.0 / ch, th = (e - ie) / (e + ie);
     c = th * g.cb + sech * g.sb;
@@ -183,7 +126,7 @@ EBEM_DI void crossing_theta(const ChildE& g, double rho, bool positive, double& 
     const double irho = 1.0 / rho;
     double sp = g.F * irho;                                      // sin(phi)
     double cp = sqrt_c((rho - g.F) * (rho + g.F)) * irho;        // |cos(phi)|
-    double phi = asin_c(sp);
+    double phi = std::asin(std::fmin(1.0, sp));
     if (!positive) { phi = kPi - phi; cp = -cp; }
     th = phi - g.beta;                                           // theta = phi - beta
     c = cp * g.cb + sp * g.sb;                                   // cos(phi - beta)
@@ -198,32 +141,6 @@ EBEM_DI void clipped_theta(const ChildE& g, double rho, double sx, bool positive
     if (sx >= g.s0) { th = 0.0; c = 1.0; sn = 0.0; }
     else if (sx <= smin) { th = thg; c = cg; sn = sgm; }
     else crossing_theta(g, rho, positive, th, c, sn);
-}
-
-// Both crossings s = +-sX, sX = acosh(rho/F), of a front of in-plane radius
-// rho with the edge line (the caller has checked that it crosses), clipped to
-// the child as clipped_theta does: (thA, cA, sA) at +sX, (thB, cB, sB) at -sX.
-// One square root, one logarithm and at most one arcsine serve both sides
-// (the angles are phi and pi - phi).
-EBEM_DI void front_cross(const ChildE& g, double rho, double smin, double thg, double cg, double sgm, double& sX,
-                         double& thA, double& cA, double& sA, double& thB, double& cB, double& sB) {
-    const double q = sqrt_c((rho - g.F) * (rho + g.F));
-    sX = m_log((rho + q) / g.F);
-    const bool a0 = sX >= g.s0, ag = !a0 && sX <= smin;
-    const bool b0 = -sX >= g.s0, bg = !b0 && -sX <= smin;
-    double phi = 0.0, sp = 0.0, cp = 0.0;
-    if (!(a0 || ag) || !(b0 || bg)) {
-        const double irho = 1.0 / rho;
-        sp = g.F * irho;
-        cp = q * irho;
-        phi = asin_c(sp);
-    }
-    if (a0) { thA = 0.0; cA = 1.0; sA = 0.0; }
-    else if (ag) { thA = thg; cA = cg; sA = sgm; }
-    else { thA = phi - g.beta; cA = cp * g.cb + sp * g.sb; sA = sp * g.cb - cp * g.sb; }
-    if (b0) { thB = 0.0; cB = 1.0; sB = 0.0; }
-    else if (bg) { thB = thg; cB = cg; sB = sgm; }
-    else { thB = (kPi - phi) - g.beta; cB = -cp * g.cb + sp * g.sb; sB = sp * g.cb + cp * g.sb; }
 }
 
 // Circle-bounded piece between polar angles (tha; ca, sa) and (thb; cb_, sb_):
@@ -246,7 +163,7 @@ EBEM_DI void add_circle(AccE& A, const W4& w, double tha, double ca, double sa, 
 
 // Edge-bounded piece s in [slo, shi]: upper radial limit R(s) = F cosh s,
 // lower limit fixed (its radial vector `lo`).
-EBEM_EFN void add_edge(AccE& A, const ChildE& g, double slo, double shi, const Rad& lo, bool p_terms,
+EBEM_DI void add_edge(AccE& A, const ChildE& g, double slo, double shi, const Rad& lo, bool p_terms,
                       const LevelCtx& L, double zeta, double zs) {
     double len = shi - slo;
     if (!(len > 0)) return;
@@ -260,7 +177,7 @@ EBEM_EFN void add_edge(AccE& A, const ChildE& g, double slo, double shi, const R
             int k = (q < EBEM_GL_N2) ? q : q - EBEM_GL_N2;
             double s = (q < EBEM_GL_N2) ? mid - half * gl_x(k) : mid + half * gl_x(k);
             double wq = half * gl_w(k);
-            double e = m_exp(s), ie = 1.0 / e;
+            double e = std::exp(s), ie = 1.0 / e;
             double ch = 0.5 * (e + ie), sech = 1.0 / ch, th = (e - ie) / (e + ie);
             double c = th * g.cb + sech * g.sb;
             double sn = sech * g.cb - th * g.sb;
@@ -285,7 +202,7 @@ EBEM_EFN void add_edge(AccE& A, const ChildE& g, double slo, double shi, const R
 // (p = |u||v|): tan(x/2) = cr / (p + d), with p + d = cr^2 / (p - d) when d < 0.
 EBEM_DI double log_tan_half(double cr, double d, double p) {
     double pd = (d >= 0) ? (p + d) : (cr * cr) / (p - d);
-    return m_log(cr / pd);
+    return std::log(cr / pd);
 }
 
 // Child (O, V1, V2) oriented counter-clockwise: level-independent data.
@@ -303,8 +220,8 @@ EBEM_DI void child_geo_e(ChildE& g, double v1x, double v1y, double v2x, double v
     g.cb = db / (a * c);
     g.sb = cr / (a * c);
     g.bm = -db / c;
-    g.beta = m_atan2(cr, db);
-    g.gamma = m_atan2(cr, dg);
+    g.beta = std::atan2(cr, db);
+    g.gamma = std::atan2(cr, dg);
     g.s0 = -log_tan_half(cr, db, a * c);          // s at phi = beta
     g.s1 = log_tan_half(cr, da, b * c);           // s at phi = pi - alpha
     g.amax = fmax(a, b);
@@ -334,11 +251,12 @@ EBEM_DI void child_level_e(double& Sout, double T[6], const ChildE& g, const Lev
     // boundary angles: theta = 0 at s0, gamma at s1
     const double th0 = 0.0, c0 = 1.0, sn0 = 0.0;
     double thg = g.gamma, cg, sgm;
-    m_sincos(thg, &sgm, &cg);
+    sgm = std::sin(thg);
+    cg = std::cos(thg);
     if (!xP) {
         add_circle(A, wPc, th0, c0, sn0, thg, cg, sgm, zs);
     } else {
-        double sP = m_log((rhoP + sqrt_c((rhoP - g.F) * (rhoP + g.F))) / g.F);     // acosh(rhoP/F)
+        double sP = std::log((rhoP + sqrt_c((rhoP - g.F) * (rhoP + g.F))) / g.F);     // acosh(rhoP/F)
         // polar angles at s = +sP (phi < pi/2) and s = -sP, clipped to the child
         double thA, cA, sA, thB, cB, sB;
         clipped_theta(g, rhoP, sP, true, smin, thg, cg, sgm, thA, cA, sA);
@@ -348,7 +266,7 @@ EBEM_DI void child_level_e(double& Sout, double T[6], const ChildE& g, const Lev
         if (-sP > smin) add_circle(A, wPc, thB, cB, sB, thg, cg, sgm, zs);
         // edge pieces of the P terms
         if (xS && !isP) {
-            double sS = m_log((rhoS + sqrt_c((rhoS - g.F) * (rhoS + g.F))) / g.F);
+            double sS = std::log((rhoS + sqrt_c((rhoS - g.F) * (rhoS + g.F))) / g.F);
             add_edge(A, g, fmax(sS, smin), fmin(sP, smax), VSe, true, L, zeta, zs);
             add_edge(A, g, fmax(-sP, smin), fmin(-sS, smax), VSe, true, L, zeta, zs);
         } else {
@@ -364,7 +282,7 @@ EBEM_DI void child_level_e(double& Sout, double T[6], const ChildE& g, const Lev
         if (!xS) {
             add_circle(A, wSc, th0, c0, sn0, thg, cg, sgm, zs);
         } else {
-            double sS = m_log((rhoS + sqrt_c((rhoS - g.F) * (rhoS + g.F))) / g.F);
+            double sS = std::log((rhoS + sqrt_c((rhoS - g.F) * (rhoS + g.F))) / g.F);
             double thA, cA, sA, thB, cB, sB;
             clipped_theta(g, rhoS, sS, true, smin, thg, cg, sgm, thA, cA, sA);
             clipped_theta(g, rhoS, -sS, false, smin, thg, cg, sgm, thB, cB, sB);
@@ -383,6 +301,71 @@ EBEM_DI void child_level_e(double& Sout, double T[6], const ChildE& g, const Lev
     T[3] += w * (c * A.t13 - s * A.t23);
     T[4] += w * (s * A.t13 + c * A.t23);
     T[5] += w * A.t33;
+}
+
+EBEM_DI bool node_child_e(ChildE& g, const NodeGeo& G, int k) {
+    const int k1 = (k == 2) ? 0 : k + 1;
+    double C = G.c[k];
+    if (fabs(C) < 1.0e-06) return false;
+    double v1x = G.tri[k][0], v1y = G.tri[k][1], v2x = G.tri[k1][0], v2y = G.tri[k1][1];
+    if (C < 0) { double tx = v1x, ty = v1y; v1x = v2x; v1y = v2y; v2x = tx; v2y = ty; }
+    child_geo_e(g, v1x, v1y, v2x, v2y, sgn(C));
+    return true;
+}
+
+// F(t_k) for one pair: sum over the outer nodes of the source triangle of the
+// weighted closed-form inner integrals, combined (calcMatrixSubBlock.m:101-104)
+// and rotated back to global axes; 6 symmetric entries (11,12,13,22,23,33).
+EBEM_DI void level_value(double Fk[6], int k, double velP, double velS, double dt, const TriGeom& F,
+                         const NodeW* __restrict__ nodes, int n_gh) {
+    const double t = k * dt;
+    LevelCtx L;
+    L.t2 = t * t;
+    L.RP = velP * t;
+    L.RS = velS * t;
+    double vp2 = velP * velP, vs2 = velS * velS, den = (velP * velS) * (velP * velS);
+    L.k1 = 1.0 / vp2;
+    L.k5 = (vp2 + vs2) / den;
+    L.k6 = (vp2 - vs2) / den;
+    double S = 0.0, T[6] = {0, 0, 0, 0, 0, 0};
+    for (int g = 0; g < n_gh; g++) {
+        NodeW sp = nodes[g];
+        NodeGeo G;
+        node_geo(G, sp, F);
+        double rhoP, rhoS;
+        int type = classify(G.zeta, L.RP, L.RS, G.dMIN, rhoP, rhoS);
+        if (type == T_NONE) continue;
+        double s = 0.0, tt[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+        for (int c = 0; c < 3; c++) {
+            ChildE cg;
+            if (!node_child_e(cg, G, c)) continue;
+            child_level_e(s, tt, cg, L, G.zeta, G.sigma, rhoP, rhoS, type);
+        }
+        S += sp.w * s;
+#pragma unroll
+        for (int e = 0; e < 6; e++) T[e] += sp.w * tt[e];
+    }
+    // local tensor (child-frame order 11,12,22,13,23,33) -> full symmetric
+    double M[3][3] = {{T[0], T[1], T[3]}, {T[1], T[2], T[4]}, {T[3], T[4], T[5]}};
+    const double* C = F.C;
+    // R = C^T M C
+    double MC[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) MC[r][c] = M[r][0] * C[c] + M[r][1] * C[3 + c] + M[r][2] * C[6 + c];
+    double R[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int c = r; c < 3; c++) R[r][c] = C[r] * MC[0][c] + C[3 + r] * MC[1][c] + C[6 + r] * MC[2][c];
+    Fk[0] = 0.5 * (S + R[0][0]);
+    Fk[1] = 0.5 * R[0][1];
+    Fk[2] = 0.5 * R[0][2];
+    Fk[3] = 0.5 * (S + R[1][1]);
+    Fk[4] = 0.5 * R[1][2];
+    Fk[5] = 0.5 * (S + R[2][2]);
 }
 
 }  // namespace ebem

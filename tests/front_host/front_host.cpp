@@ -1,10 +1,11 @@
 // Host build of the device algebra of the semi-analytic blocks: F(t_k) of one
 // (source, field) pair from the closed form of sa_front.cuh, the levels,
 // children and fronts walked one after the other, and from the edge
-// quadrature of sa_edge.cuh (level_value).
+// quadrature of edge_quadrature.hpp (level_value).
 #include <cmath>
 #include <vector>
 
+#include "edge_quadrature.hpp"
 #include "sa_front.cuh"
 
 using namespace ebem;

@@ -1,5 +1,5 @@
 """The per-front closed form of the inner integral (csrc/sa_front.cuh) against
-the edge quadrature (csrc/sa_edge.cuh) and the binary128 oracle, both compiled
+an edge quadrature (front_host/edge_quadrature.hpp) and the binary128 oracle, both compiled
 for the host: every level, front and child state of meshes whose children are
 thin, coplanar, collinear with a side, seen from inside, or scaled.
 
