@@ -1208,8 +1208,7 @@ int march_dn_device(const MeshData& m, const double* dV, int LV, const double* d
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cusolverDnHandle_t hs = nullptr;
     cublasHandle_t hb = nullptr;
-    double *A = nullptr, *Q = nullptr, *X = nullptr, *tau = nullptr, *work = nullptr, *beta = nullptr, *rev = nullptr,
-           *y = nullptr;
+    double *A = nullptr, *Q = nullptr, *X = nullptr, *tau = nullptr, *work = nullptr, *beta = nullptr, *rev = nullptr;
     int* info = nullptr;
     const double one = 1.0, zero = 0.0;
     auto cu = [&](cudaError_t e, const char* what) {
@@ -1230,7 +1229,7 @@ int march_dn_device(const MeshData& m, const double* dV, int LV, const double* d
     if (!cu(ws_malloc(&A, sizeof(double) * RC, s), "alloc") || !cu(ws_malloc(&Q, sizeof(double) * RC, s), "alloc") ||
         !cu(ws_malloc(&X, sizeof(double) * RC, s), "alloc") || !cu(ws_malloc(&tau, sizeof(double) * Cn, s), "alloc") ||
         !cu(ws_malloc(&beta, sizeof(double) * (size_t)R * nT, s), "alloc") ||
-        !cu(ws_malloc(&rev, sizeof(double) * (size_t)Cn * nT, s), "alloc") || !cu(ws_malloc(&y, sizeof(double) * R, s), "alloc") ||
+        !cu(ws_malloc(&rev, sizeof(double) * (size_t)Cn * nT, s), "alloc") ||
         !cu(ws_malloc(&info, sizeof(int), s), "alloc")) {
         rc = fail(EBEM_ERR_NOMEM, "direct time-marching workspace allocation failed");
         goto done;
@@ -1264,17 +1263,18 @@ int march_dn_device(const MeshData& m, const double* dV, int LV, const double* d
         goto done;
     // u in reversed time order: u_n at column nT-1-n
     if (!cu(cudaMemsetAsync(rev, 0, sizeof(double) * (size_t)Cn * nT, s), "memset")) goto done;
+    // steps in blocks of kHistBlock, as march_device: beta's columns collect the
+    // right-hand sides
     for (int n = 0; n < nT; n++) {
-        if (!cu(cudaMemcpyAsync(y, beta + (size_t)n * R, sizeof(double) * R, cudaMemcpyDeviceToDevice, s), "copy")) goto done;
-        double* un = rev + (size_t)(nT - 1 - n) * Cn;
+        const int i = n % kHistBlock, M = std::min(i, LK - 1);          // K_1 .. K_M inside the block
+        double *un = rev + (size_t)(nT - 1 - n) * Cn, *y = beta + (size_t)n * R;
+        if (i == 0 && (rc = launch_hist_block(dK + RC, R, Cn, LK - 1, rev, nT, n, beta, sms, s))) goto done;
         if (n > 0) {
             mass_apply_kernel<<<(m.nt + 127) / 128, 128, 0, s>>>(m.d_dir, m.d_tris, m.nt, un + Cn, y);
             if (!cu(cudaGetLastError(), "mass apply")) goto done;
         }
-        const int M = std::min(n + 1, LK) - 1;          // K_1 .. K_M
         if (M > 0 && (rc = launch_hist_gemv(dK + RC, R, (long long)Cn * M, un + Cn, y, sms, s))) goto done;
-        if (!blas_ok(cublasDgemv(hb, CUBLAS_OP_N, Cn, R, &one, X, Cn, y, 1, &zero, un, 1), "least-squares product"))
-            goto done;
+        if ((rc = launch_gemv_add(X, Cn, R, y, un, sms, s))) goto done;
     }
     {
         const long long tot = (long long)Cn * nT;
@@ -1284,7 +1284,7 @@ int march_dn_device(const MeshData& m, const double* dV, int LV, const double* d
     cu(cudaStreamSynchronize(s), "direct time marching");
 done:
     ws_free(A, s); ws_free(Q, s); ws_free(X, s); ws_free(tau, s); ws_free(work, s); ws_free(beta, s); ws_free(rev, s);
-    ws_free(y, s); ws_free(info, s);
+    ws_free(info, s);
     return rc;
 }
 

@@ -261,7 +261,12 @@ int march_dn_device(const MeshData& m, const double* dV, int LV, const double* d
                     double* d_u, cudaStream_t s);
 int march_dd_device(const MeshData& m, const double* dV, int LV, const double* dK, int LK, const double* d_rhs,
                     const double* d_gK, int nT, double* d_phi, cudaStream_t s);
-int launch_hist_gemv(const double* A, int n3, long long K, const double* x, double* y, int sm_count, cudaStream_t s);
+int launch_hist_gemv(const double* A, int rows, long long K, const double* x, double* y, int sm_count, cudaStream_t s);
+int launch_gemv_add(const double* A, int rows, int K, const double* x, double* y, int sm_count, cudaStream_t s);
+// Steps of a marching whose common history is one product (march.cu).
+constexpr int kHistBlock = 8;
+int launch_hist_block(const double* E1, int rows, int cols, int M, const double* rev, int nT, int n0, double* Y, int sm_count,
+                      cudaStream_t s);
 
 // ---------------------------------------------------------------------------
 // learned quadrature selector (selector.cu)
