@@ -15,7 +15,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libebem.so")
 
-SOURCES = ["capi.cu", "quadrature.cu", "sa_assemble.cu", "march.cu", "ghc.cu", "direct.cu", "selector.cu", "banded.cu", "pp_num.cu", "sa_twopass.cu"]
+SOURCES = ["capi.cu", "quadrature.cu", "sa_assemble.cu", "march.cu", "inverse.cu", "ghc.cu", "direct.cu", "selector.cu", "banded.cu", "pp_num.cu", "sa_twopass.cu"]
 HEADERS = ["sa_device.cuh", "sa_pair.cuh", "sa_front.cuh", "sa_group.cuh", "sa_math.cuh", "ebem_internal.h", "ptr_kind.h"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

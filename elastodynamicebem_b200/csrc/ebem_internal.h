@@ -213,6 +213,9 @@ int band_to_dense(const BandOp& op, int lag0, int nlag, double* d_E, cudaStream_
 int band_march(const BandOp& op, const double* d_rhs, int nT, double* d_phi, cudaStream_t s);
 int launch_sa_assemble_banded(const MeshData& m, const PhysParams& P, int n_gh, int L, double* d_Eb,
                               const long long* d_boff, const int* d_blo, cudaStream_t s);
+// A^{-1} by blocked Gauss-Jordan elimination (inverse.cu), n <= gj_max_n().
+int gj_max_n();
+int gj_inverse(const double* dA, int n, double* d_inv, int* singular, cudaStream_t s);
 int lu_plan_create(const double* dA, int n, cudaStream_t s, LuPlan* plan, bool pooled = false, bool cholesky = false);
 int lu_plan_solve(LuPlan* plan, double* db, int nrhs, cudaStream_t s);
 void lu_plan_destroy(LuPlan* plan);
