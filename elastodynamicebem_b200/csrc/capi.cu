@@ -36,7 +36,8 @@ int fail(int code, const std::string& msg) {
 namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
-cudaMemPool_t g_pool[kMaxDevices] = {};
+cudaMemPool_t g_pool[kMaxDevices] = {};          // per-call workspace
+cudaMemPool_t g_store_pool[kMaxDevices] = {};    // storage of handles (store_malloc)
 // Bumped by ebem_device_release: state cached under an older generation
 // (per-thread library handles, the allocation-free scratch address) is
 // abandoned and rebuilt on next use.
@@ -49,11 +50,12 @@ unsigned device_generation(int dev) {
 
 namespace {
 
-// The workspace pool of device dev, created on first use.
-cudaError_t workspace_pool(int dev, cudaMemPool_t* pool) {
+// The pool of device dev in `pools`, created on first use; up to `keep` bytes
+// stay reserved in it.
+cudaError_t device_pool(cudaMemPool_t* pools, int dev, unsigned long long keep, cudaMemPool_t* pool) {
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pool[dev]) {
+    if (!pools[dev]) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -61,31 +63,37 @@ cudaError_t workspace_pool(int dev, cudaMemPool_t* pool) {
         cudaMemPool_t p = nullptr;
         cudaError_t e = cudaMemPoolCreate(&p, &props);
         if (e != cudaSuccess) return e;
-        unsigned long long keep = kWorkspaceKeep;
         e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
         if (e != cudaSuccess) {
             cudaMemPoolDestroy(p);
             return e;
         }
-        g_pool[dev] = p;
+        pools[dev] = p;
     }
-    *pool = g_pool[dev];
+    *pool = pools[dev];
     return cudaSuccess;
 }
-}  // namespace
 
-cudaError_t ws_malloc(void** p, size_t bytes, cudaStream_t s) {
+cudaError_t pool_malloc(cudaMemPool_t* pools, unsigned long long keep, void** p, size_t bytes, cudaStream_t s) {
     *p = nullptr;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     cudaMemPool_t pool = nullptr;
-    if (e == cudaSuccess) e = workspace_pool(dev, &pool);
+    if (e == cudaSuccess) e = device_pool(pools, dev, keep, &pool);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, s);
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
     }
     return e;
+}
+
+}  // namespace
+
+cudaError_t ws_malloc(void** p, size_t bytes, cudaStream_t s) { return pool_malloc(g_pool, kWorkspaceKeep, p, bytes, s); }
+
+cudaError_t store_malloc(void** p, size_t bytes, cudaStream_t s) {
+    return pool_malloc(g_store_pool, kStoreKeep, p, bytes, s);
 }
 
 cudaError_t ws_free(void* p, cudaStream_t s) { return p ? cudaFreeAsync(p, s) : cudaSuccess; }
@@ -260,10 +268,11 @@ int ebem_release_workspace(void) {
     int prev = -1;
     cudaGetDevice(&prev);
     for (int dev = 0; dev < kMaxDevices; dev++) {
-        if (!g_pool[dev]) continue;
+        if (!g_pool[dev] && !g_store_pool[dev]) continue;
         cudaError_t e = cudaSetDevice(dev);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
-        if (e == cudaSuccess) e = cudaMemPoolTrimTo(g_pool[dev], 0);
+        if (e == cudaSuccess && g_pool[dev]) e = cudaMemPoolTrimTo(g_pool[dev], 0);
+        if (e == cudaSuccess && g_store_pool[dev]) e = cudaMemPoolTrimTo(g_store_pool[dev], 0);
         if (e != cudaSuccess) {
             if (prev >= 0) cudaSetDevice(prev);
             return fail(EBEM_ERR_CUDA, std::string("workspace release: ") + cudaGetErrorString(e));
@@ -305,12 +314,13 @@ int ebem_device_release(int device) {
     cudaError_t e = cudaSuccess;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
-        if (g_pool[device]) {
+        for (cudaMemPool_t* pool : {&g_pool[device], &g_store_pool[device]}) {
+            if (!*pool) continue;
             DeviceGuard dg(device);
-            e = cudaDeviceSynchronize();
-            cudaError_t e2 = cudaMemPoolDestroy(g_pool[device]);
-            if (e == cudaSuccess) e = e2;
-            g_pool[device] = nullptr;
+            cudaError_t e1 = cudaDeviceSynchronize();
+            cudaError_t e2 = cudaMemPoolDestroy(*pool);
+            if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : e2;
+            *pool = nullptr;
         }
     }
     release_thread_handles(device);
@@ -822,17 +832,16 @@ static int timemarch_impl(const ebem_mesh* m, const ebem_problem* p, int n_gh, i
     cudaStream_t s = (cudaStream_t)stream;
     const size_t n3 = 3 * (size_t)m->d.nt;
     double *dE = nullptr, *dr = nullptr;
-    if (cudaMalloc(&dE, n3 * n3 * L * sizeof(double)) != cudaSuccess || cudaMalloc(&dr, n3 * p->nt * sizeof(double)) != cudaSuccess) {
-        cudaGetLastError();
-        if (dE) cudaFree(dE);
+    if (ws_malloc(&dE, n3 * n3 * L * sizeof(double), s) != cudaSuccess ||
+        ws_malloc(&dr, n3 * p->nt * sizeof(double), s) != cudaSuccess) {
+        ws_free(dE, s);
         return fail(EBEM_ERR_NOMEM, "device allocation of E or the right-hand side failed");
     }
     int rc = assemble_impl(m, p, n_gh, 0, L, 0, m->d.nt, dE, 3LL * m->d.nt, 0, stream, nullptr, prec);
     if (!rc) rc = ebem_rhs(m, p, n_gh, datum, dr, stream);
     if (!rc) rc = ebem_march(dE, (int)n3, L, dr, p->nt, phi, stream);
-    cudaStreamSynchronize(s);
-    cudaFree(dE);
-    cudaFree(dr);
+    ws_free(dE, s);
+    ws_free(dr, s);
     return rc;
 }
 

@@ -38,6 +38,16 @@ void release_thread_handles(int dev);
 constexpr unsigned long long kWorkspaceKeep = 2ull << 30;
 cudaError_t ws_malloc(void** p, size_t bytes, cudaStream_t s);
 cudaError_t ws_free(void* p, cudaStream_t s);
+// Storage that a handle keeps (a banded operator, a mesh's node tables), from
+// a pool of its own: given back with cudaFree (which waits for the device, as
+// a destroyed handle's users do), without the mapping and unmapping of
+// cudaMalloc; up to kStoreKeep bytes of destroyed handles stay reserved.
+constexpr unsigned long long kStoreKeep = 1ull << 30;
+cudaError_t store_malloc(void** p, size_t bytes, cudaStream_t s);
+template <class T>
+cudaError_t store_malloc(T** p, size_t bytes, cudaStream_t s) {
+    return store_malloc(reinterpret_cast<void**>(p), bytes, s);
+}
 template <class T>
 cudaError_t ws_malloc(T** p, size_t bytes, cudaStream_t s) {
     return ws_malloc(reinterpret_cast<void**>(p), bytes, s);

@@ -65,6 +65,32 @@ __global__ void map_nodes_kernel(const double* __restrict__ coords, const int32_
     out[idx] = o;
 }
 
+// Outer rule passed by value (no device table).
+struct RuleParam {
+    double b[28][3];
+    double w[28];
+};
+
+__global__ void map_nodes_param_kernel(const double* __restrict__ coords, const int32_t* __restrict__ tris, int nt,
+                                       const TriGeom* __restrict__ geo, RuleParam rule, int n_gh,
+                                       NodeW* __restrict__ out) {
+    int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= nt * n_gh) return;
+    int t = idx / n_gh, g = idx % n_gh;
+    double V[3][3];
+    for (int v = 0; v < 3; v++) {
+        int id = tris[3 * t + v];
+        for (int c = 0; c < 3; c++) V[v][c] = coords[3 * id + c];
+    }
+    const double b0 = rule.b[g][0], b1 = rule.b[g][1], b2 = rule.b[g][2];
+    NodeW o;
+    o.x = b0 * V[0][0] + b1 * V[1][0] + b2 * V[2][0];
+    o.y = b0 * V[0][1] + b1 * V[1][1] + b2 * V[2][1];
+    o.z = b0 * V[0][2] + b1 * V[1][2] + b2 * V[2][2];
+    o.w = geo[t].area * rule.w[g];
+    out[idx] = o;
+}
+
 int prep_mesh(MeshData& m, cudaStream_t s) {
     int threads = 128, blocks = (m.nt + threads - 1) / threads;
     prep_kernel<<<blocks, threads, 0, s>>>(m.d_coords, m.d_tris, m.nt, m.d_geo);
@@ -83,32 +109,19 @@ int map_nodes(MeshData& m, int n_gh, cudaStream_t s) {
         m.nodes_rule = n_gh;
         return EBEM_OK;
     }
-    double bary[28 * 3], w[28];
-    int rc = gh_composite(n_gh, 1, bary, w);
-    if (rc) return fail(rc, "unsupported Gauss-Hammer rule");
+    RuleParam rule;
+    if (int rc = gh_composite(n_gh, 1, &rule.b[0][0], rule.w)) return fail(rc, "unsupported Gauss-Hammer rule");
     // the table enters the cache only once the mapping has finished, so a
     // failed call leaves no half-built table behind
     NodeW* table = nullptr;
-    double* d_tab = nullptr;
-    if (cudaMalloc(&table, sizeof(NodeW) * (size_t)m.nt * n_gh) != cudaSuccess ||
-        cudaMalloc(&d_tab, sizeof(double) * 4 * n_gh) != cudaSuccess) {
-        cudaGetLastError();
-        if (table) cudaFree(table);
+    if (store_malloc(&table, sizeof(NodeW) * (size_t)m.nt * n_gh, s) != cudaSuccess)
         return fail(EBEM_ERR_NOMEM, "outer-node table allocation failed");
-    }
-    cudaError_t e = cudaMemcpyAsync(d_tab, bary, sizeof(double) * 3 * n_gh, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_tab + 3 * n_gh, w, sizeof(double) * n_gh, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) {
-        int total = m.nt * n_gh, threads = 128;
-        map_nodes_kernel<<<(total + threads - 1) / threads, threads, 0, s>>>(m.d_coords, m.d_tris, m.nt, m.d_geo, d_tab,
-                                                                               d_tab + 3 * n_gh, n_gh, table);
-        e = cudaGetLastError();
-    }
+    const int total = m.nt * n_gh;
+    map_nodes_param_kernel<<<(total + 127) / 128, 128, 0, s>>>(m.d_coords, m.d_tris, m.nt, m.d_geo, rule, n_gh, table);
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_tab);
     if (e != cudaSuccess) {
-        cudaFree(table);
+        ws_free(table, s);
         return fail(EBEM_ERR_CUDA, std::string("outer-node mapping: ") + cudaGetErrorString(e));
     }
     m.d_node_tables[slot] = table;
@@ -756,32 +769,6 @@ static int noalloc_scratch(int device, unsigned char** out) {
     }
     *out = addr[device];
     return EBEM_OK;
-}
-
-// Outer rule passed by value (no device table).
-struct RuleParam {
-    double b[28][3];
-    double w[28];
-};
-
-__global__ void map_nodes_param_kernel(const double* __restrict__ coords, const int32_t* __restrict__ tris, int nt,
-                                       const TriGeom* __restrict__ geo, RuleParam rule, int n_gh,
-                                       NodeW* __restrict__ out) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nt * n_gh) return;
-    int t = idx / n_gh, g = idx % n_gh;
-    double V[3][3];
-    for (int v = 0; v < 3; v++) {
-        int id = tris[3 * t + v];
-        for (int c = 0; c < 3; c++) V[v][c] = coords[3 * id + c];
-    }
-    const double b0 = rule.b[g][0], b1 = rule.b[g][1], b2 = rule.b[g][2];
-    NodeW o;
-    o.x = b0 * V[0][0] + b1 * V[1][0] + b2 * V[2][0];
-    o.y = b0 * V[0][1] + b1 * V[1][1] + b2 * V[2][1];
-    o.z = b0 * V[0][2] + b1 * V[1][2] + b2 * V[2][2];
-    o.w = geo[t].area * rule.w[g];
-    out[idx] = o;
 }
 
 int launch_sa_assemble_noalloc(const MeshData& m, const PhysParams& P, int n_gh, int lag0, int nlag, double* d_E,

@@ -67,6 +67,8 @@ const char* ebem_last_error(void);
 /* Per-call device workspace comes from a stream-ordered memory pool that the
  * library keeps for each device; up to 2 GiB per device stay reserved between
  * calls so that repeated calls neither allocate nor synchronise the device.
+ * The storage of banded operators and the node tables of meshes come from a
+ * second pool, which keeps up to 1 GiB of what destroyed handles held.
  * ebem_release_workspace returns every device's reserved workspace memory
  * that no call in flight uses (after the calls in flight have finished). */
 int ebem_release_workspace(void);
