@@ -16,7 +16,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libebem.so")
 
 SOURCES = ["capi.cu", "quadrature.cu", "sa_assemble.cu", "march.cu", "inverse.cu", "ghc.cu", "direct.cu", "selector.cu", "banded.cu", "pp_num.cu", "sa_twopass.cu"]
-HEADERS = ["sa_device.cuh", "sa_pair.cuh", "sa_front.cuh", "sa_group.cuh", "sa_math.cuh", "ebem_internal.h", "ptr_kind.h"]
+HEADERS = ["sa_device.cuh", "sa_pair.cuh", "sa_front.cuh", "sa_group.cuh", "sa_math.cuh", "front_bins.cuh", "ebem_internal.h", "ptr_kind.h"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",

@@ -13,30 +13,16 @@
 // (:88-99), entries written only when |value| > 1e-14 before the division by
 // 4 pi rho (:164-165), accumulated into the output (+=).
 //
-// B200 design: one thread per (source, field) pair (consecutive lanes take
-// consecutive sources of one field triangle).  The lag combination E_l =
-// K_{l+1} - 2 K_l + K_{l-1} is taken per node pair on the kernel's scalar time
-// functions (ghc_window2), so a node pair costs work only in the lags whose
-// window a front crosses or lies between the fronts, where the difference
-// has a closed form; windows before the P front or after the S front are
-// skipped on r^2 (the reference evaluates every node pair at every instant
-// of every lag and reduces through shared memory).
+// B200 design: the lag combination E_l = K_{l+1} - 2 K_l + K_{l-1} is taken per
+// node pair and front, where it is non-zero in two lags and a constant after
+// them; a warp per (source, field) pair sorts its node pairs by the level of
+// the arrival and evaluates each once per front (the reference evaluates every
+// node pair at every instant of every lag and reduces through shared memory).
 #include "ebem_internal.h"
 #include "sa_pair.cuh"
 
-// Dispatch between the warp-per-pair and thread-per-pair kernels (compile-time
-// knobs for measuring other thresholds).  Measured with the exact lag skip in
-// both kernels: the warp kernel wins up to about 16k pairs per SM at 84 node
-// pairs and more (sphere of 320 triangles, rule 7/4/3: 5.5 -> 3.3 ms; sphere
-// of 1280, 1.6 M pairs, rule 7/16/3: 166 -> 97 ms); on the 2800-triangle bar
-// (7.8 M pairs, most of them done after the skip test) the thread kernel is
-// 1.4x faster at rule 7/4/3 and even at 7/16/3.
-#ifndef EBEM_GHC_WARP_MIN_NODE_PAIRS
-#define EBEM_GHC_WARP_MIN_NODE_PAIRS 64
-#endif
-#ifndef EBEM_GHC_WARP_MAX_PAIRS_PER_SM
-#define EBEM_GHC_WARP_MAX_PAIRS_PER_SM 16384
-#endif
+#include "front_bins.cuh"
+#include "sa_math.cuh"
 
 namespace ebem {
 
@@ -103,7 +89,10 @@ __host__ __device__ __forceinline__ void ghc_pair(double nu[6], const double x[3
     nu[5] = g1 * x[2] * x[2] + g2;
 }
 
-__global__ void __launch_bounds__(128, 6) ghc_assemble_kernel(GHCArgs A) {
+// Thread per pair, for rules of few node pairs on many pairs (see the launch).
+// 80 registers: bound by the latency of its FP64 chains (157 without the cap:
+// bar of 2800 triangles, rule 7/4/3 188 ms against 137).
+__global__ void __launch_bounds__(128, 6) ghc_assemble_thread_kernel(GHCArgs A) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (long long)A.N * A.N) return;
     const int i = (int)(p % A.N);          // source (outer rule)
@@ -184,28 +173,63 @@ __global__ void __launch_bounds__(128, 6) ghc_assemble_kernel(GHCArgs A) {
     }
 }
 
-// Warp-per-pair variant for small meshes and rules with at least 160 node
-// pairs (see the dispatch in launch_ghc_assemble): the lanes
-// take the node pairs (inner node q, outer node o) of the pair, the same
-// per-node-pair arithmetic as ghc_assemble_kernel, and a warp reduction per
-// lag gives the 6 entries (the thread kernel leaves half of each warp's
-// lanes idle on the skip test).  Both kernels are capped at 80 registers (6
-// blocks of 128 threads per SM); with the compiler's 157 and 170 registers
-// 3 blocks fitted and the FP64 dependency chains were not hidden: sphere of
-// 320 triangles, rule 7/16/3 13.7 -> 6.6 ms (warp kernel); bar of 2800
-// triangles, rule 7/4/3 188 -> 137 ms (thread kernel); 128 registers gave
-// 7.3 and 152 ms.
-__global__ void __launch_bounds__(128, 6) ghc_assemble_warp_kernel(GHCArgs A) {
+// Warp per (source, field) pair.  Bound by instruction issue: 8200 warp
+// instructions a pair at 336 node pairs, of which the items 3200, the arrival
+// levels and the sort 1600, the reductions and sums per lag 2500; 57 % of the
+// issue slots are used with 16 warps an SM (126 registers; 80 registers and 24
+// warps: 1.23 ms against 0.99 for 4 blocks at rule 7/4/3, 12 warps 1.14).  The
+// form before evaluated every node pair in every lag between its P and S
+// arrival.  Sphere of 320 triangles, 40 lags, rule 7/16/3: 6.6 -> 1.3 ms,
+// 7/4/3: 2.4 -> 0.92; sphere of 1280, 7/16/3: 76 -> 16.5 ms; bar of 2800,
+// lags 40..59, 7/4/3: 96 -> 42 ms.
+//
+// Node pair (inner node q, outer node o) at
+// distance r meets front X (P, S) at the first level k with t_k > r / c_X.  The
+// second difference (levels l-1, l, l+1 of t_k = k dt, kernelGHC.cu:88-99) of
+// the kernel kernelGHC.cu:204-259 (nucleo), H = [t > r/c] and Q = (t^2 -
+// r^2/c^2) H per front, is then, with sigma = 1 for P and -1 for S,
+//   lag k - 1:   Hm + Q_k T,      lag k:  -Hm + ((2k + 1) dt^2 - Q_k) T,
+//   lags > k:    2 dt^2 T,
+//   T = sigma (3/2 ir^5 x x^T - 1/2 ir^3 I),
+//   Hm = sigma ir^3/c^2 x x^T (+ ir/c^2 I for S),
+// and zero before.  The items (node pair, front) are sorted by k
+// (front_bins.cuh) and evaluated once each; cur and nxt collect the lags k - 1
+// and k, run every lag from k - 1 on, which the other two take back where the
+// constant does not hold yet.  A warp reduction per lag adds into the pair's
+// sums in shared memory (node pairs beyond kBinChunk in further chunks).
+constexpr int kGHCWarps = 4;
+constexpr size_t kGHCSmem = 200 * 1024;
+
+inline __host__ __device__ int ghc_chunk(int n_in, int n_out) {        // inner nodes of one chunk
+    const int q = kBinChunk / n_out;
+    return q < n_in ? q : n_in;
+}
+inline __host__ __device__ size_t ghc_warp_bytes(int n_in, int n_out, int lag0, int nlag) {
+    const size_t b = (size_t)(4 * (ghc_chunk(n_in, n_out) + n_out) + 6 * ((nlag + 1) / 2 * 2)) * sizeof(double) + front_bins_bytes(bin_window(lag0, nlag).bins);
+    return (b + 15) / 16 * 16;
+}
+
+__global__ void __launch_bounds__(32 * kGHCWarps, 4) ghc_assemble_kernel(GHCArgs A) {
+    extern __shared__ __align__(16) unsigned char ghc_smem[];
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const int n_in = A.n_sub * A.n_sing, NP = n_in * A.n_out;
-    const double cP = A.velP, cS = A.velS, dt = A.dt;
-    const double icP2 = 1 / (cP * cP), icS2 = 1 / (cS * cS);
+    const int n_in = A.n_sub * A.n_sing, chunk = ghc_chunk(n_in, A.n_out);
+    const int lend = A.lag0 + A.nlag - 1;
+    const BinWindow win = bin_window(A.lag0, A.nlag);
+    // nodes (x, y, z, weight), sums (6 per lag), bins
+    double* ys = reinterpret_cast<double*>(ghc_smem + (threadIdx.x >> 5) * ghc_warp_bytes(n_in, A.n_out, A.lag0, A.nlag));
+    double* xs = ys + 4 * chunk;
+    double* acc = xs + 4 * A.n_out;
+    FrontBins B = front_bins_at(reinterpret_cast<unsigned char*>(acc + 6 * ((A.nlag + 1) / 2 * 2)), win.bins);
+    const float iout = 1.0f / (float)A.n_out;          // (np + 1/2) iout: exact quotient for np < kBinChunk
+    const double cP = A.velP, cS = A.velS, dt = A.dt, dt2 = dt * dt;
+    const double icdtP = 1 / (cP * dt), icdtS = 1 / (cS * dt);
+    const double icP2 = 1 / (cP * cP), icS2 = 1 / (cS * cS), ic4 = 1 / A.c4pirho;
     const size_t n3 = A.ld;
     for (long long p = warp; p < (long long)A.N * A.N; p += nwarps) {
-        const int i = (int)(p % A.N);      // source (outer rule)
-        const int j = (int)(p / A.N);      // field (inner rule)
+        const int j = (int)((p <= 0xffffffffLL) ? (long long)((unsigned)p / (unsigned)A.N) : p / A.N);      // field (inner rule)
+        const int i = (int)(p - (long long)j * A.N);                                                    // source (outer rule)
         if (i == j) continue;
         double VS[3][3], VF[3][3];
         for (int v = 0; v < 3; v++)
@@ -217,70 +241,110 @@ __global__ void __launch_bounds__(128, 6) ghc_assemble_warp_kernel(GHCArgs A) {
         for (int a = 0; a < 3; a++)
             for (int b = 0; b < 3; b++) {
                 double d0 = VS[a][0] - VF[b][0], d1 = VS[a][1] - VF[b][1], d2 = VS[a][2] - VF[b][2];
-                distMax = fmax(distMax, sqrt(d0 * d0 + d1 * d1 + d2 * d2));
+                distMax = fmax(distMax, d0 * d0 + d1 * d1 + d2 * d2);
             }
-        int lhi = A.lag0 + A.nlag - 1;
+        distMax = sqrt(distMax);
+        // lags computed: not null, i.e. (l-1) c_S dt <= distMax
+        int lhi = lend;
         while (lhi >= A.lag0 && (lhi - 1) * A.velS * A.dt > distMax) lhi--;
         if (lhi < A.lag0) continue;
         const double aS = A.geo[i].area, aF = A.geo[j].area;
-        // the node pairs' exact distance range (warp min/max): lags whose
-        // window lies before the P front or after the S front for every node
-        // pair add nothing and are skipped by the whole warp
-        double r2min = 1e300, r2max = 0.0;
-        for (int np = lane; np < NP; np += 32) {
-            const int q = np / A.n_out, o = np - q * A.n_out;
-            const double* bq = A.inner + 3 * q;
-            const double* bl = A.outer + 3 * o;
-            double r2 = 0.0;
-            for (int c = 0; c < 3; c++) {
-                const double xc = (bq[0] * VF[0][c] + bq[1] * VF[1][c] + bq[2] * VF[2][c]) -
-                                  (bl[0] * VS[0][c] + bl[1] * VS[1][c] + bl[2] * VS[2][c]);
-                r2 += xc * xc;
-            }
-            r2min = fmin(r2min, r2);
-            r2max = fmax(r2max, r2);
+        __syncwarp();
+        for (int o = lane; o < A.n_out; o += 32) {
+            const double* b = A.outer + 3 * o;
+#pragma unroll
+            for (int c = 0; c < 3; c++) xs[4 * o + c] = b[0] * VS[0][c] + b[1] * VS[1][c] + b[2] * VS[2][c];
+            xs[4 * o + 3] = A.wout[o] * aS;
         }
-        for (int off = 16; off > 0; off >>= 1) {
-            r2min = fmin(r2min, __shfl_xor_sync(0xffffffffu, r2min, off));
-            r2max = fmax(r2max, __shfl_xor_sync(0xffffffffu, r2max, off));
+        for (int t = lane; t < 6 * A.nlag; t += 32) acc[t] = 0.0;
+        __syncwarp();
+        bool any = false;
+        for (int q0 = 0; q0 < n_in; q0 += chunk) {
+            const int nq = min(chunk, n_in - q0), n = nq * A.n_out;
+            for (int q = lane; q < nq; q += 32) {
+                const double* b = A.inner + 3 * (size_t)(q0 + q);
+#pragma unroll
+                for (int c = 0; c < 3; c++) ys[4 * q + c] = b[0] * VF[0][c] + b[1] * VF[1][c] + b[2] * VF[2][c];
+                ys[4 * q + 3] = A.win[(q0 + q) % A.n_sing] * aF;
+            }
+            __syncwarp();
+            bool late = false, met = false;
+            for (int t = lane; t < n; t += 32) {
+                const int q = (int)(((float)t + 0.5f) * iout), o = t - q * A.n_out;
+                const double x0 = ys[4 * q] - xs[4 * o], x1 = ys[4 * q + 1] - xs[4 * o + 1], x2 = ys[4 * q + 2] - xs[4 * o + 2];
+                const double r2 = x0 * x0 + x1 * x1 + x2 * x2, r = q_sqrt(r2);
+                unsigned bP = front_bin(r2, r, cP, icdtP, dt, win);
+                unsigned bS = front_bin(r2, r, cS, icdtS, dt, win);
+                if (bS == 0) bP = bS = kNoBin;                    // past both fronts before the window: the constants cancel
+                else late = late || bS == kNoBin;
+                met = met || bP != kNoBin;
+                B.bin[t] = make_ushort2((unsigned short)bP, (unsigned short)bS);
+            }
+            if (!__any_sync(0xffffffffu, met)) continue;            // both fronts miss the window
+            late = __any_sync(0xffffffffu, late);
+            any = true;
+            const int total = bins_sort(B, n, win.bins, lane);
+            double cur[6] = {0, 0, 0, 0, 0, 0}, nxt[6] = {0, 0, 0, 0, 0, 0}, run[6] = {0, 0, 0, 0, 0, 0};
+            double last = 0.0;                        // this lane's reduced entry of the lag before
+            int first = 0, idle = 0;                  // idle: bins without items up to this one
+            for (int b = 0; b < win.bins; b++) {
+                const int k = win.kbase + b - 1, lastitem = B.off[b], items = lastitem - first;
+                if (items == 0 && first == 0) continue;                 // before the first arrival
+                idle = items ? 0 : idle + 1;
+                const double early = b == 0 ? 0.0 : 1.0;                // bin 0: the constant only
+                const double tk2 = (k * dt) * (k * dt), step = (2 * k + 1) * dt2, tail = 2 * dt2;
+                for (int t = first + lane; t < lastitem; t += 32) {
+                    const unsigned it = B.list[t];
+                    const bool isS = it >> 31;
+                    const int np = (int)(it & 0x7fffffffu), q = (int)(((float)np + 0.5f) * iout), o = np - q * A.n_out;
+                    const double x0 = ys[4 * q] - xs[4 * o], x1 = ys[4 * q + 1] - xs[4 * o + 1], x2 = ys[4 * q + 2] - xs[4 * o + 2];
+                    const double r2 = x0 * x0 + x1 * x1 + x2 * x2, ir = q_rcp(q_sqrt(r2));
+                    const double w = xs[4 * o + 3] * ys[4 * q + 3], ic2 = isS ? icS2 : icP2;
+                    const double ir3 = ir * ir * ir, sw = isS ? -w : w;
+                    const double Q = tk2 - r2 * ic2;
+                    // entries 11, 12, 13, 22, 23, 33 of x x^T times f plus I times d
+                    const double fT = sw * 1.5 * ir3 * ir * ir, dT = -0.5 * sw * ir3;
+                    const double fH = early * (sw * ir3 * ic2), dH = isS ? early * (w * ir * ic2) : 0.0;
+                    const double xx[6] = {x0 * x0, x0 * x1, x0 * x2, x1 * x1, x1 * x2, x2 * x2};
+                    const double e1 = early * (Q - tail), e2 = early * (step - Q - tail);
+#pragma unroll
+                    for (int e = 0; e < 6; e++) {
+                        const bool diag = e == 0 || e == 3 || e == 5;
+                        const double T = fT * xx[e] + (diag ? dT : 0.0), H = fH * xx[e] + (diag ? dH : 0.0);
+                        cur[e] += H + e1 * T;
+                        nxt[e] += e2 * T - H;
+                        if (r2 > 0) run[e] += tail * T;       // r = 0: both fronts here at once, no constant remains
+                    }
+                }
+                const int l = k - 1;
+                if (b > 0 && l >= A.lag0 && l <= lhi) {
+                    if (idle < 3 || l == A.lag0) {
+                        double v[8];
+#pragma unroll
+                        for (int e = 0; e < 6; e++) v[e] = cur[e] + run[e];
+                        v[6] = v[7] = 0.0;
+                        last = warp_reduce_scatter8(v, lane);
+                    }
+                    const int e = scatter8_entry(lane);
+                    if ((lane & 3) == 0 && e < 6) acc[(l - A.lag0) * 6 + e] += last;
+                }
+                first = lastitem;
+#pragma unroll
+                for (int e = 0; e < 6; e++) {
+                    cur[e] = nxt[e];
+                    nxt[e] = 0.0;
+                }
+                if (!late && first == total && items == 0) break;       // every node pair is past both fronts
+            }
+            __syncwarp();
         }
-        for (int l = A.lag0; l <= lhi; l++) {
-            const double thi = (l + 1) * dt, tlo = (l - 1) * dt;
-            const double skipP2 = (cP * thi) * (cP * thi) * (1 + 1e-12);
-            const double skipS2 = (l >= 1) ? (cS * tlo) * (cS * tlo) * (1 - 1e-12) : -1.0;
-            if (r2min > skipP2 || r2max < skipS2) continue;
-            double K[6] = {0, 0, 0, 0, 0, 0};
-            for (int np = lane; np < NP; np += 32) {
-                const int q = np / A.n_out, o = np - q * A.n_out;
-                const double* bq = A.inner + 3 * q;
-                const double* bl = A.outer + 3 * o;
-                double x[3];
-                for (int c = 0; c < 3; c++)
-                    x[c] = (bq[0] * VF[0][c] + bq[1] * VF[1][c] + bq[2] * VF[2][c]) -
-                           (bl[0] * VS[0][c] + bl[1] * VS[1][c] + bl[2] * VS[2][c]);
-                const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-                if (r2 > skipP2 || r2 < skipS2) continue;
-                const double r = sqrt(r2);
-                const Win2 P = ghc_window2(r, cP, l, dt), S = ghc_window2(r, cS, l, dt);
-                const double w = (A.wout[o] * aS) * (A.win[q % A.n_sing] * aF);
-                double nu[6];
-                ghc_pair(nu, x, 1 / r, P.H, S.H, P.Q - S.Q, icP2, icS2);
-#pragma unroll
-                for (int e = 0; e < 6; e++) K[e] += w * nu[e];
-            }
-#pragma unroll
-            for (int e = 0; e < 6; e++)
-                for (int off = 16; off > 0; off >>= 1) K[e] += __shfl_xor_sync(0xffffffffu, K[e], off);
-            if (lane < 9) {
-                const int c = lane / 3, r = lane - 3 * c;
-                const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-                double v = 0;
-#pragma unroll
-                for (int e = 0; e < 6; e++)
-                    if (e == map[lane]) v = K[e];
-                double* base = A.E + (size_t)(l - A.lag0) * A.ld_lag + (3 * (size_t)j) * n3 + 3 * (size_t)i;
-                if (fabs(v) > 1.0e-14) base[c * n3 + r] += v / A.c4pirho;
-            }
+        if (!any) continue;
+        const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+        double* base = A.E + (3 * (size_t)j) * n3 + 3 * (size_t)i;
+        for (int t = lane; t < 9 * (lhi - A.lag0 + 1); t += 32) {
+            const int l = t / 9, e = t - 9 * l, c = e / 3, r = e - 3 * c;
+            const double v = acc[6 * l + map[e]];
+            if (fabs(v) > 1.0e-14) base[(size_t)l * A.ld_lag + c * n3 + r] += v * ic4;
         }
     }
 }
@@ -325,19 +389,36 @@ int launch_ghc_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_
     A.E = d_E;
     A.ld = ld;
     A.ld_lag = ld_lag;
-    long long NN = (long long)m.nt * m.nt;
-    int threads = 128;
-    // warp per pair below the thresholds at the top of this file
+    const long long NN = (long long)m.nt * m.nt;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device);
-    if ((long long)n_gh * n_sub * n_sing >= EBEM_GHC_WARP_MIN_NODE_PAIRS &&
-        NN < (long long)sms * EBEM_GHC_WARP_MAX_PAIRS_PER_SM) {
-        const long long want = (NN + 3) / 4, cap = (long long)sms * 64;
-        ghc_assemble_warp_kernel<<<(unsigned)(want < cap ? want : cap), threads, 0, s>>>(A);
-    } else {
-        ghc_assemble_kernel<<<(unsigned)((NN + threads - 1) / threads), threads, 0, s>>>(A);
+    cudaError_t e = cudaSuccess;
+    const long long np = (long long)n_gh * n_sub * n_sing;
+    // A pair costs the thread kernel time in proportion to the node pairs, the
+    // warp kernel mostly the lags: equal at about 20 node pairs on 700 triangles
+    // and 1280 (9 node pairs: 1.9 against 3.2 ms and 4.3 against 8.8; 36: 5.8
+    // against 3.5 and 13.7 against 9.6).  Below 48 pairs an SM and node pair
+    // the threads do not fill the chip (3 node pairs: 80 triangles 0.15 ms
+    // against 0.08, 252 triangles 0.28 against 0.42).
+    const bool byThread = np <= 24 && NN >= 48LL * sms * np;
+    if (byThread) {
+        ghc_assemble_thread_kernel<<<(unsigned)((NN + 127) / 128), 128, 0, s>>>(A);
+        e = cudaGetLastError();
     }
-    cudaError_t e = cudaGetLastError();
+    for (int l0 = 0; !byThread && l0 < nlag && e == cudaSuccess; l0 += kBinLags) {
+        A.lag0 = lag0 + l0;
+        A.nlag = nlag - l0 < kBinLags ? nlag - l0 : kBinLags;
+        A.E = d_E + (size_t)l0 * ld_lag;
+        const size_t each = ghc_warp_bytes(n_sub * n_sing, n_gh, A.lag0, A.nlag);
+        int warps = kGHCWarps;
+        while (warps > 1 && warps * each > kGHCSmem) warps--;
+        const size_t smem = warps * each;
+        e = cudaFuncSetAttribute(ghc_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) break;
+        const long long want = (NN + warps - 1) / warps, cap = (long long)sms * 64;
+        ghc_assemble_kernel<<<(unsigned)(want < cap ? want : cap), 32 * warps, smem, s>>>(A);
+        e = cudaGetLastError();
+    }
     ws_free(d_tab, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(EBEM_ERR_CUDA, std::string("numerical-inner assembly: ") + cudaGetErrorString(e));
