@@ -34,14 +34,8 @@
 #include <cmath>
 #include <vector>
 
-// Dispatch between the warp-per-pair and thread-per-pair K kernels
-// (compile-time knobs for measuring other thresholds).
-#ifndef EBEM_K_WARP_MIN_NODE_PAIRS
-#define EBEM_K_WARP_MIN_NODE_PAIRS 32
-#endif
-#ifndef EBEM_K_WARP_MAX_PAIRS_PER_SM
-#define EBEM_K_WARP_MAX_PAIRS_PER_SM 4096
-#endif
+#include "front_bins.cuh"
+#include "sa_math.cuh"
 
 namespace ebem {
 
@@ -431,11 +425,10 @@ __host__ __device__ __forceinline__ void k_pair(double out[9], const double x[3]
                              b3 * w[i] * x[k] - b4 * u[3 * i + k];
 }
 
-// Register caps of the double-layer kernels, from an A/B of builds on the
-// 448- and 2800-triangle bars (rule 7/4/3): the thread kernel at 128
-// registers (4 blocks per SM: 725 -> 633 ms; 80 registers 721 ms), the warp
-// kernel at 80 (6 blocks per SM: 28.8 -> 23.4 ms; 128 registers 24.3 ms).
-__global__ void __launch_bounds__(128, 4) k_assemble_kernel(KArgs A) {
+// Thread per pair, for the rules of fewer than 6 node pairs a triangle on many
+// pairs (see the launch): 128 registers (4 blocks an SM; 2800-triangle bar, rule
+// 7/4/3: 633 ms, uncapped 725, 80 registers 721).
+__global__ void __launch_bounds__(128, 4) k_assemble_thread_kernel(KArgs A) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (long long)A.N * A.Nv) return;
     const int x = (int)(p % A.N), s = (int)(p / A.N);
@@ -512,19 +505,62 @@ __global__ void __launch_bounds__(128, 4) k_assemble_kernel(KArgs A) {
     }
 }
 
-// Warp-per-pair variant of k_assemble_kernel: one warp per (triangle x,
-// vertex s), the lanes over the node pairs (star triangle of s, inner node,
-// outer node), the same per-node-pair arithmetic, a warp reduction per lag.
-__global__ void __launch_bounds__(128, 6) k_assemble_warp_kernel(KArgs A) {
+// Warp per (row triangle x, vertex s), by front arrivals (front_bins.cuh).
+// Bound by FP64 issue of the items, about 160 operations each, a quarter of them
+// lanes without an item: rule 7/4/3 on 448 triangles 1000 items a pair.  The
+// form before evaluated every node pair in every lag between its P and S
+// arrival.  Rule 7/4/3: 448 triangles, 40 lags 16.1 -> 2.9 ms, 700 triangles
+// 43 -> 7.5 ms, 2800 triangles, lags 40..49 283 -> 62 ms.  168 registers, 3
+// blocks an SM; 2 blocks without the 100 bytes of spills 3.4 ms, 4 blocks 3.7.
+//
+// Over the levels k, k + 1, k + 2 from a front's arrival on, with a = t_k - tX
+// and S_j = (a + j dt)^2 (a + j dt + 3 tX) / 6, the third difference is
+//   lag k - 1:  a A + B + S_0 C,
+//   lag k:      (dt - 2 a) A - 2 B + (S_1 - 3 S_0) C,
+//   lag k + 1:  (a - dt) A + B + (S_2 - 3 S_1 + 3 S_0) C,
+//   later:      dt^3 C,
+// with the coefficients of R, H and S of the kernel as k_pair collects them,
+// per front (sigma = 1 for P, -1 for S; M_ik = a1 x_i n_k + a2 x_k n_i):
+//   A = sigma phik ir^3 M - sigma c2 ir^3/c^2 (w x) - sigma c1 ir/c^2 u
+//       + [S] phik (x.n) ir^3 I   (the u term of P only with `fix`),
+//   B = sigma phik ir^2/c M + [S] phik (x.n) ir^2/c I,
+//   C = -sigma (3 c2 ir^5 (w x) + c2 ir^3 u).
+// Without `fix` the reference's linear u term (lin_window3) is added over all
+// node pairs in the lags below 3.
+constexpr int kKWarps = 4;
+constexpr size_t kKSmem = 200 * 1024;
+constexpr int kKNode = 12;               // x, y, z, weight, phik, -, normal, vms
+
+// inner nodes of one chunk; 73 fill kBinChunk at 7 outer nodes, and the 170 of 3
+// outer nodes would take the shared memory of a third block
+inline __host__ __device__ int k_chunk(int n_gh) { return kBinChunk / n_gh < 73 ? kBinChunk / n_gh : 73; }
+inline __host__ __device__ size_t k_warp_bytes(int n_gh, int lag0, int nlag) {
+    const size_t b = (size_t)(kKNode * k_chunk(n_gh) + 4 * n_gh + 9 * nlag + 1) / 2 * 16 +
+                     front_bins_bytes(bin_window(lag0, nlag).bins);
+    return (b + 15) / 16 * 16;
+}
+
+__global__ void __launch_bounds__(32 * kKWarps, 3) k_assemble_kernel(KArgs A) {
+    extern __shared__ __align__(16) unsigned char k_smem[];
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const double cP = A.p.cP, cS = A.p.cS, dt = A.dt;
+    const int chunk = k_chunk(A.n_gh);
+    const BinWindow win = bin_window(A.lag0, A.nlag);
+    double* nodes = reinterpret_cast<double*>(k_smem + (threadIdx.x >> 5) * k_warp_bytes(A.n_gh, A.lag0, A.nlag));
+    double* xs = nodes + kKNode * chunk;
+    double* acc = xs + 4 * A.n_gh;                     // 9 per lag
+    FrontBins B = front_bins_at(reinterpret_cast<unsigned char*>(nodes + (kKNode * chunk + 4 * A.n_gh + 9 * A.nlag + 1) / 2 * 2),
+                                win.bins);
+    const float iout = 1.0f / (float)A.n_gh;           // (t + 1/2) iout: exact quotient for t < kBinChunk
+    const double cP = A.p.cP, cS = A.p.cS, dt = A.dt, icdtP = 1 / (cP * dt), icdtS = 1 / (cS * dt);
+    const double tail = dt * dt * dt, isc = 1 / (4 * kPi * dt);
     const KCoef cd = k_coef(A.p);
-    const int per_tri = A.n_in * A.n_gh;
     for (long long p = warp; p < (long long)A.N * A.Nv; p += nwarps) {
-        const int x = (int)(p % A.N), s = (int)(p / A.N);
+        const int s = (int)((p <= 0xffffffffLL) ? (long long)((unsigned)p / (unsigned)A.N) : p / A.N);
+        const int x = (int)(p - (long long)s * A.N);
         const DirTri& X = A.tri[x];
+        // isBlockNull (kernelK.cu:234-262), distMin starting at 100 unless fixed
         double distMax = 0.0, distMin = A.fix ? 1e300 : 100.0;
         for (int a = 0; a < 3; a++) {
             const double d0 = X.V[a][0] - A.coords[3 * s], d1 = X.V[a][1] - A.coords[3 * s + 1],
@@ -533,89 +569,197 @@ __global__ void __launch_bounds__(128, 6) k_assemble_warp_kernel(KArgs A) {
             distMax = fmax(distMax, d);
             distMin = fmin(distMin, d);
         }
-        int llo = -1, lhi = -2;
-        for (int q = 0; q < A.nlag; q++) {
+        int llo = 0x7fffffff, lhi = -1;
+        for (int q = lane; q < A.nlag; q += 32) {
             const int l = A.lag0 + q;
             if (l >= A.nblocks) break;
             const bool null = ((l - 2) * A.p.cS * A.dt > distMax + A.max_len) ||
                               ((l + 1) * A.p.cP * A.dt < distMin - 2 * A.max_len);
             if (!null) {
-                if (llo < 0) llo = l;
+                llo = min(llo, l);
                 lhi = l;
             }
         }
-        if (llo < 0) continue;
-        const int e0 = A.vt_off[s], e1 = A.vt_off[s + 1];
-        const int NP = (e1 - e0) * per_tri;
-        // the node pairs' exact distance range (warp min/max): lags in which
-        // every node pair would be skipped below add nothing and are skipped
-        // by the whole warp (the null test above bounds them by vertex
-        // distances and triangle sizes only)
-        double r2min = 1e300, r2max = 0.0;
-        for (int np = lane; np < NP; np += 32) {
-            const int ee = e0 + np / per_tri, rem = np - (np / per_tri) * per_tri;
-            const int m = A.vt_tri[ee];
-            if (m == x) continue;
-            const int qi = rem / A.n_gh, o = rem - qi * A.n_gh;
-            double y[3], xo[3];
-            bary_point(y, A.inner + 3 * qi, A.tri[m].V);
-            bary_point(xo, A.outer + 3 * o, X.V);
-            const double pt[3] = {xo[0] - y[0], xo[1] - y[1], xo[2] - y[2]};
-            const double r2 = pt[0] * pt[0] + pt[1] * pt[1] + pt[2] * pt[2];
-            r2min = fmin(r2min, r2);
-            r2max = fmax(r2max, r2);
+        llo = __reduce_min_sync(0xffffffffu, llo);
+        lhi = __reduce_max_sync(0xffffffffu, lhi);
+        if (lhi < llo) continue;
+        // star triangles but x itself
+        const int e0 = A.vt_off[s], deg = A.vt_off[s + 1] - e0;
+        int own = deg;
+        for (int e = 0; e < deg; e++)
+            if (A.vt_tri[e0 + e] == x) own = e;
+        const int n_all = (deg - (own < deg)) * A.n_in;
+        __syncwarp();
+        for (int o = lane; o < A.n_gh; o += 32) {
+            bary_point(xs + 4 * o, A.outer + 3 * o, X.V);
+            xs[4 * o + 3] = A.wout[o] * X.area;
         }
-        for (int off = 16; off > 0; off >>= 1) {
-            r2min = fmin(r2min, __shfl_xor_sync(0xffffffffu, r2min, off));
-            r2max = fmax(r2max, __shfl_xor_sync(0xffffffffu, r2max, off));
-        }
-        for (int l = llo; l <= lhi; l++) {
-            const bool lin = !A.fix && l < 3;
-            const double thi = (l + 1) * dt, tlo = (l - 2) * dt;
-            const double skipP2 = lin ? 1e300 : (cP * thi) * (cP * thi) * (1 + 1e-12);
-            const double skipS2 = (l >= 3) ? (cS * tlo) * (cS * tlo) * (1 - 1e-12) : -1.0;
-            if (r2min > skipP2 || r2max < skipS2) continue;
-            double T[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-            for (int np = lane; np < NP; np += 32) {
-                const int ee = e0 + np / per_tri, rem = np - (np / per_tri) * per_tri;
-                const int m = A.vt_tri[ee];
-                if (m == x) continue;
-                const int qi = rem / A.n_gh, o = rem - qi * A.n_gh;
-                const int kv = local_index(A.tris, m, s);
+        for (int t = lane; t < 9 * A.nlag; t += 32) acc[t] = 0.0;
+        __syncwarp();
+        bool any = false;
+        for (int q0 = 0; q0 < n_all; q0 += chunk) {
+            const int nq = min(chunk, n_all - q0), n = nq * A.n_gh;
+            for (int q = lane; q < nq; q += 32) {
+                int e = (q0 + q) / A.n_in;
+                const int qi = (q0 + q) - e * A.n_in;
+                e += e >= own;
+                const int m = A.vt_tri[e0 + e], kv = local_index(A.tris, m, s) - 1;
                 const DirTri& F = A.tri[m];
-                const double g[3] = {F.M[3 * (kv - 1)], F.M[3 * (kv - 1) + 1], F.M[3 * (kv - 1) + 2]};
-                double y[3], xo[3];
-                bary_point(y, A.inner + 3 * qi, F.V);
-                bary_point(xo, A.outer + 3 * o, X.V);
-                const double pt[3] = {xo[0] - y[0], xo[1] - y[1], xo[2] - y[2]};
-                const double r2 = pt[0] * pt[0] + pt[1] * pt[1] + pt[2] * pt[2];
-                if (r2 > skipP2 || r2 < skipS2) continue;
-                const double vms[3] = {F.n[1] * g[2] - F.n[2] * g[1], F.n[2] * g[0] - F.n[0] * g[2],
-                                       F.n[0] * g[1] - F.n[1] * g[0]};
-                const double phik = F.v[kv - 1] + g[0] * y[0] + g[1] * y[1] + g[2] * y[2];
-                const double wi = A.win[qi % A.n_sing] * F.area;
-                const double r = sqrt(r2);
-                const double tP = r / cP, tS = r / cS;
-                const Win3 P = front_window3(tP, l, dt), S = front_window3(tS, l, dt);
-                const double dRPl = A.fix ? P.R : ((r - tP > 0) ? lin_window3(tP, l, dt) : 0.0);
-                const double w = (A.wout[o] * X.area) * wi;
-                double v[9];
-                k_pair(v, pt, 1.0 / r, F.n, vms, phik, P.R, S.R, P.H, S.H, dRPl, S.S - P.S, cd);
+                const double g[3] = {F.M[3 * kv], F.M[3 * kv + 1], F.M[3 * kv + 2]};
+                double* d = nodes + kKNode * q;
+                bary_point(d, A.inner + 3 * qi, F.V);
+                d[3] = A.win[qi % A.n_sing] * F.area;
+                d[4] = F.v[kv] + g[0] * d[0] + g[1] * d[1] + g[2] * d[2];
 #pragma unroll
-                for (int e = 0; e < 9; e++) T[e] += w * v[e];
+                for (int c = 0; c < 3; c++) {
+                    d[6 + c] = F.n[c];
+                    d[9 + c] = F.n[(c + 1) % 3] * g[(c + 2) % 3] - F.n[(c + 2) % 3] * g[(c + 1) % 3];
+                }
             }
-#pragma unroll
-            for (int e = 0; e < 9; e++)
-                for (int off = 16; off > 0; off >>= 1) T[e] += __shfl_xor_sync(0xffffffffu, T[e], off);
-            if (lane < 9) {
-                const int ii = lane / 3, jj = lane - 3 * ii;
-                double v = 0;
-#pragma unroll
-                for (int e = 0; e < 9; e++)
-                    if (e == lane) v = T[e];
-                double* base = A.K + (size_t)(l - A.lag0) * A.ld_lag + (3 * (size_t)s) * A.ld + 3 * (size_t)x;
-                if (fabs(v) > 1.0e-14) base[(size_t)jj * A.ld + ii] += v / (4 * kPi * dt);
+            __syncwarp();
+            bool late = false, met = false;
+            for (int t = lane; t < n; t += 32) {
+                const int q = (int)(((float)t + 0.5f) * iout), o = t - q * A.n_gh;
+                const double* d = nodes + kKNode * q;
+                const double x0 = xs[4 * o] - d[0], x1 = xs[4 * o + 1] - d[1], x2 = xs[4 * o + 2] - d[2];
+                const double r2 = x0 * x0 + x1 * x1 + x2 * x2, r = q_sqrt(r2);
+                unsigned bP = front_bin(r2, r, cP, icdtP, dt, win);
+                unsigned bS = front_bin(r2, r, cS, icdtS, dt, win);
+                if (bS == 0) bP = bS = kNoBin;                    // past both fronts before the window: the constants cancel
+                else late = late || bS == kNoBin;
+                met = met || bP != kNoBin;
+                B.bin[t] = make_ushort2((unsigned short)bP, (unsigned short)bS);
             }
+            if (!A.fix && A.lag0 < 3) {
+                for (int l = llo; l <= min(lhi, 2); l++) {
+                    double u0 = 0.0, u1 = 0.0, u2 = 0.0;
+                    for (int t = lane; t < n; t += 32) {
+                        const int q = (int)(((float)t + 0.5f) * iout), o = t - q * A.n_gh;
+                        const double* d = nodes + kKNode * q;
+                        const double x0 = xs[4 * o] - d[0], x1 = xs[4 * o + 1] - d[1], x2 = xs[4 * o + 2] - d[2];
+                        const double r = q_sqrt(x0 * x0 + x1 * x1 + x2 * x2), tP = r / cP;
+                        if (r - tP > 0) {
+                            const double f = lin_window3(tP, l, dt) * (xs[4 * o + 3] * d[3]) / r;
+                            u0 += f * d[9];
+                            u1 += f * d[10];
+                            u2 += f * d[11];
+                        }
+                    }
+                    for (int off = 16; off > 0; off >>= 1) {
+                        u0 += __shfl_xor_sync(0xffffffffu, u0, off);
+                        u1 += __shfl_xor_sync(0xffffffffu, u1, off);
+                        u2 += __shfl_xor_sync(0xffffffffu, u2, off);
+                    }
+                    if (lane == 0) {
+                        const double f = -cd.c1 * cd.icP2;
+                        double* a = acc + 9 * (l - A.lag0);
+                        a[1] += f * u2;
+                        a[2] -= f * u1;
+                        a[3] -= f * u2;
+                        a[5] += f * u0;
+                        a[6] += f * u1;
+                        a[7] -= f * u0;
+                    }
+                    any = true;
+                }
+                __syncwarp();
+            }
+            if (!__any_sync(0xffffffffu, met)) continue;            // both fronts miss the window
+            late = __any_sync(0xffffffffu, late);
+            any = true;
+            const int total = bins_sort(B, n, win.bins, lane);
+            double cur[9] = {0}, n1[9] = {0}, n2[9] = {0}, run[9] = {0};
+            double last = 0.0, last9 = 0.0;           // this lane's reduced entry and entry 33 of the lag before
+            int first = 0, idle = 0;                  // idle: bins without items up to this one
+            for (int b = 0; b < win.bins; b++) {
+                const int k = win.kbase + b - 1, l = k - 1, lastitem = B.off[b], items = lastitem - first;
+                if (items == 0 && first == 0) continue;                 // before the first arrival
+                if (l > lhi) break;
+                idle = items ? 0 : idle + 1;
+                const double early = b == 0 ? 0.0 : 1.0, tk = k * dt;   // bin 0: the constant only
+                for (int i = first + lane; i < lastitem; i += 32) {
+                    const unsigned it = B.list[i];
+                    const bool isS = it >> 31;
+                    const int t = (int)(it & 0x7fffffffu), q = (int)(((float)t + 0.5f) * iout), o = t - q * A.n_gh;
+                    const double* d = nodes + kKNode * q;
+                    const double y[3] = {xs[4 * o] - d[0], xs[4 * o + 1] - d[1], xs[4 * o + 2] - d[2]};
+                    const double nn[3] = {d[6], d[7], d[8]}, v[3] = {d[9], d[10], d[11]};
+                    const double r2 = y[0] * y[0] + y[1] * y[1] + y[2] * y[2], r = q_sqrt(r2), ir = q_rcp(r);
+                    const double w = xs[4 * o + 3] * d[3], sw = isS ? -w : w, wp = w * d[4];
+                    const double ic = isS ? cd.icS : cd.icP, ic2 = isS ? cd.icS2 : cd.icP2;
+                    const double ir2 = ir * ir, ir3 = ir2 * ir, tX = r * ic;
+                    const double mB = early * ((isS ? -wp : wp) * ir2 * ic), mA = early * ((isS ? -wp : wp) * ir3);
+                    const double xn = isS ? y[0] * nn[0] + y[1] * nn[1] + y[2] * nn[2] : 0.0;
+                    const double uC = -cd.c2 * sw * ir3, wA = early * (uC * ic2), wC = 3 * uC * ir2;
+                    const double uA = isS || A.fix ? early * (-cd.c1 * sw * ir * ic2) : 0.0;
+                    const double a0 = tk - tX, a1 = a0 + dt, a2 = a1 + dt;
+                    const double S0 = a0 * a0 * (a0 + 3 * tX) * (1.0 / 6), S1 = a1 * a1 * (a1 + 3 * tX) * (1.0 / 6),
+                                 S2 = a2 * a2 * (a2 + 3 * tX) * (1.0 / 6);
+                    const double al[3] = {a0, dt - 2 * a0, a0 - dt}, be[3] = {1.0, -2.0, 1.0};
+                    const double ga[3] = {early * (S0 - tail), early * (S1 - 3 * S0 - tail), early * (S2 - 3 * S1 + 3 * S0 - tail)};
+                    const double wx[3] = {v[1] * y[2] - v[2] * y[1], v[2] * y[0] - v[0] * y[2], v[0] * y[1] - v[1] * y[0]};
+                    double pM[3], pI[3], pW[3], pU[3];
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        pM[j] = al[j] * mA + be[j] * mB;
+                        pI[j] = -xn * pM[j];
+                        pW[j] = al[j] * wA + ga[j] * wC;
+                        pU[j] = al[j] * uA + ga[j] * uC;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; i++)
+#pragma unroll
+                        for (int c = 0; c < 3; c++) {
+                            const int e = 3 * i + c;
+                            const double M = cd.a1 * y[i] * nn[c] + cd.a2 * y[c] * nn[i], W = wx[i] * y[c];
+                            double f[3], g = tail * (wC * W);
+#pragma unroll
+                            for (int j = 0; j < 3; j++) f[j] = pM[j] * M + pW[j] * W;
+                            if (i == c) {
+#pragma unroll
+                                for (int j = 0; j < 3; j++) f[j] += pI[j];
+                            } else {
+                                const double u = (c - i + 3) % 3 == 1 ? v[(c + 1) % 3] : -v[(i + 1) % 3];
+#pragma unroll
+                                for (int j = 0; j < 3; j++) f[j] += pU[j] * u;
+                                g += tail * (uC * u);
+                            }
+                            cur[e] += f[0];
+                            n1[e] += f[1];
+                            n2[e] += f[2];
+                            if (r2 > 0) run[e] += g;                    // r = 0: both fronts here at once, no constant remains
+                        }
+                }
+                if (b > 0 && l >= A.lag0) {
+                    if (idle < 4 || l == A.lag0) {
+                        double v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e++) v[e] = cur[e] + run[e];
+                        last = warp_reduce_scatter8(v, lane);
+                        last9 = cur[8] + run[8];
+                        for (int off = 16; off > 0; off >>= 1) last9 += __shfl_xor_sync(0xffffffffu, last9, off);
+                    }
+                    double* a = acc + 9 * (l - A.lag0);
+                    if ((lane & 3) == 0) a[scatter8_entry(lane)] += last;
+                    if (lane == 1) a[8] += last9;
+                }
+                first = lastitem;
+#pragma unroll
+                for (int e = 0; e < 9; e++) {
+                    cur[e] = n1[e];
+                    n1[e] = n2[e];
+                    n2[e] = 0.0;
+                }
+                if (!late && first == total && idle > 1) break;         // every node pair is past both fronts
+            }
+            __syncwarp();
+        }
+        if (!any) continue;
+        double* base = A.K + (3 * (size_t)s) * A.ld + 3 * (size_t)x;
+        for (int t = lane; t < 9 * (lhi - llo + 1); t += 32) {
+            const int l = t / 9, e = t - 9 * l, j = e / 3, i = e - 3 * j;
+            const double v = acc[9 * (llo + l - A.lag0) + 3 * i + j];
+            if (fabs(v) > 1.0e-14) base[(size_t)(llo + l - A.lag0) * A.ld_lag + (size_t)j * A.ld + i] += v * isc;
         }
     }
 }
@@ -854,18 +998,29 @@ int launch_k_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_su
     A.ld = 3 * (size_t)m.nt;
     A.ld_lag = A.ld * 3 * (size_t)m.nv;
     const long long pairs = (long long)m.nt * m.nv;
-    // warp per pair only when the thread kernel would not fill the GPU
-    // (fewer pairs than two waves of threads; measured: bar of 448 triangles
-    // 1.08x faster, bar of 2800 triangles 1.37x slower)
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device);
-    if (n_sub * n_sing * n_gh >= EBEM_K_WARP_MIN_NODE_PAIRS && pairs < (long long)sms * EBEM_K_WARP_MAX_PAIRS_PER_SM) {
-        const long long want = (pairs + 3) / 4, cap = (long long)sms * 64;
-        k_assemble_warp_kernel<<<(unsigned)(want < cap ? want : cap), 128, 0, s>>>(A);
-    } else {
-        k_assemble_kernel<<<(unsigned)((pairs + 127) / 128), 128, 0, s>>>(A);
+    // The pair's sums per lag cost the warp kernel a fixed share: rule 3/1/1 takes
+    // it 29 ms on the 2800-triangle bar (lags 40..49) against 14 by threads, rule
+    // 3/1/3 25 against 34, 7/1/3 30 against 72.  On few pairs the threads do not
+    // fill the chip (3/1/1: 448 triangles 1.4 against 2.0 ms, 80: 0.13 against 0.60).
+    const bool byThread = n_gh * n_sub * n_sing < 6 && pairs >= 1024LL * sms;
+    if (byThread) {
+        k_assemble_thread_kernel<<<(unsigned)((pairs + 127) / 128), 128, 0, s>>>(A);
+        EBEM_CUDA_TRY(cudaGetLastError());
     }
-    EBEM_CUDA_TRY(cudaGetLastError());
+    KArgs W = A;
+    for (int l0 = 0; !byThread && l0 < nlag; l0 += kBinLags) {
+        W.lag0 = lag0 + l0;
+        W.nlag = std::min(nlag - l0, kBinLags);
+        W.K = d_K + (size_t)l0 * A.ld_lag;
+        const size_t each = k_warp_bytes(n_gh, W.lag0, W.nlag);
+        const int warps = (int)std::max<size_t>(1, std::min<size_t>(kKWarps, kKSmem / each));
+        EBEM_CUDA_TRY(cudaFuncSetAttribute(k_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(warps * each)));
+        const long long want = (pairs + warps - 1) / warps, cap = (long long)sms * 64;
+        k_assemble_kernel<<<(unsigned)(want < cap ? want : cap), 32 * warps, warps * each, s>>>(W);
+        EBEM_CUDA_TRY(cudaGetLastError());
+    }
     if (n_diag > 0) {
         const int kmin = std::max(1, lag0 - 2), nk = lag0 + nlag - kmin + 1;
         double* Tb = nullptr;

@@ -1,4 +1,4 @@
-"""Numerical-inner assembly by front arrivals: lag windows, rules beyond one
+"""Numerical-inner assemblies (E and K) by front arrivals: lag windows, rules beyond one
 chunk of node pairs, more lags than one launch takes, and the kernel of few
 node pairs, against the oracle's evaluation lag by lag."""
 import numpy as np
@@ -37,3 +37,31 @@ def test_ghc_front_bins(oracle, refine, rule, nT, lag0, nlag):
     Eo = oracle.assemble_ghc(m, prm, *rule, lag0, nlag)
     assert np.abs(Eo).max() > 0
     assert np.abs(E - Eo).max() <= TOL * np.abs(Eo).max()
+
+
+@pytest.mark.parametrize("refine,rule,fix,T,nT,lag0,nlag", [
+    (1, (3, 1, 1), False, 1, 20, 0, 6),            # 3 node pairs a triangle: one partly filled warp
+    (1, (3, 64, 3), False, 1, 20, 0, 21),          # chunks of 73 inner nodes
+    (1, (19, 4, 12), True, 1, 20, 0, 21),          # 26 inner nodes a chunk
+    (1, (7, 4, 3), False, 1, 20, 2, 1),            # one lag, with the linear term
+    (1, (12, 4, 3), True, 1, 100, 30, 9),          # window that starts between the fronts
+    (0, (7, 4, 3), False, 0.4, 600, 0, 530),       # two launches
+    (3, (3, 1, 1), False, 1, 20, 1, 4),            # thread per pair
+])
+def test_k_front_bins(oracle, refine, rule, fix, T, nT, lag0, nlag):
+    if not cuda_available():
+        pytest.skip("no CUDA device")
+    import elastodynamicebem_b200.core as core
+    from elastodynamicebem_b200 import mesh, problem
+    m = mesh.icosphere(refine)
+    x = m.coordinates + np.random.default_rng(3).uniform(-0.02, 0.02, m.coordinates.shape) * m.lMin
+    m = mesh.Mesh(x, m.triangles)
+    prm = problem.ProblemParams(1, 1, 1, T, nT)
+    dm = core.DeviceMesh(m)
+    LK = core.num_blocks_dir(dm, prm)[1]
+    K = core.assemble_k(dm, prm, *rule, 0, lag0, nlag, fix=fix).cpu().numpy()
+    Ko = oracle.assemble_k(m, prm, *rule, lag0, nlag, nblocks=LK, fix=fix)
+    # the oracle's third differences of levels that grow like (t / dt)^3
+    tol = TOL + 1e-15 * (lag0 + nlag) ** 3
+    assert np.abs(Ko).max() > 0
+    assert np.abs(K - Ko).max() <= tol * np.abs(Ko).max()
