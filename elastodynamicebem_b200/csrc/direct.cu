@@ -260,30 +260,6 @@ __device__ __forceinline__ void kern_v(double nu[9], const double x[3], double r
         }
 }
 
-// Traction kernel of kernelP.cu times phik, x = source - node.
-__device__ void kern_p(double nu[9], const double x[3], const double n[3], double r, double t, double phik,
-                       const Mat& p) {
-    const TimeF f = time_f(r, t, p);
-    const double xn = x[0] * n[0] + x[1] * n[1] + x[2] * n[2];
-    const double ir = 1.0 / r, ir2 = ir * ir, ir3 = ir2 * ir, ir4 = ir2 * ir2, ir5 = ir4 * ir, ir7 = ir5 * ir2;
-    const double lam = p.lam, mu = p.mu;
-    const double fP3 = f.HP / (p.cP * p.cP * p.cP), fS3 = f.HS / (p.cS * p.cS * p.cS);
-    const double fP2 = f.RP / (p.cP * p.cP), fS2 = f.RS / (p.cS * p.cS), fH = f.SP - f.SS;
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            const double d = (i == j) ? 1.0 : 0.0;
-            const double a = x[i] * n[j], b = x[j] * n[i], xx = x[j] * x[i];
-            const double v = (lam * a * ir2 + 2 * mu * xx * ir4 * xn) * fP3 +
-                             mu * (b * ir2 + (d * ir2 - 2 * xx * ir4) * xn) * fS3 +
-                             ((lam - 2 * mu) * a * ir3 - 2 * mu * b * ir3 - 2 * mu * (d * ir3 - 6 * xx * ir5) * xn) * fP2 +
-                             mu * (2 * a * ir3 + 3 * b * ir3 + 3 * (d * ir3 - 4 * xx * ir5) * xn) * fS2 -
-                             6 * mu * (a * ir5 + b * ir5 + (d * ir5 - 5 * xx * ir7) * xn) * fH;
-            nu[3 * i + j] = v * phik;
-        }
-}
-
 __device__ __forceinline__ void bary_point(double y[3], const double* b, const double V[3][3]) {
 #pragma unroll
     for (int c = 0; c < 3; c++) y[c] = b[0] * V[0][c] + b[1] * V[1][c] + b[2] * V[2][c];
@@ -1164,73 +1140,194 @@ __global__ void __launch_bounds__(128, 4) pp_g_kernel(PPArgs A, int kchunk) {
 }
 
 // P part: minus the sum over slices n of clamp(P_{n-1} - 2 P_n + P_{n+1}) / (4 pi rho dt) b_n.
-// Chunked over the slices as pp_g_kernel; a chunk evaluates P at the levels
-// n_lo - 1 .. n_hi + 1.
-__global__ void __launch_bounds__(128, 4) pp_p_kernel(PPArgs A, int kchunk) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ev = blockIdx.y;
-    const int q = ev / A.npts, ip = ev % A.npts;
-    const double t = A.times[q];
-    const double* src = A.pts + 3 * ip;
-    const int nhat = (t > 0) ? (int)ceil(t / A.dt) : 0;
-    const int n_lo = blockIdx.z * kchunk + 1, n_hi = min((int)(blockIdx.z + 1) * kchunk, nhat);
-    double u0 = 0.0, u1 = 0.0, u2 = 0.0;
-    if (s < A.Nv && n_lo <= n_hi) {
-        double Pm2[9] = {0}, Pm1[9] = {0}, Pk[9];
-        const double c4 = 4 * kPi * A.p.rho * A.dt;
-        const int e0 = A.vt_off[s], e1 = A.vt_off[s + 1];
-        for (int k = n_lo - 1; k <= n_hi + 1; k++) {
-            const double tk = t - k * A.dt;
-#pragma unroll
-            for (int e = 0; e < 9; e++) Pk[e] = 0.0;
-            if (tk > 0) {
-                for (int ee = e0; ee < e1; ee++) {
-                    const int m = A.vt_tri[ee];
-                    const int kv = local_index(A.tris, m, s);
-                    const DirTri& F = A.tri[m];
-                    const double* g = F.M + 3 * (kv - 1);
-                    for (int tx = 0; tx < A.n_sub; tx++)
-                        for (int l = 0; l < A.n_sing; l++) {
-                            double y[3];
-                            bary_point(y, A.pn + 3 * (A.n_sing * tx + l), F.V);
-                            const double pt[3] = {src[0] - y[0], src[1] - y[1], src[2] - y[2]};
-                            const double phik = F.v[kv - 1] + g[0] * y[0] + g[1] * y[1] + g[2] * y[2];
-                            double nu[9];
-                            kern_p(nu, pt, F.n, sqrt(pt[0] * pt[0] + pt[1] * pt[1] + pt[2] * pt[2]), tk, phik, A.p);
-                            const double w = A.pw[l] * F.area;
-#pragma unroll
-                            for (int e = 0; e < 9; e++) Pk[e] += w * nu[e];
-                        }
-                }
-            }
-            if (k >= n_lo + 1) {
-                const int n = k - 1;                    // slice n: P_{n-1} - 2 P_n + P_{n+1}
-                double S[9];
-#pragma unroll
-                for (int e = 0; e < 9; e++) {
-                    const double v = (Pm2[e] - 2 * Pm1[e]) + Pk[e];
-                    S[e] = (fabs(v) > 1.0e-14) ? v / c4 : 0.0;
-                }
-                if (n <= nhat) {
-                    if (A.mode == 1) {
-                        const size_t R = 3 * (size_t)nhat;
-#pragma unroll
-                        for (int i = 0; i < 3; i++)
-#pragma unroll
-                            for (int j = 0; j < 3; j++) A.Pm[(3 * (size_t)s + j) * R + 3 * (size_t)(n - 1) + i] = S[3 * i + j];
-                    } else if (n <= A.nT) {
-                        const double* bn = A.b + (size_t)(n - 1) * 3 * A.Nv + 3 * (size_t)s;
-                        u0 -= S[0] * bn[0] + S[1] * bn[1] + S[2] * bn[2];
-                        u1 -= S[3] * bn[0] + S[4] * bn[1] + S[5] * bn[2];
-                        u2 -= S[6] * bn[0] + S[7] * bn[1] + S[8] * bn[2];
-                    }
-                }
-            }
-#pragma unroll
-            for (int e = 0; e < 9; e++) { Pm2[e] = Pm1[e]; Pm1[e] = Pk[e]; }
+//
+// Warp per (evaluation, vertex, chunk of slices), by front arrivals
+// (front_bins.cuh) in the levels j = nhat + 1 - k, ascending in time: slice n has
+// the centre c = nhat + 1 - n and takes the levels c - 1, c, c + 1.  With a the
+// time since the arrival at the first level k of a front and S_j = (a + j dt)^2
+// (a + j dt + 3 tX) / 6, its second difference is
+//   centre k - 1:  H + a R + S_0 S,   centre k:  -H + (dt - a) R + (S_1 - 2 S_0) S,
+//   later:         dt^2 t_c S,
+// H, R, S the coefficients of the front's time functions in the traction kernel
+// of kernelP.cu times phik, x = source - node, xn = x . n, in x_i n_j, x_j n_i,
+// xn delta_ij, xn x_i x_j:
+//   P:  H  (lam, 0, 0, 2 mu ir^2) ir^2 / c_P^3,  S: H  mu (0, 1, 1, -2 ir^2) ir^2 / c_S^3,
+//       R  (lam - 2 mu, -2 mu, -2 mu, 12 mu ir^2) ir^3 / c_P^2,
+//                                                  R  mu (2, 3, 3, -12 ir^2) ir^3 / c_S^2,
+//       S  mu (-6, -6, -6, 30 ir^2) ir^5,          S  minus P's.
+// Evaluating the kernel at every level (thread per vertex) was bound by FP64 latency, most of
+// it at levels past both fronts, where the second difference vanishes: 16 points
+// x 4 times on the 448-triangle bar 2.62 -> 0.17 ms.
+constexpr int kPPWarps = 4, kPPSlices = 64, kPPNodes = 128, kPPNode = 8;
+
+inline __host__ __device__ size_t pp_warp_bytes() {
+    return (size_t)(kPPNode * kPPNodes + 9 * kPPSlices) * sizeof(double) + (front_bins_bytes(kPPSlices + 3) + 15) / 16 * 16;
+}
+
+// Bin (bin_window(c0, .) of the centres from c0 on) of the first level j with
+// t_k - r / c > 0, t_k = t - k dt, k = nhat + 1 - j, as the reference tests it.
+__device__ __forceinline__ unsigned pp_front_bin(double r2, double r, double c, double ic, double t, double dt, double idt,
+                                                 int nhat, const BinWindow& w) {
+    const double g = (t - r * ic) * idt;               // levels k < g are past the arrival
+    if (!(g > -1.0)) return kNoBin;
+    int k = (int)ceil(g) - 1;
+    if (fabs(g - rint(g)) <= 1e-9 * (t * idt) + 1e-12) {
+        const double tX = sqrt(r2) / c;
+        for (k += 3; k >= 0; k--) {
+            const double tk = t - k * dt;
+            if (tk - tX > 0) break;
         }
     }
-    if (A.mode == 0) warp_add3(A.u + 3 * (size_t)ev, u0, u1, u2);
+    if (k < 0) return kNoBin;
+    const int j = nhat + 1 - k;
+    return j > w.kbase + w.bins - 2 ? kNoBin : j < w.kbase ? 0u : (unsigned)(j - w.kbase + 1);
+}
+
+__global__ void __launch_bounds__(32 * kPPWarps, 3) pp_p_kernel(PPArgs A, int nz) {
+    extern __shared__ __align__(16) unsigned char pp_smem[];
+    const int lane = threadIdx.x & 31;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    double* nodes = reinterpret_cast<double*>(pp_smem + (threadIdx.x >> 5) * pp_warp_bytes());
+    double* acc = nodes + kPPNode * kPPNodes;          // 9 per centre
+    FrontBins B = front_bins_at(reinterpret_cast<unsigned char*>(acc + 9 * kPPSlices), kPPSlices + 3);
+    const double cP = A.p.cP, cS = A.p.cS, icP = 1 / cP, icS = 1 / cS, dt = A.dt, idt = 1 / dt, dt2 = dt * dt;
+    const double lam = A.p.lam, mu = A.p.mu, ic4 = 1 / (4 * kPi * A.p.rho * A.dt);
+    const int n_in = A.n_sub * A.n_sing;
+    for (long long w0 = warp; w0 < (long long)A.npts * A.ntimes * A.Nv * nz; w0 += nwarps) {
+        const int z = (int)(w0 % nz), s = (int)(w0 / nz % A.Nv), ev = (int)(w0 / nz / A.Nv);
+        const int q = ev / A.npts, ip = ev % A.npts;
+        const double t = A.times[q];
+        const double src[3] = {A.pts[3 * ip], A.pts[3 * ip + 1], A.pts[3 * ip + 2]};
+        const int nhat = (t > 0) ? (int)ceil(t / A.dt) : 0;
+        const int c0 = z * kPPSlices + 1, nc = min(kPPSlices, nhat + 1 - c0);      // centres c0 .. c0 + nc - 1
+        if (nc <= 0) continue;
+        const BinWindow win = bin_window(c0, nc);
+        const int e0 = A.vt_off[s], n_all = (A.vt_off[s + 1] - e0) * n_in;
+        __syncwarp();
+        for (int i = lane; i < 9 * nc; i += 32) acc[i] = 0.0;
+        for (int q0 = 0; q0 < n_all; q0 += kPPNodes) {
+            const int n = min(kPPNodes, n_all - q0);
+            bool met = false, late = false;
+            __syncwarp();
+            for (int i = lane; i < n; i += 32) {
+                const int e = (q0 + i) / n_in, qi = (q0 + i) - e * n_in;
+                const int m = A.vt_tri[e0 + e], kv = local_index(A.tris, m, s) - 1;
+                const DirTri& F = A.tri[m];
+                double y[3], *d = nodes + kPPNode * i;
+                bary_point(y, A.pn + 3 * qi, F.V);
+                const double phik = F.v[kv] + F.M[3 * kv] * y[0] + F.M[3 * kv + 1] * y[1] + F.M[3 * kv + 2] * y[2];
+                double r2 = 0.0;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    d[c] = src[c] - y[c];
+                    d[3 + c] = F.n[c];
+                }
+                d[6] = A.pw[qi % A.n_sing] * F.area * phik;
+                r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+                const double r = q_sqrt(r2);
+                unsigned bP = pp_front_bin(r2, r, cP, icP, t, dt, idt, nhat, win);
+                unsigned bS = pp_front_bin(r2, r, cS, icS, t, dt, idt, nhat, win);
+                if (bS == 0 && r2 > 0) bP = bS = kNoBin;          // past both fronts before the window: nothing left
+                else late = late || bS == kNoBin;
+                met = met || bP != kNoBin;
+                B.bin[i] = make_ushort2((unsigned short)bP, (unsigned short)bS);
+            }
+            if (!__any_sync(0xffffffffu, met)) continue;
+            late = __any_sync(0xffffffffu, late);
+            const int total = bins_sort(B, n, win.bins, lane);
+            double cur[9] = {0}, nxt[9] = {0}, run[9] = {0};
+            double last = 0.0, last9 = 0.0;           // this lane's reduced entry and entry 33 of run
+            int first = 0, idle = 0;                  // idle: bins without items up to this one
+            for (int b = 0; b < win.bins; b++) {
+                const int k = win.kbase + b - 1, c = k - 1, lastitem = B.off[b], items = lastitem - first;
+                if (items == 0 && first == 0) continue;                 // before the first arrival
+                if (c >= c0 + nc) break;
+                idle = items ? 0 : idle + 1;
+                const double early = b == 0 ? 0.0 : 1.0;                // bin 0: the linear part only
+                const double tk = t - (nhat + 1 - k) * dt, tc = t - (nhat + 1 - c) * dt;
+                const double f1 = dt2 * tc, f2 = dt2 * tk;
+                for (int i = first + lane; i < lastitem; i += 32) {
+                    const unsigned it = B.list[i];
+                    const bool isS = it >> 31;
+                    const double* d = nodes + kPPNode * (int)(it & 0x7fffffffu);
+                    const double x[3] = {d[0], d[1], d[2]}, nn[3] = {d[3], d[4], d[5]}, w = d[6];
+                    const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2], r = q_sqrt(r2), ir = q_rcp(r);
+                    const double xn = x[0] * nn[0] + x[1] * nn[1] + x[2] * nn[2];
+                    const double ic = isS ? icS : icP, tX = r * ic, ir2 = ir * ir;
+                    const double h = early * (w * ic * ic * ic * ir2), g = early * (w * ic * ic * ir2 * ir);
+                    // coefficients of x_i n_j, x_j n_i, xn delta_ij, xn x_i x_j
+                    const double H[4] = {isS ? 0.0 : lam * h, isS ? mu * h : 0.0, isS ? mu * h : 0.0,
+                                         (isS ? -2 * mu : 2 * mu) * h * ir2};
+                    const double R[4] = {(isS ? 2 * mu : lam - 2 * mu) * g, (isS ? 3 * mu : -2 * mu) * g,
+                                         (isS ? 3 * mu : -2 * mu) * g, (isS ? -12 * mu : 12 * mu) * g * ir2};
+                    const double sc = (isS ? 6 * mu : -6 * mu) * w * ir2 * ir2 * ir, sx = -5 * sc * ir2;
+                    const double a0 = tk - tX, a1 = a0 + dt;
+                    const double S0 = a0 * a0 * (a0 + 3 * tX) * (1.0 / 6), S1 = a1 * a1 * (a1 + 3 * tX) * (1.0 / 6);
+                    const double g1 = early * (S0 - f1), g2 = early * (S1 - 2 * S0 - f2);
+                    double p1[4], p2[4];
+#pragma unroll
+                    for (int m = 0; m < 4; m++) {
+                        const double sm = m == 3 ? sx : sc;
+                        p1[m] = H[m] + a0 * R[m] + g1 * sm;
+                        p2[m] = (dt - a0) * R[m] - H[m] + g2 * sm;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; i++)
+#pragma unroll
+                        for (int j = 0; j < 3; j++) {
+                            const double a = x[i] * nn[j], bb = x[j] * nn[i], xx = xn * x[i] * x[j], dd = i == j ? xn : 0.0;
+                            cur[3 * i + j] += p1[0] * a + p1[1] * bb + p1[2] * dd + p1[3] * xx;
+                            nxt[3 * i + j] += p2[0] * a + p2[1] * bb + p2[2] * dd + p2[3] * xx;
+                            run[3 * i + j] += sc * (a + bb + dd) + sx * xx;
+                        }
+                }
+                if (b > 0 && c >= c0) {
+                    // idle: run is the sum of the slice before, and all there is from the third slice on
+                    const bool all = idle < 2;
+                    if (all || idle == 2 || c == c0) {
+                        double v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e++) v[e] = all ? cur[e] + f1 * run[e] : run[e];
+                        last = warp_reduce_scatter8(v, lane);
+                        last9 = all ? cur[8] + f1 * run[8] : run[8];
+                        for (int off = 16; off > 0; off >>= 1) last9 += __shfl_xor_sync(0xffffffffu, last9, off);
+                    }
+                    double* a = acc + 9 * (c - c0);
+                    if ((lane & 3) == 0) a[scatter8_entry(lane)] += all ? last : f1 * last;
+                    if (lane == 1) a[8] += all ? last9 : f1 * last9;
+                }
+                first = lastitem;
+#pragma unroll
+                for (int e = 0; e < 9; e++) {
+                    cur[e] = nxt[e];
+                    nxt[e] = 0.0;
+                }
+                if (!late && first == total && items == 0) break;       // every node is past both fronts
+            }
+        }
+        __syncwarp();
+        double u[3] = {0.0, 0.0, 0.0};
+        for (int i = lane; i < 3 * nc; i += 32) {      // column j of slice n
+            const int c = i / 3, j = i - 3 * c, n = nhat + 1 - (c0 + c);
+            double S[3];
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const double v = acc[9 * c + 3 * r + j];
+                S[r] = (fabs(v) > 1.0e-14) ? v * ic4 : 0.0;
+            }
+            if (A.mode == 1) {
+                const size_t R = 3 * (size_t)nhat;
+#pragma unroll
+                for (int r = 0; r < 3; r++) A.Pm[(3 * (size_t)s + j) * R + 3 * (size_t)(n - 1) + r] = S[r];
+            } else if (n <= A.nT) {
+                const double bn = A.b[(size_t)(n - 1) * 3 * A.Nv + 3 * (size_t)s + j];
+#pragma unroll
+                for (int r = 0; r < 3; r++) u[r] -= S[r] * bn;
+            }
+        }
+        if (A.mode == 0) warp_add3(A.u + 3 * (size_t)ev, u[0], u[1], u[2]);
+    }
 }
 
 int launch_pp_dir(const MeshData& m, const PhysParams& P, int n_sub, int n_sing, int fix, const double* d_pts, int npts,
@@ -1273,8 +1370,8 @@ int launch_pp_dir(const MeshData& m, const PhysParams& P, int n_sub, int n_sing,
     A.mode = mode;
     if (e == cudaSuccess) {
         // slices split into chunks over grid z so that about 8 blocks per SM
-        // run (a chunk re-evaluates 1 (G) or 2 (P) boundary levels: at least
-        // 4 and 8 slices per chunk keep that under a quarter)
+        // run (G; a chunk re-evaluates 1 boundary level: at least 4 slices
+        // per chunk keep that under a quarter)
         int nhat_max = 0;
         for (int q = 0; q < ntimes; q++)
             if (h_times[q] > 0) nhat_max = std::max(nhat_max, (int)std::ceil(h_times[q] / P.dt));
@@ -1286,15 +1383,19 @@ int launch_pp_dir(const MeshData& m, const PhysParams& P, int n_sub, int n_sing,
             const long long want = (nhat_max * bxy + target - 1) / target;
             return (int)std::min<long long>(nhat_max, std::max<long long>(kmin, want));
         };
-        const long long bg = (m.nt + 127) / 128, bp = (m.nv + 127) / 128;
-        const int kg = chunk_of(bg * evs, 4), kp = chunk_of(bp * evs, 8);
+        const long long bg = (m.nt + 127) / 128;
+        const int kg = chunk_of(bg * evs, 4), nz = (nhat_max + kPPSlices - 1) / kPPSlices;
         dim3 gg((unsigned)bg, (unsigned)evs, (unsigned)((nhat_max + kg - 1) / kg));
-        dim3 gp((unsigned)bp, (unsigned)evs, (unsigned)((nhat_max + kp - 1) / kp));
+        const long long gp = std::min<long long>((evs * m.nv * nz + kPPWarps - 1) / kPPWarps, 64LL * sms);
         if (mode == 0) e = cudaMemsetAsync(d_u, 0, sizeof(double) * 3 * (size_t)npts * ntimes, s);
         if (e == cudaSuccess) {
             pp_g_kernel<<<gg, 128, 0, s>>>(A, kg);
-            pp_p_kernel<<<gp, 128, 0, s>>>(A, kp);
-            e = cudaGetLastError();
+            const size_t smem = kPPWarps * pp_warp_bytes();
+            e = cudaFuncSetAttribute(pp_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e == cudaSuccess) {
+                pp_p_kernel<<<(unsigned)gp, 32 * kPPWarps, smem, s>>>(A, nz);
+                e = cudaGetLastError();
+            }
         }
     }
     ws_free(d_times, s);
