@@ -16,10 +16,11 @@
 //
 // The marching (BEMenerg_coreGPU_timeMarching.m:151-169) is unchanged in
 // arithmetic content: E_0 is expanded to a dense matrix and factorised once
-// (cuSOLVER getrf); step n forms b_n - sum_{l=1}^{min(n, L-1)} E_l phi_{n-l}
+// (inverted); step n forms b_n - sum_{l=1}^{min(n, L-1)} E_l phi_{n-l}
 // with band_hist_kernel (warps over ranges of a source row's pairs, lanes
 // over the (pair, lag) blocks of 32 pairs at a time, the past densities stored
-// time-contiguous per field triangle) and solves with the LU factors.
+// time-contiguous per field triangle), what the steps before a block of 8
+// contribute to its steps in one pass, and multiplies by the inverse.
 #include "ebem_internal.h"
 #include "sa_pair.cuh"
 
@@ -193,8 +194,12 @@ int band_to_dense(const BandOp& op, int lag0, int nlag, double* d_E, cudaStream_
 // ---------------------------------------------------------------------------
 // marching
 
-// y[3i + c] -= sum_j sum_{l = max(lo,1)}^{min(hi, n)} (E_l)_{ij} phi_{n-l, j}:
-// each source row i is split into `split` ranges of its pairs, one warp per
+// Steps n .. n + B - 1: y_{n+b}[3i + c] -= sum_j sum_l (E_l)_{ij} phi_{n+b-l, j}
+// over the steps t0 <= n + b - l < t1 and l >= 1 (y: ldy apart).  Bound by reading
+// the band: with B = 8 a pass over it serves 8 steps (480 triangles, 64 steps:
+// 3.3 -> 1.05 ms, and 0.5 for the lags inside the blocks with B = 1; the
+// densities, 24 loads a band block, come from L1).
+// Each source row i is split into `split` ranges of its pairs, one warp per
 // range, added into y with one atomic per component (the order of those
 // additions varies from run to run, as in the dense history product).  The
 // pairs of a range are taken 32 at a time:
@@ -203,9 +208,11 @@ int band_to_dense(const BandOp& op, int lag0, int nlag, double* d_E, cudaStream_
 // run over those blocks (consecutive lanes read consecutive blocks of the
 // band storage), each finding its pair by a binary search over the scanned
 // counts.  phiT[(j nT + t) 3 + c].
+template <int B>
 __global__ void __launch_bounds__(256) band_hist_kernel(const double* __restrict__ Eb, const long long* __restrict__ off,
-                                                        const int* __restrict__ lo, int N, int split, int n, int nT,
-                                                        const double* __restrict__ phiT, double* __restrict__ y) {
+                                                        const int* __restrict__ lo, int N, int split, int n, int t0, int t1,
+                                                        int nT, const double* __restrict__ phiT, double* __restrict__ y,
+                                                        int ldy) {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -214,7 +221,9 @@ __global__ void __launch_bounds__(256) band_hist_kernel(const double* __restrict
         const long long i = w / split;
         const int part = (int)(w - i * split);
         const int jb0 = 32 * (int)((long long)nchunk * part / split), jb1 = 32 * (int)((long long)nchunk * (part + 1) / split);
-        double a0 = 0, a1 = 0, a2 = 0;
+        double a[3 * B];
+#pragma unroll
+        for (int e = 0; e < 3 * B; e++) a[e] = 0.0;
         for (int jb = jb0; jb < jb1; jb += 32) {
             const int jl = jb + lane;
             long long first = 0;          // block index of the pair's first active lag
@@ -223,8 +232,8 @@ __global__ void __launch_bounds__(256) band_hist_kernel(const double* __restrict
                 const long long p = i * N + jl;
                 const long long b0 = off[p];
                 const int len = (int)(off[p + 1] - b0), l0 = lo[p];
-                ls = max(l0, 1);
-                const int le = min(l0 + len - 1, n);
+                ls = max(l0, max(1, n - t1 + 1));
+                const int le = min(l0 + len - 1, n + B - 1 - t0);
                 cnt = max(0, le - ls + 1);
                 first = b0 + (ls - l0);
             }
@@ -235,8 +244,8 @@ __global__ void __launch_bounds__(256) band_hist_kernel(const double* __restrict
                 if (lane >= o) incl += v;
             }
             const int total = __shfl_sync(0xffffffffu, incl, 31);
-            for (int t0 = 0; t0 < total; t0 += 32) {      // uniform over the warp: full-mask shuffles
-                const int t = t0 + lane;
+            for (int k0 = 0; k0 < total; k0 += 32) {      // uniform over the warp: full-mask shuffles
+                const int t = k0 + lane;
                 int q = 0;                // first lane whose inclusive count exceeds t (31 when t >= total)
 #pragma unroll
                 for (int step = 16; step > 0; step >>= 1) {
@@ -248,23 +257,24 @@ __global__ void __launch_bounds__(256) band_hist_kernel(const double* __restrict
                 const int lsq = __shfl_sync(0xffffffffu, ls, q);
                 if (t >= total) continue;
                 const int k = t - excl, l = lsq + k;
-                const double* B = Eb + (fq + k) * 6;
-                const double* ph = phiT + ((size_t)(jb + q) * nT + (n - l)) * 3;
-                const double p0 = ph[0], p1 = ph[1], p2 = ph[2];
-                a0 += B[0] * p0 + B[1] * p1 + B[2] * p2;
-                a1 += B[1] * p0 + B[3] * p1 + B[4] * p2;
-                a2 += B[2] * p0 + B[4] * p1 + B[5] * p2;
+                const double* e = Eb + (fq + k) * 6;
+                const double e0 = e[0], e1 = e[1], e2 = e[2], e3 = e[3], e4 = e[4], e5 = e[5];
+                const double* ph = phiT + ((long long)(jb + q) * nT + (n - l)) * 3;
+#pragma unroll
+                for (int b = 0; b < B; b++) {
+                    const int step = n + b - l;
+                    if (step < t0 || step >= t1) continue;
+                    const double p0 = ph[3 * b], p1 = ph[3 * b + 1], p2 = ph[3 * b + 2];
+                    a[3 * b] += e0 * p0 + e1 * p1 + e2 * p2;
+                    a[3 * b + 1] += e1 * p0 + e3 * p1 + e4 * p2;
+                    a[3 * b + 2] += e2 * p0 + e4 * p1 + e5 * p2;
+                }
             }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-        }
-        if (lane == 0 && (a0 != 0.0 || a1 != 0.0 || a2 != 0.0)) {
-            atomicAdd(y + 3 * i, -a0);
-            atomicAdd(y + 3 * i + 1, -a1);
-            atomicAdd(y + 3 * i + 2, -a2);
+#pragma unroll
+        for (int e = 0; e < 3 * B; e++) {
+            for (int o = 16; o > 0; o >>= 1) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
+            if (lane == 0 && a[e] != 0.0) atomicAdd(y + (size_t)(e / 3) * ldy + 3 * i + e % 3, -a[e]);
         }
     }
 }
@@ -294,15 +304,16 @@ __global__ void phi_to_time_major_kernel(const double* __restrict__ y, int N, in
 int band_march(const BandOp& op, const double* d_rhs, int nT, double* d_phi, cudaStream_t s) {
     const int N = op.N, n3 = 3 * N;
     double* E0 = nullptr;
-    double* phiT = nullptr;
+    double *phiT = nullptr, *Y = nullptr;
     LuPlan lu;
     int rc = EBEM_OK;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long NN = (long long)N * N;
+    const size_t tot = (size_t)n3 * nT * sizeof(double);
     if (ws_malloc(&E0, (size_t)n3 * n3 * sizeof(double), s) != cudaSuccess ||
-        ws_malloc(&phiT, (size_t)n3 * nT * sizeof(double), s) != cudaSuccess) {
+        ws_malloc(&phiT, 2 * tot, s) != cudaSuccess) {
         ws_free(E0, s);
         return fail(EBEM_ERR_NOMEM, "banded marching workspace allocation failed");
     }
@@ -316,20 +327,31 @@ int band_march(const BandOp& op, const double* d_rhs, int nT, double* d_phi, cud
     const int nchunk = (N + 31) / 32;
     const int split = (int)std::max<long long>(1, std::min<long long>(nchunk, ((long long)sms * 48 + N - 1) / N));
     const int hist_blocks = (int)std::min<long long>(((long long)N * split + 7) / 8, (long long)sms * 8);
+    // Y: right-hand sides (copied first: d_phi may be d_rhs).  Steps in blocks of
+    // kHistBlock, the lags inside the block step by step.
+    Y = phiT + (size_t)n3 * nT;
+    if (!rc && (cudaMemcpyAsync(Y, d_rhs, tot, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+                cudaMemsetAsync(d_phi, 0, tot, s) != cudaSuccess))
+        rc = fail(EBEM_ERR_CUDA, "right-hand side copy failed");
     for (int n = 0; n < nT && !rc; n++) {
-        double* y = d_phi + (size_t)n * n3;
-        if (cudaMemcpyAsync(y, d_rhs + (size_t)n * n3, (size_t)n3 * sizeof(double), cudaMemcpyDeviceToDevice, s) !=
-            cudaSuccess) {
-            rc = fail(EBEM_ERR_CUDA, "right-hand side copy failed");
-            break;
+        double *y = Y + (size_t)n * n3, *phi = d_phi + (size_t)n * n3;
+        const int n0 = n - n % kHistBlock;
+        if (op.L > 1 && n == n0 && n > 0) {
+            if (nT - n >= kHistBlock)
+                band_hist_kernel<kHistBlock><<<hist_blocks, 256, 0, s>>>(op.Eb, op.off, op.lo, N, split, n, 0, n, nT, phiT, y, n3);
+            else
+                for (int m = n; m < nT; m++)
+                    band_hist_kernel<1><<<hist_blocks, 256, 0, s>>>(op.Eb, op.off, op.lo, N, split, m, 0, n, nT, phiT,
+                                                                    Y + (size_t)m * n3, n3);
+        } else if (op.L > 1 && n > n0) {
+            band_hist_kernel<1><<<hist_blocks, 256, 0, s>>>(op.Eb, op.off, op.lo, N, split, n, n0, n, nT, phiT, y, n3);
         }
-        if (n > 0 && op.L > 1) band_hist_kernel<<<hist_blocks, 256, 0, s>>>(op.Eb, op.off, op.lo, N, split, n, nT, phiT, y);
         if (cudaGetLastError() != cudaSuccess) {
             rc = fail(EBEM_ERR_CUDA, "banded history failed");
             break;
         }
-        if ((rc = lu_plan_solve(&lu, y, 1, s))) break;
-        phi_to_time_major_kernel<<<(n3 + 255) / 256, 256, 0, s>>>(y, N, n, nT, phiT);
+        if ((rc = launch_gemv_add(lu.inv, n3, n3, y, phi, sms, s))) break;
+        phi_to_time_major_kernel<<<(n3 + 255) / 256, 256, 0, s>>>(phi, N, n, nT, phiT);
     }
     if (!rc && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(EBEM_ERR_CUDA, "banded marching failed");
     lu_plan_destroy(&lu);
