@@ -62,9 +62,13 @@ __device__ __forceinline__ void lame_kernel(double out[6], const double x[3], do
 
 }  // namespace
 
-// M for one (point, distinct instant, triangle) per thread; triangle fastest.
+// M for one (point, distinct instant, triangle) per LANES lanes; triangle fastest.
 // At most 80 registers (6 blocks of 128 threads per SM; 116 without the
 // cap): 64 points at one time on the 320-triangle sphere 0.39 -> 0.36 ms.
+// 8 lanes share the rule's nodes where one thread each leaves the SMs with a
+// warp or less per scheduler, bound by the chain of one node's roots and
+// quotients: 1 point, 40 instants, 320 triangles, 48 nodes 59 -> 22 us.
+template <int LANES>
 __global__ void __launch_bounds__(128, 6) pp_num_level_kernel(const double* __restrict__ coords,
                                                            const int32_t* __restrict__ tris,
                                                            const TriGeom* __restrict__ geo, int N,
@@ -78,8 +82,12 @@ __global__ void __launch_bounds__(128, 6) pp_num_level_kernel(const double* __re
     const int nn = n_sub * n_sing;
     for (int q = threadIdx.x; q < 3 * nn + n_sing; q += blockDim.x) sh[q] = (q < 3 * nn) ? nodes[q] : w[q - 3 * nn];
     __syncthreads();
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)N * np * nu) return;
+    const int part = threadIdx.x % LANES;
+    const long long last = (long long)N * np * nu - 1;
+    long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const bool live = idx <= last;
+    if (LANES == 1 && !live) return;
+    idx = live ? idx : last;                       // whole warps take part in the sums
     const int m = (int)(idx % N);
     const long long rr = idx / N;
     const int ui = (int)(rr % nu), pl = (int)(rr / nu);
@@ -100,24 +108,26 @@ __global__ void __launch_bounds__(128, 6) pp_num_level_kernel(const double* __re
         }
         const double area = G.area;
         const double* wsh = sh + 3 * nn;
-        for (int sub = 0; sub < n_sub; sub++) {
-            for (int l = 0; l < n_sing; l++) {
-                const double* b = sh + 3 * (sub * stride + l);
-                double y[3];
+        int sub = 0, l = part;
+        for (int q = part; q < nn; q += LANES, l += LANES) {
+            for (; l >= n_sing; l -= n_sing) sub++;
+            const double* b = sh + 3 * (sub * stride + l);
+            double y[3];
 #pragma unroll
-                for (int c = 0; c < 3; c++) y[c] = b[0] * V[0][c] + b[1] * V[1][c] + b[2] * V[2][c] - x[c];
-                const double r = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
-                double K[6];
-                lame_kernel(K, y, r, tau, velP, velS);
-                const double wt = wsh[l] * area;
+            for (int c = 0; c < 3; c++) y[c] = b[0] * V[0][c] + b[1] * V[1][c] + b[2] * V[2][c] - x[c];
+            const double r = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
+            double K[6];
+            lame_kernel(K, y, r, tau, velP, velS);
+            const double wt = wsh[l] * area;
 #pragma unroll
-                for (int e = 0; e < 6; e++) S[e] += wt * K[e];
-            }
+            for (int e = 0; e < 6; e++) S[e] += wt * K[e];
         }
     }
     double* dst = Mbuf + (((size_t)pl * nu + ui) * N + m) * 6;
 #pragma unroll
     for (int e = 0; e < 6; e++) {
+        for (int o = LANES / 2; o > 0; o >>= 1) S[e] += __shfl_xor_sync(0xffffffffu, S[e], o);
+        if (LANES > 1 && (part != e || !live)) continue;
         double v;
         if (layer) {
             v = S[e] / c4;
@@ -136,8 +146,11 @@ __device__ __forceinline__ void sym_apply(double acc[3], const double* M, const 
 }
 
 // One block per (time q, point pl): the time sum of the variant.  Blocks of
-// 128 threads, or of 1024 when there are too few (time, point) pairs to
-// fill the GPU (one point at its 40 times: 40 blocks).
+// 128 threads, a triangle each, or (FLAT) of 1024 over (instant, triangle) when
+// there are too few (time, point) pairs to fill the GPU (one point at its 40
+// times: 40 blocks; walking the instants one after the other, on the latency of
+// their loads, took 24.7 us on 320 triangles, now 19.6).
+template <bool FLAT>
 __global__ void __launch_bounds__(1024) pp_num_sum_kernel(const double* __restrict__ Mbuf, int N, int p0, int np,
                                                          int nu, const int* __restrict__ tab, int kmax,
                                                          const int* __restrict__ nhat, int npts,
@@ -148,31 +161,39 @@ __global__ void __launch_bounds__(1024) pp_num_sum_kernel(const double* __restri
     const int* tq = tab + (size_t)q * kmax;
     const size_t n3 = 3 * (size_t)N;
     double acc[3] = {0, 0, 0};
-    for (int m = threadIdx.x; m < N; m += blockDim.x) {
-        for (int k = 0; k <= nh; k++) {
-            const double* Mk = Mbuf + (((size_t)pl * nu + tq[k]) * N + m) * 6;
-            const double* pk = phi + (size_t)k * n3 + 3 * (size_t)m;
-            if (layer) {
-                double d[3] = {pk[0], pk[1], pk[2]};
-                if (k > 0) {
-                    const double* pm = pk - n3;
-                    d[0] -= pm[0]; d[1] -= pm[1]; d[2] -= pm[2];
-                }
-                sym_apply(acc, Mk, d);
-            } else {
-                double D[6];
-                if (k < nh) {
-                    const double* Mn = Mbuf + (((size_t)pl * nu + tq[k + 1]) * N + m) * 6;
-#pragma unroll
-                    for (int e = 0; e < 6; e++) D[e] = Mk[e] - Mn[e];
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 6; e++) D[e] = Mk[e];
-                }
-                const double d[3] = {pk[0], pk[1], pk[2]};
-                sym_apply(acc, D, d);
+    auto add = [&](int k, int m) {
+        const double* Mk = Mbuf + (((size_t)pl * nu + tq[k]) * N + m) * 6;
+        const double* pk = phi + (size_t)k * n3 + 3 * (size_t)m;
+        if (layer) {
+            double d[3] = {pk[0], pk[1], pk[2]};
+            if (k > 0) {
+                const double* pm = pk - n3;
+                d[0] -= pm[0]; d[1] -= pm[1]; d[2] -= pm[2];
             }
+            sym_apply(acc, Mk, d);
+        } else {
+            double D[6];
+            if (k < nh) {
+                const double* Mn = Mbuf + (((size_t)pl * nu + tq[k + 1]) * N + m) * 6;
+#pragma unroll
+                for (int e = 0; e < 6; e++) D[e] = Mk[e] - Mn[e];
+            } else {
+#pragma unroll
+                for (int e = 0; e < 6; e++) D[e] = Mk[e];
+            }
+            const double d[3] = {pk[0], pk[1], pk[2]};
+            sym_apply(acc, D, d);
         }
+    };
+    if (FLAT) {
+        const long long total = (long long)N * (nh + 1);
+        for (long long t = threadIdx.x; t < total; t += blockDim.x) {
+            const int k = total <= 0x7fffffff ? (int)t / N : (int)(t / N);
+            add(k, (int)(t - (long long)k * N));
+        }
+    } else {
+        for (int m = threadIdx.x; m < N; m += blockDim.x)
+            for (int k = 0; k <= nh; k++) add(k, m);
     }
     __shared__ double red[3][32];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -261,11 +282,17 @@ int launch_pp_num(const MeshData& m, const PhysParams& P, int n_sub, int n_sing,
     for (int p0 = 0; p0 < npts && e == cudaSuccess; p0 += chunk) {
         const int np = std::min(chunk, npts - p0);
         const long long lv = (long long)m.nt * np * nu;
-        pp_num_level_kernel<<<(unsigned)((lv + 127) / 128), 128, shmem, s>>>(
+        // 8 lanes an item up to about three waves of a thread each: 80 triangles,
+        // 64 points, 40 instants (205 k items) 189 us against 217, 320 triangles
+        // (819 k) 404 against 360
+        const bool split = lv < 2048LL * sms;
+        const auto level = split ? pp_num_level_kernel<8> : pp_num_level_kernel<1>;
+        level<<<(unsigned)(((split ? 8 : 1) * lv + 127) / 128), 128, shmem, s>>>(
             m.d_coords, m.d_tris, m.d_geo, m.nt, d_pts, p0, np, nu, d_taus, d_rule, d_rule + nodes.size(), n_sub,
             n_sing, stride, layer, P.velP, P.velS, 4 * kPi * P.rho, Mbuf);
-        const int sum_threads = ((long long)ntimes * np < 2LL * sms) ? 1024 : 128;
-        pp_num_sum_kernel<<<(unsigned)((long long)ntimes * np), sum_threads, 0, s>>>(Mbuf, m.nt, p0, np, nu, d_tab, kmax,
+        const bool flat = (long long)ntimes * np < 2LL * sms;
+        const auto sum = flat ? pp_num_sum_kernel<true> : pp_num_sum_kernel<false>;
+        sum<<<(unsigned)((long long)ntimes * np), flat ? 1024 : 128, 0, s>>>(Mbuf, m.nt, p0, np, nu, d_tab, kmax,
                                                                              d_nh, npts, d_phi, layer, d_u);
         e = cudaGetLastError();
     }
