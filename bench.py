@@ -31,21 +31,22 @@ sys.path.insert(0, ROOT)
 METRIC = "E_l assembly pair-integrals/s (plain FP64 SA, sphere N=1280, L=40, GH7)"
 UNIT = "pair-integrals/s"
 
-# FP64 operation census of the SA path (oracle compiled with a counting
-# scalar; +,-,*,/,sqrt and each transcendental = 1 flop), on 5000 seeded
+# FP64 operation census of the reference's formulas (oracle compiled with a
+# counting scalar; +,-,*,/,sqrt and each transcendental = 1 flop), on 5000 seeded
 # pairs of this workload: flops per non-null pair-lag when every time level
-# is evaluated once (the schedule the kernel runs), and under the
-# reference's three-instants-per-lag schedule.
+# is evaluated once.
 FLOPS_PER_PAIR_INTEGRAL = 19_232.0
-FLOPS_PER_PAIR_INTEGRAL_REF_SCHEDULE = 53_560.0
 
-# DRAM bytes (read + write) of the dominant kernel, the level pass of the
-# two-pass assembly (sa_level_kernel storing F(t_k) of every pair and level):
-# ncu on the sphere N=320 case (2,478,740 pair-integrals, one launch) measured
-# 11.78 MB read + 105.78 MB written; the writes are the stored levels, which
-# grow with the pair-integrals, so a launch's traffic is scaled by the
-# pair-integrals it processes.
-NCU_LEVEL_PASS_BYTES_N320 = 11.780352e6 + 105.780480e6
+# FP64 operations the level pass executes: ncu's counters on the sphere N=320
+# case (2,478,740 pair-integrals, 2 launches), 2 dfma + dadd + dmul = 6.885e9.  It
+# evaluates closed forms per front, so the census above is not what it does; the
+# roofline takes these.
+EXECUTED_FLOPS_PER_PAIR_INTEGRAL = 6_884_643_120 / 2_478_740
+
+# DRAM bytes (read + write) of the level pass in the same capture: 12.16 MB read
+# + 46.64 MB written.  Its block records stay in L2 for the most part; a launch's
+# traffic is scaled by the pair-integrals it processes.
+NCU_LEVEL_PASS_BYTES_N320 = 12.162560e6 + 46.642688e6
 NCU_LEVEL_PASS_UNITS_N320 = 2_478_740
 
 
@@ -210,7 +211,7 @@ def forms(core, problem, torch, w, dm, L, plain_rate):
                "points": int(len(w.points)), "times": int(len(w.times)),
                "e0_asymmetry": asym,
                "cholesky_vs_lu_density_rel": float((phi_ch - phi64).norm() / phi64.norm()),
-               "scope": "FP32 edge Gauss-Legendre nodes, FP64 closed forms / moments / marching"}
+               "scope": "the FP64 closed form: no quadrature node is left for FP32"}
         del buf64, phi64, phi32, phi_ch
         torch.cuda.empty_cache()
         return res
@@ -483,7 +484,7 @@ def main():
 
     if rank == 0:
         peak = float("nan") if args.no_peak else fp64_peak_tflops(torch)
-        achieved = FLOPS_PER_PAIR_INTEGRAL * (my_pairs / launches) / kernel_s / 1e12
+        achieved = EXECUTED_FLOPS_PER_PAIR_INTEGRAL * (my_pairs / launches) / kernel_s / 1e12
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": t_max / args.steps * 1e3, "higher_is_better": True,
@@ -494,7 +495,8 @@ def main():
                          "frac": achieved / peak,
                          "traffic": NCU_LEVEL_PASS_BYTES_N320 * (my_pairs / launches) / NCU_LEVEL_PASS_UNITS_N320,
                          "peak_source": "measured: cuBLAS DGEMM 8192^3 via torch.matmul float64, best of 5",
-                         "flops_per_unit": FLOPS_PER_PAIR_INTEGRAL,
+                         "flops_per_unit": EXECUTED_FLOPS_PER_PAIR_INTEGRAL,
+                         "reference_formula_flops_per_unit": FLOPS_PER_PAIR_INTEGRAL,
                          "units_per_launch": my_pairs / launches, "launches_per_step": launches,
                          "kernel": KERNEL, "kernel_ms": kernel_s * 1e3,
                          "emission_ms_per_step": emit_ms},

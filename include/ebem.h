@@ -80,8 +80,8 @@ int ebem_workspace_info(int device, unsigned long long* reserved, unsigned long 
 
 /* Device-time profile of the semi-analytic assembly of dense outputs, which
  * runs in two passes (per chunk of field columns: the level kernel that stores
- * F(t_k) of every pair and level, then the emission kernel that writes the
- * blocks).  While enabled, each such call records CUDA events around its
+ * the non-null blocks of every pair, then the emission kernel that writes them
+ * and the zeros in place).  While enabled, each such call records CUDA events around its
  * launches on its stream and waits for them at its end; ebem_profile_read
  * returns the summed milliseconds and launch counts of both passes since the
  * last reset (ms[0], launches[0]: levels; ms[1], launches[1]: emission) and
