@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(128, 4) k_assemble_thread_kernel(KArgs A) {
 // Without `fix` the reference's linear u term (lin_window3) is added over all
 // node pairs in the lags below 3.
 constexpr int kKWarps = 4;
-constexpr size_t kKSmem = 200 * 1024;
+constexpr size_t kKSmem = 200 * 1024;      // as kGHCSmem in ghc.cu
 constexpr int kKNode = 12;               // x, y, z, weight, phik, -, normal, vms
 
 // inner nodes of one chunk; 73 fill kBinChunk at 7 outer nodes, and the 170 of 3
@@ -992,7 +992,7 @@ int launch_k_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_su
         W.K = d_K + (size_t)l0 * A.ld_lag;
         const size_t each = k_warp_bytes(n_gh, W.lag0, W.nlag);
         const int warps = (int)std::max<size_t>(1, std::min<size_t>(kKWarps, kKSmem / each));
-        EBEM_CUDA_TRY(cudaFuncSetAttribute(k_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(warps * each)));
+        EBEM_CUDA_TRY(cudaFuncSetAttribute(k_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKSmem));
         const long long want = (pairs + warps - 1) / warps, cap = (long long)sms * 64;
         k_assemble_kernel<<<(unsigned)(want < cap ? want : cap), 32 * warps, warps * each, s>>>(W);
         EBEM_CUDA_TRY(cudaGetLastError());

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(128, 6) ghc_assemble_thread_kernel(GHCArgs A) 
 // constant does not hold yet.  A warp reduction per lag adds into the pair's
 // sums in shared memory (node pairs beyond kBinChunk in further chunks).
 constexpr int kGHCWarps = 4;
-constexpr size_t kGHCSmem = 200 * 1024;
+constexpr size_t kGHCSmem = 200 * 1024;    // of a block at most; the opt-in of every launch, so that threads' calls do not lower each other's
 
 inline __host__ __device__ int ghc_chunk(int n_in, int n_out) {        // inner nodes of one chunk
     const int q = kBinChunk / n_out;
@@ -413,7 +413,7 @@ int launch_ghc_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_
         int warps = kGHCWarps;
         while (warps > 1 && warps * each > kGHCSmem) warps--;
         const size_t smem = warps * each;
-        e = cudaFuncSetAttribute(ghc_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(ghc_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGHCSmem);
         if (e != cudaSuccess) break;
         const long long want = (NN + warps - 1) / warps, cap = (long long)sms * 64;
         ghc_assemble_kernel<<<(unsigned)(want < cap ? want : cap), 32 * warps, smem, s>>>(A);
