@@ -151,9 +151,7 @@ int band_structure(const MeshData& m, const PhysParams& P, int L, BandOp* op, cu
 }
 
 void band_free(BandOp* op) {
-    if (op->Eb) cudaFree(op->Eb);
-    if (op->off) cudaFree(op->off);
-    if (op->lo) cudaFree(op->lo);
+    store_free({op->Eb, op->off, op->lo});
     op->Eb = nullptr;
     op->off = nullptr;
     op->lo = nullptr;

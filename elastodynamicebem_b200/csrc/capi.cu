@@ -96,6 +96,19 @@ cudaError_t store_malloc(void** p, size_t bytes, cudaStream_t s) {
     return pool_malloc(g_store_pool, kStoreKeep, p, bytes, s);
 }
 
+void store_free(std::initializer_list<void*> buffers) {
+    bool any = false;
+    for (void* p : buffers) any = any || p;
+    if (!any) return;
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+        // a failed context, or a wait that a capture forbids: the buffers may be in use and stay
+        cudaGetLastError();
+        return;
+    }
+    for (void* p : buffers)
+        if (p) cudaFree(p);
+}
+
 cudaError_t ws_free(void* p, cudaStream_t s) { return p ? cudaFreeAsync(p, s) : cudaSuccess; }
 
 PhysParams phys_from(const ebem_problem* p) {
@@ -391,11 +404,10 @@ int ebem_mesh_create(const double* coords, int n_vertices, const int32_t* tris, 
 int ebem_mesh_destroy(ebem_mesh* m) {
     if (!m) return EBEM_OK;
     DeviceGuard dg(m->d.device);
+    for (NodeW* t : m->d.d_node_tables) store_free({t});
     if (m->d.d_coords) cudaFree(m->d.d_coords);
     if (m->d.d_tris) cudaFree(m->d.d_tris);
     if (m->d.d_geo) cudaFree(m->d.d_geo);
-    for (NodeW* t : m->d.d_node_tables)
-        if (t) cudaFree(t);
     for (NodeW* t : m->d.d_comp_tables)
         if (t) cudaFree(t);
     free_direct(m->d);

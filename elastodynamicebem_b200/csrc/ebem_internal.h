@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -39,11 +40,14 @@ constexpr unsigned long long kWorkspaceKeep = 2ull << 30;
 cudaError_t ws_malloc(void** p, size_t bytes, cudaStream_t s);
 cudaError_t ws_free(void* p, cudaStream_t s);
 // Storage that a handle keeps (a banded operator, a mesh's node tables), from
-// a pool of its own: given back with cudaFree (which waits for the device, as
-// a destroyed handle's users do), without the mapping and unmapping of
-// cudaMalloc; up to kStoreKeep bytes of destroyed handles stay reserved.
+// a pool of its own, without the mapping and unmapping of cudaMalloc; up to
+// kStoreKeep bytes of destroyed handles stay reserved.  Kernels of several
+// streams may still read it when the handle is destroyed, and freeing pool
+// memory waits for nothing (cudaFree of a cudaMalloc'ed buffer does): store_free
+// waits for the device, then gives the buffers back.
 constexpr unsigned long long kStoreKeep = 1ull << 30;
 cudaError_t store_malloc(void** p, size_t bytes, cudaStream_t s);
+void store_free(std::initializer_list<void*> buffers);
 template <class T>
 cudaError_t store_malloc(T** p, size_t bytes, cudaStream_t s) {
     return store_malloc(reinterpret_cast<void**>(p), bytes, s);
