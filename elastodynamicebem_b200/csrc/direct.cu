@@ -318,10 +318,10 @@ struct Win3 {
     double R, H, S;
 };
 
-__host__ __device__ __forceinline__ Win3 front_window3(double tX, int l, double dt) {
+__device__ __forceinline__ Win3 front_window3(double tX, int l, double dt) {
     Win3 d = {0.0, 0.0, 0.0};
-    if ((l + 1) * dt - tX <= 0) return d;
-    if (l >= 3 && (l - 2) * dt - tX > 0) {
+    if (level_minus(l + 1, dt, tX) <= 0) return d;
+    if (l >= 3 && level_minus(l - 2, dt, tX) > 0) {
         d.S = dt * dt * dt;
         return d;
     }
@@ -329,7 +329,7 @@ __host__ __device__ __forceinline__ Win3 front_window3(double tX, int l, double 
     for (int w = 0; w < 4; w++) {
         const int k = l - 2 + w;
         if (k < 1) continue;
-        const double t = k * dt, a = t - tX;
+        const double t = k * dt, a = level_minus(k, dt, tX);
         if (a > 0) {
             d.R += c[w] * a;
             d.H += c[w];
@@ -1095,7 +1095,7 @@ __global__ void __launch_bounds__(128, 4) pp_g_kernel(PPArgs A, int kchunk) {
         double Gp[9] = {0}, Gk[9];
         const double c4 = 4 * kPi * A.p.rho;
         for (int k = n_lo - 1; k <= n_hi; k++) {
-            const double tk = t - k * A.dt;
+            const double tk = minus_level(t, k, A.dt);
 #pragma unroll
             for (int e = 0; e < 9; e++) Gk[e] = 0.0;
             if (tk > 0) {
@@ -1174,8 +1174,7 @@ __device__ __forceinline__ unsigned pp_front_bin(double r2, double r, double c, 
     if (fabs(g - rint(g)) <= 1e-9 * (t * idt) + 1e-12) {
         const double tX = sqrt(r2) / c;
         for (k += 3; k >= 0; k--) {
-            const double tk = t - k * dt;
-            if (tk - tX > 0) break;
+            if (minus_level(t, k, dt) - tX > 0) break;
         }
     }
     if (k < 0) return kNoBin;

@@ -52,10 +52,11 @@ struct Win2 {
     double H, Q;
 };
 
-__host__ __device__ __forceinline__ Win2 ghc_window2(double r, double c, int l, double dt) {
+__device__ __forceinline__ Win2 ghc_window2(double r, double c, int l, double dt) {
     Win2 d = {0.0, 0.0};
-    if ((l + 1) * dt - r / c <= 0) return d;
-    if (l >= 1 && (l - 1) * dt - r / c > 0) {
+    const double tX = r / c;
+    if (level_minus(l + 1, dt, tX) <= 0) return d;
+    if (l >= 1 && level_minus(l - 1, dt, tX) > 0) {
         d.Q = 2 * dt * dt;
         return d;
     }
@@ -64,7 +65,7 @@ __host__ __device__ __forceinline__ Win2 ghc_window2(double r, double c, int l, 
         const int k = l - 1 + j;
         if (k < 0) continue;
         const double t = k * dt;
-        if (t - r / c > 0) {
+        if (level_minus(k, dt, tX) > 0) {
             d.H += w[j];
             d.Q += w[j] * ((c * c * t * t - r * r) / (c * c));
         }
