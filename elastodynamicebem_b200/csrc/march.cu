@@ -243,10 +243,13 @@ int launch_rhs(const MeshData& m, const PhysParams& P, int n_gh, int datum, doub
 //   Y_i += alpha sum_k A(:, k) x_i(k),   i < B,
 // A = [E_1 E_2 ...] (rows x K, `cols` columns per lag) and x_i the density in
 // reversed time order from step n0 + i - 1 back (contiguous: x_i = x0 - i
-// cols), of which only steps before n0 count: later ones are zero in the
-// reversed storage when the product runs, and k >= kmax0 + i cols would be
-// before step 0.  Each matrix is read once for B steps instead of once per
-// step.
+// cols), of which only steps 0 .. n0 - 1 count: columns k < i cols are step n0
+// or later (zero in the reversed storage when the product runs), k >= kmax0 + i
+// cols would be before step 0.  Each matrix is read once for B steps instead of
+// once per step.  A product with such a zero adds nothing unless the matrix
+// entry is an infinity or NaN, which must not reach a step before the first of
+// its lag: a block whose sum for a step is not finite takes that sum again over
+// the step's own columns.
 // A block takes 64 rows and a range of columns, its 8 warps every eighth
 // column (two 256-byte runs each, 16 loads in flight per lane), the x_i of 128
 // columns at a time in shared memory; the warps' sums are added in shared
@@ -306,12 +309,28 @@ toeplitz_kernel(const double* __restrict__ A, int rows, long long K, int cols, l
         red[w][lane] = acc[0][i];
         red[w][lane + 32] = acc[1][i];
         __syncthreads();
-        if (threadIdx.x < kToepRows && row0 + (int)threadIdx.x < rows) {
+        const bool out = threadIdx.x < kToepRows && row0 + (int)threadIdx.x < rows;
+        auto total = [&]() {
             double v = 0.0;
 #pragma unroll
             for (int q = 0; q < 8; q++) v += red[q][threadIdx.x];
-            if (v != 0.0) atomicAdd(Y + i * ldy + row0 + threadIdx.x, alpha * v);
+            return v;
+        };
+        double v = out ? total() : 0.0;
+        if (__syncthreads_or(!isfinite(v))) {
+            const long long shift = (long long)i * cols, end = min(k1, kmax0 + shift);
+            double s0 = 0.0, s1 = 0.0;
+            for (long long k = max(k0, shift) + w; k < end; k += 8) {
+                const double x = x0[k - shift];
+                s0 += A[k * rows + r0] * x;
+                s1 += A[k * rows + r1] * x;
+            }
+            red[w][lane] = s0;
+            red[w][lane + 32] = s1;
+            __syncthreads();
+            if (out) v = total();
         }
+        if (out && v != 0.0) atomicAdd(Y + i * ldy + row0 + threadIdx.x, alpha * v);
     }
 }
 
