@@ -229,7 +229,7 @@ int launch_sa_assemble_banded(const MeshData& m, const PhysParams& P, int n_gh, 
                               const long long* d_boff, const int* d_blo, cudaStream_t s);
 // A^{-1} by blocked Gauss-Jordan elimination (inverse.cu), n <= gj_max_n().
 int gj_max_n();
-int gj_inverse(const double* dA, int n, double* d_inv, int* singular, cudaStream_t s);
+int gj_inverse(const double* dA, int n, double* d_inv, int* singular, bool* placed, cudaStream_t s);
 int lu_plan_create(const double* dA, int n, cudaStream_t s, LuPlan* plan, bool pooled = false, bool cholesky = false);
 int lu_plan_solve(LuPlan* plan, double* db, int nrhs, cudaStream_t s);
 void lu_plan_destroy(LuPlan* plan);

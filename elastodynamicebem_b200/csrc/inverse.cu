@@ -188,9 +188,30 @@ __global__ void gj_unscramble_kernel(const double* __restrict__ M, int n, const 
 int gj_max_n() { return kGJThreads * kGJMaxCluster; }
 
 // d_inv = A^{-1} (device, column-major n x n, n <= gj_max_n()); *singular: the
-// number of the first zero pivot, 0 for none.  Waits for the stream.
-int gj_inverse(const double* dA, int n, double* d_inv, int* singular, cudaStream_t s) {
+// number of the first zero pivot, 0 for none.  Waits for the stream.  *placed is
+// false, and nothing has run, when the device cannot hold the panel's cluster
+// (more than 8 blocks are not portable, and a context may be given a part of the
+// SMs).
+int gj_inverse(const double* dA, int n, double* d_inv, int* singular, bool* placed, cudaStream_t s) {
     const size_t nn = (size_t)n * n;
+    const unsigned cluster = (unsigned)((n + kGJThreads - 1) / kGJThreads);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(kGJThreads);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int resident = 0;
+    *placed = (cluster <= 8 || cudaFuncSetAttribute(gj_panel_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+              cudaOccupancyMaxActiveClusters(&resident, gj_panel_kernel, &cfg) == cudaSuccess && resident > 0;
+    if (!*placed) {
+        cudaGetLastError();
+        return EBEM_OK;
+    }
     double* buf = nullptr;
     int* idx = nullptr;
     if (ws_malloc(&buf, (2 * nn + (size_t)n * kGJCols) * sizeof(double), s) != cudaSuccess ||
@@ -203,22 +224,10 @@ int gj_inverse(const double* dA, int n, double* d_inv, int* singular, cudaStream
     int *piv = idx, *used = idx + n, *info = idx + 2 * n;
     cudaError_t e = cudaMemsetAsync(idx, 0xff, 2 * (size_t)n * sizeof(int), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(info, 0x7f, sizeof(int), s);      // 0x7f7f7f7f: none
-    const unsigned cluster = (unsigned)((n + kGJThreads - 1) / kGJThreads);
-    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(gj_panel_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     const dim3 tiles((unsigned)((n + kGJTileR - 1) / kGJTileR), (unsigned)((n + kGJTileC - 1) / kGJTileC));
     const double* cur = dA;
     for (int k0 = 0, t = 0; k0 < n && e == cudaSuccess; k0 += kGJCols, t ^= 1) {
         const int nb = n - k0 < kGJCols ? n - k0 : kGJCols;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cluster;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(cluster);
-        cfg.blockDim = dim3(kGJThreads);
-        cfg.stream = s;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
         e = cudaLaunchKernelEx(&cfg, gj_panel_kernel, cur, n, k0, nb, Pn, piv, used, info);
         if (e != cudaSuccess) break;
         double* nxt = buf + (size_t)t * nn;

@@ -514,8 +514,9 @@ int march_device(const double* dE, int n3, int L, const double* drhs, int nT, do
 // ---------------------------------------------------------------------------
 // A^{-1} of one matrix kept on the device (the E_0 solve of the marching,
 // also for callers that drive the steps themselves): Gauss-Jordan elimination
-// with partial pivoting, past its size LU (getrf) and getrs on the identity,
-// whose n right-hand sides run as matrix-matrix triangular solves.
+// with partial pivoting; past its size, or where the device cannot place its
+// cluster, LU (getrf) and getrs on the identity, whose n right-hand sides run as
+// matrix-matrix triangular solves.
 __global__ void set_identity_kernel(double* __restrict__ a, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[(size_t)i * n + i] = 1.0;
@@ -541,7 +542,6 @@ int lu_plan_create(const double* dA, int n, cudaStream_t s, LuPlan* plan, bool p
     plan->n = n;
     plan->pooled = pooled;
     plan->st = s;
-    if ((rc = solver_handle(s, &h))) return rc;
     cudaError_t e = pooled ? ws_malloc(&plan->inv, nn * sizeof(double), s) : cudaMalloc(&plan->inv, nn * sizeof(double));
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -553,10 +553,12 @@ int lu_plan_create(const double* dA, int n, cudaStream_t s, LuPlan* plan, bool p
         // one cluster, 4096 rows at most.  n = 4096 with one marching step: 17.5 ms
         // against 24.6 ms for the library's LU and triangular solves, which larger
         // matrices take.
-        rc = gj_inverse(dA, n, plan->inv, &hinfo, s);
+        bool placed = false;
+        rc = gj_inverse(dA, n, plan->inv, &hinfo, &placed, s);
         if (!rc && hinfo != 0) rc = fail(EBEM_ERR_SINGULAR, "matrix is singular (zero pivot " + std::to_string(hinfo) + ")");
-        return rc;
+        if (rc || placed) return rc;
     }
+    if ((rc = solver_handle(s, &h))) return rc;
     if (ws_malloc(&lu, nn * sizeof(double), s) != cudaSuccess || ws_malloc(&ipiv, n * sizeof(int), s) != cudaSuccess ||
         ws_malloc(&info, sizeof(int), s) != cudaSuccess) {
         rc = fail(EBEM_ERR_NOMEM, "LU workspace allocation failed");
