@@ -191,7 +191,7 @@ int gj_max_n() { return kGJThreads * kGJMaxCluster; }
 // number of the first zero pivot, 0 for none.  Waits for the stream.  *placed is
 // false, and nothing has run, when the device cannot hold the panel's cluster
 // (more than 8 blocks are not portable, and a context may be given a part of the
-// SMs).
+// SMs) or the two buffers (LU needs one).
 int gj_inverse(const double* dA, int n, double* d_inv, int* singular, bool* placed, cudaStream_t s) {
     const size_t nn = (size_t)n * n;
     const unsigned cluster = (unsigned)((n + kGJThreads - 1) / kGJThreads);
@@ -218,7 +218,8 @@ int gj_inverse(const double* dA, int n, double* d_inv, int* singular, bool* plac
         ws_malloc(&idx, (2 * (size_t)n + 1) * sizeof(int), s) != cudaSuccess) {
         cudaGetLastError();
         ws_free(buf, s);
-        return fail(EBEM_ERR_NOMEM, "inverse workspace allocation failed");
+        *placed = false;
+        return EBEM_OK;
     }
     double* Pn = buf + 2 * nn;
     int *piv = idx, *used = idx + n, *info = idx + 2 * n;

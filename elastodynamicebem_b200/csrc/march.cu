@@ -514,8 +514,8 @@ int march_device(const double* dE, int n3, int L, const double* drhs, int nT, do
 // ---------------------------------------------------------------------------
 // A^{-1} of one matrix kept on the device (the E_0 solve of the marching,
 // also for callers that drive the steps themselves): Gauss-Jordan elimination
-// with partial pivoting; past its size, or where the device cannot place its
-// cluster, LU (getrf) and getrs on the identity, whose n right-hand sides run as
+// with partial pivoting; past its size, or where the device has no room for
+// its cluster or buffers, LU (getrf) and getrs on the identity, whose n right-hand sides run as
 // matrix-matrix triangular solves.
 __global__ void set_identity_kernel(double* __restrict__ a, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -906,16 +906,17 @@ int launch_pp_sa(const MeshData& m, const PhysParams& P, const double* d_phi, co
                 tab[(size_t)q * kmax + k] = (int)(std::lower_bound(uniq.begin(), uniq.end(), taus[c++]) - uniq.begin());
     }
     const size_t per_point = (size_t)nu * m.nt * 6 * sizeof(double);
-    if (per_point > ((size_t)1 << 30) && ntimes > 1) {
-        // times off the grid have their own instants each: in two halves
+    auto by_halves = [&]() {
         const int half = ntimes / 2;
         if (int rc = launch_pp_sa(m, P, d_phi, d_pts, npts, h_times, half, d_u, s)) return rc;
         return launch_pp_sa(m, P, d_phi, d_pts, npts, h_times + half, ntimes - half, d_u + 3 * (size_t)npts * half, s);
-    }
+    };
+    // times off the grid have their own instants each
+    if (per_point > ((size_t)1 << 30) && ntimes > 1) return by_halves();
     // up to 1 GiB of M at a time.  1280 triangles, 256 points, 40 grid times (114
     // distinct instants, 7 MB a point): 1.18 ms; 512 MB 1.35, 192 MB 1.88, 96 MB
     // 2.98 (a chunk of 14 points has fewer warps than the GPU holds).
-    const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)npts, ((size_t)1 << 30) / per_point));
+    int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)npts, ((size_t)1 << 30) / per_point));
     // the tables in one upload: instants, index table, nHat
     HostPack pk;
     const size_t o_taus = pk.add(uniq.data(), nu * sizeof(double));
@@ -923,10 +924,18 @@ int launch_pp_sa(const MeshData& m, const PhysParams& P, const double* d_phi, co
     const size_t o_nh = pk.add(nh.data(), ntimes * sizeof(int));
     unsigned char* d_pack = nullptr;
     double* Mbuf = nullptr;
-    if (pk.upload(&d_pack, s) != cudaSuccess || ws_malloc(&Mbuf, per_point * chunk, s) != cudaSuccess) {
+    if (pk.upload(&d_pack, s) != cudaSuccess) {
         cudaGetLastError();
         ws_free(d_pack, s);
         return fail(EBEM_ERR_NOMEM, "post-processing workspace allocation failed");
+    }
+    while (ws_malloc(&Mbuf, per_point * chunk, s) != cudaSuccess) {
+        // a device with less to spare: fewer points, then fewer times at a time
+        if (chunk == 1) {
+            ws_free(d_pack, s);
+            return ntimes > 1 ? by_halves() : fail(EBEM_ERR_NOMEM, "post-processing workspace allocation failed");
+        }
+        chunk = (chunk + 1) / 2;
     }
     const double* d_taus = reinterpret_cast<const double*>(d_pack + o_taus);
     const int* d_tab = reinterpret_cast<const int*>(d_pack + o_tab);

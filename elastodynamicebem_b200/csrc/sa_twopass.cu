@@ -91,10 +91,13 @@ int launch_sa_twopass(const MeshData& m, const PhysParams& P, int n_gh, int lag0
     const size_t budget = (size_t)128 << 20;
     const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)m.nt, budget / per_col));
     const int chunks = (m.nt + most - 1) / most;
-    const int cols = (m.nt + chunks - 1) / chunks;
+    int cols = (m.nt + chunks - 1) / chunks;
     double* Fb = nullptr;
-    if (ws_malloc(&Fb, per_col * cols, s) != cudaSuccess)
-        return fail(EBEM_ERR_NOMEM, "assembly workspace allocation failed");
+    while (ws_malloc(&Fb, per_col * cols, s) != cudaSuccess) {
+        // a device with less to spare: fewer columns at a time
+        if (cols == 1) return fail(EBEM_ERR_NOMEM, "assembly workspace allocation failed");
+        cols = (cols + 1) / 2;
+    }
     int2* band = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(Fb) + fbytes * cols);
     const bool prof = g_profile.load() != 0;
     std::vector<cudaEvent_t> ev;
