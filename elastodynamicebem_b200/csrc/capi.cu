@@ -854,6 +854,9 @@ static int timemarch_impl(const ebem_mesh* m, const ebem_problem* p, int n_gh, i
     if (!rc) rc = ebem_march(dE, (int)n3, L, dr, p->nt, phi, stream);
     ws_free(dE, s);
     ws_free(dr, s);
+    // the pool gives back what it holds beyond kWorkspaceKeep when the stream is
+    // waited for, and the blocks can be most of the device
+    if (cudaStreamSynchronize(s) != cudaSuccess && rc == EBEM_OK) rc = fail(EBEM_ERR_CUDA, "time marching failed");
     return rc;
 }
 
