@@ -318,22 +318,23 @@ struct Win3 {
     double R, H, S;
 };
 
-__device__ __forceinline__ Win3 front_window3(double tX, int l, double dt) {
+// tl: the four levels, rounded products.
+__device__ __forceinline__ Win3 front_window3(double tX, int l, const double tl[4], double dt) {
     Win3 d = {0.0, 0.0, 0.0};
-    if (level_minus(l + 1, dt, tX) <= 0) return d;
-    if (l >= 3 && level_minus(l - 2, dt, tX) > 0) {
+    if (tl[3] - tX <= 0) return d;
+    if (l >= 3 && tl[0] - tX > 0) {
         d.S = dt * dt * dt;
         return d;
     }
     const double c[4] = {-1.0, 3.0, -3.0, 1.0};
+#pragma unroll
     for (int w = 0; w < 4; w++) {
-        const int k = l - 2 + w;
-        if (k < 1) continue;
-        const double t = k * dt, a = level_minus(k, dt, tX);
+        if (l - 2 + w < 1) continue;
+        const double a = tl[w] - tX;
         if (a > 0) {
             d.R += c[w] * a;
             d.H += c[w];
-            d.S += c[w] * (a * a * (t + 2 * tX) / 6);
+            d.S += c[w] * (a * a * (tl[w] + 2 * tX) / 6);
         }
     }
     return d;
@@ -436,9 +437,9 @@ __global__ void __launch_bounds__(128, 4) k_assemble_thread_kernel(KArgs A) {
         // node pairs provably outside the window's fronts are skipped on r^2:
         // all four levels before the P front, or all after the S front
         const bool lin = !A.fix && l < 3;
-        const double thi = (l + 1) * dt, tlo = (l - 2) * dt;
-        const double skipP2 = lin ? 1e300 : (cP * thi) * (cP * thi) * (1 + 1e-12);
-        const double skipS2 = (l >= 3) ? (cS * tlo) * (cS * tlo) * (1 - 1e-12) : -1.0;
+        const double tl[4] = {level_time(l - 2, dt), level_time(l - 1, dt), level_time(l, dt), level_time(l + 1, dt)};
+        const double skipP2 = lin ? 1e300 : (cP * tl[3]) * (cP * tl[3]) * (1 + 1e-12);
+        const double skipS2 = (l >= 3) ? (cS * tl[0]) * (cS * tl[0]) * (1 - 1e-12) : -1.0;
         double T[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         for (int ee = e0; ee < e1; ee++) {
             const int m = A.vt_tri[ee];
@@ -460,7 +461,7 @@ __global__ void __launch_bounds__(128, 4) k_assemble_thread_kernel(KArgs A) {
                     if (r2 > skipP2 || r2 < skipS2) continue;
                     const double r = sqrt(r2);
                     const double tP = r / cP, tS = r / cS;
-                    const Win3 P = front_window3(tP, l, dt), S = front_window3(tS, l, dt);
+                    const Win3 P = front_window3(tP, l, tl, dt), S = front_window3(tS, l, tl, dt);
                     const double dRPl = A.fix ? P.R : ((r - tP > 0) ? lin_window3(tP, l, dt) : 0.0);
                     const double dHh = S.S - P.S;
                     const double w = (A.wout[o] * X.area) * wi;
@@ -1095,7 +1096,7 @@ __global__ void __launch_bounds__(128, 4) pp_g_kernel(PPArgs A, int kchunk) {
         double Gp[9] = {0}, Gk[9];
         const double c4 = 4 * kPi * A.p.rho;
         for (int k = n_lo - 1; k <= n_hi; k++) {
-            const double tk = minus_level(t, k, A.dt);
+            const double tk = t - level_time(k, A.dt);
 #pragma unroll
             for (int e = 0; e < 9; e++) Gk[e] = 0.0;
             if (tk > 0) {
@@ -1174,7 +1175,7 @@ __device__ __forceinline__ unsigned pp_front_bin(double r2, double r, double c, 
     if (fabs(g - rint(g)) <= 1e-9 * (t * idt) + 1e-12) {
         const double tX = sqrt(r2) / c;
         for (k += 3; k >= 0; k--) {
-            if (minus_level(t, k, dt) - tX > 0) break;
+            if (t - level_time(k, dt) - tX > 0) break;
         }
     }
     if (k < 0) return kNoBin;

@@ -35,11 +35,11 @@ __host__ __device__ inline BinWindow bin_window(int lag0, int nlag) {
     return w;
 }
 
-// k dt - tX and t - k dt as the formulas round them, the product first.  A fused
-// multiply-add would leave the product unrounded and give its rounding error
-// where a front meets a distance exactly at a level: one level early.
-__device__ __forceinline__ double level_minus(int k, double dt, double tX) { return __dsub_rn(__dmul_rn((double)k, dt), tX); }
-__device__ __forceinline__ double minus_level(double t, int k, double dt) { return __dsub_rn(t, __dmul_rn((double)k, dt)); }
+// t_k = k dt, rounded before anything is subtracted from it or it from anything:
+// contracted to a fused multiply-add the difference would be the product's
+// rounding error where a front meets a distance exactly at a level, and the front
+// one level early.
+__device__ __forceinline__ double level_time(int k, double dt) { return __dmul_rn((double)k, dt); }
 
 // Bin of the first level k >= 0 with k dt - r / c > 0, as the reference tests it
 // in IEEE arithmetic (sqrt, quotient, product, difference).  r2 = r^2, icdt =
@@ -54,7 +54,7 @@ __device__ __forceinline__ unsigned front_bin(double r2, double r, double c, dou
     if (fabs(g - rint(g)) <= 1e-9 * g + 1e-12) {
         const double tX = sqrt(r2) / c;
         k = max(k - 3, 0);
-        while (k <= most && !(level_minus(k, dt, tX) > 0)) k++;
+        while (k <= most && !(level_time(k, dt) - tX > 0)) k++;
     }
     return k > most ? kNoBin : k < w.kbase ? 0u : (unsigned)(k - w.kbase + 1);
 }

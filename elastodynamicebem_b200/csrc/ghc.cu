@@ -52,22 +52,22 @@ struct Win2 {
     double H, Q;
 };
 
-__device__ __forceinline__ Win2 ghc_window2(double r, double c, int l, double dt) {
+// t: the three levels, rounded products.
+__device__ __forceinline__ Win2 ghc_window2(double r, double c, int l, const double t[3], double dt) {
     Win2 d = {0.0, 0.0};
     const double tX = r / c;
-    if (level_minus(l + 1, dt, tX) <= 0) return d;
-    if (l >= 1 && level_minus(l - 1, dt, tX) > 0) {
+    if (t[2] - tX <= 0) return d;
+    if (l >= 1 && t[0] - tX > 0) {
         d.Q = 2 * dt * dt;
         return d;
     }
     const double w[3] = {1.0, -2.0, 1.0};
+#pragma unroll
     for (int j = 0; j < 3; j++) {
-        const int k = l - 1 + j;
-        if (k < 0) continue;
-        const double t = k * dt;
-        if (level_minus(k, dt, tX) > 0) {
+        if (l - 1 + j < 0) continue;
+        if (t[j] - tX > 0) {
             d.H += w[j];
-            d.Q += w[j] * ((c * c * t * t - r * r) / (c * c));
+            d.Q += w[j] * ((c * c * t[j] * t[j] - r * r) / (c * c));
         }
     }
     return d;
@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(128, 6) ghc_assemble_thread_kernel(GHCArgs A) 
         }
     }
     for (int l = A.lag0; l <= lhi; l++) {
-        const double thi = (l + 1) * dt, tlo = (l - 1) * dt;
-        const double skipP2 = (cP * thi) * (cP * thi) * (1 + 1e-12);
-        const double skipS2 = (l >= 1) ? (cS * tlo) * (cS * tlo) * (1 - 1e-12) : -1.0;
+        const double tl[3] = {level_time(l - 1, dt), level_time(l, dt), level_time(l + 1, dt)};
+        const double skipP2 = (cP * tl[2]) * (cP * tl[2]) * (1 + 1e-12);
+        const double skipS2 = (l >= 1) ? (cS * tl[0]) * (cS * tl[0]) * (1 - 1e-12) : -1.0;
         if (r2min > skipP2 || r2max < skipS2) continue;
         double K[6] = {0, 0, 0, 0, 0, 0};
         for (int q = 0; q < A.n_sub * A.n_sing; q++) {
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(128, 6) ghc_assemble_thread_kernel(GHCArgs A) 
                 const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
                 if (r2 > skipP2 || r2 < skipS2) continue;
                 const double r = sqrt(r2);
-                const Win2 P = ghc_window2(r, cP, l, dt), S = ghc_window2(r, cS, l, dt);
+                const Win2 P = ghc_window2(r, cP, l, tl, dt), S = ghc_window2(r, cS, l, tl, dt);
                 const double w = (A.wout[o] * aS) * wq;
                 double nu[6];
                 ghc_pair(nu, x, 1 / r, P.H, S.H, P.Q - S.Q, icP2, icS2);
