@@ -647,13 +647,30 @@ __global__ void __launch_bounds__(32 * kKWarps, 3) k_assemble_kernel(KArgs A) {
             const int total = bins_sort(B, n, win.bins, lane);
             double cur[9] = {0}, n1[9] = {0}, n2[9] = {0}, run[9] = {0};
             double last = 0.0, last9 = 0.0;           // this lane's reduced entry and entry 33 of the lag before
-            int first = 0, idle = 0;                  // idle: bins without items up to this one
-            for (int b = 0; b < win.bins; b++) {
+            int first = B.off[0], idle = 0;           // idle: bins without items up to this one
+            for (int i = lane; i < first; i += 32) {  // bin 0: the constant only
+                const unsigned it = B.list[i];
+                const int t = (int)(it & 0x7fffffffu), q = (int)(((float)t + 0.5f) * iout), o = t - q * A.n_gh;
+                const double* d = nodes + kKNode * q;
+                const double y[3] = {xs[4 * o] - d[0], xs[4 * o + 1] - d[1], xs[4 * o + 2] - d[2]}, v[3] = {d[9], d[10], d[11]};
+                const double r2 = y[0] * y[0] + y[1] * y[1] + y[2] * y[2], ir = q_rcp(q_sqrt(r2)), ir2 = ir * ir;
+                const double w = xs[4 * o + 3] * d[3], uC = -cd.c2 * (it >> 31 ? -w : w) * (ir2 * ir), wC = 3 * uC * ir2;
+                const double wx[3] = {v[1] * y[2] - v[2] * y[1], v[2] * y[0] - v[0] * y[2], v[0] * y[1] - v[1] * y[0]};
+                if (r2 > 0)
+#pragma unroll
+                    for (int e = 0; e < 9; e++) {
+                        const int r = e / 3, c = e - 3 * r;
+                        double g = tail * (wC * (wx[r] * y[c]));
+                        if (r != c) g += tail * (uC * ((c - r + 3) % 3 == 1 ? v[(c + 1) % 3] : -v[(r + 1) % 3]));
+                        run[e] += g;
+                    }
+            }
+            for (int b = 1; b < win.bins; b++) {
                 const int k = win.kbase + b - 1, l = k - 1, lastitem = B.off[b], items = lastitem - first;
                 if (items == 0 && first == 0) continue;                 // before the first arrival
                 if (l > lhi) break;
                 idle = items ? 0 : idle + 1;
-                const double early = b == 0 ? 0.0 : 1.0, tk = k * dt;   // bin 0: the constant only
+                const double tk = k * dt;
                 for (int i = first + lane; i < lastitem; i += 32) {
                     const unsigned it = B.list[i];
                     const bool isS = it >> 31;
@@ -665,15 +682,15 @@ __global__ void __launch_bounds__(32 * kKWarps, 3) k_assemble_kernel(KArgs A) {
                     const double w = xs[4 * o + 3] * d[3], sw = isS ? -w : w, wp = w * d[4];
                     const double ic = isS ? cd.icS : cd.icP, ic2 = isS ? cd.icS2 : cd.icP2;
                     const double ir2 = ir * ir, ir3 = ir2 * ir, tX = r * ic;
-                    const double mB = early * ((isS ? -wp : wp) * ir2 * ic), mA = early * ((isS ? -wp : wp) * ir3);
+                    const double mB = (isS ? -wp : wp) * ir2 * ic, mA = (isS ? -wp : wp) * ir3;
                     const double xn = isS ? y[0] * nn[0] + y[1] * nn[1] + y[2] * nn[2] : 0.0;
-                    const double uC = -cd.c2 * sw * ir3, wA = early * (uC * ic2), wC = 3 * uC * ir2;
-                    const double uA = isS || A.fix ? early * (-cd.c1 * sw * ir * ic2) : 0.0;
+                    const double uC = -cd.c2 * sw * ir3, wA = uC * ic2, wC = 3 * uC * ir2;
+                    const double uA = isS || A.fix ? -cd.c1 * sw * ir * ic2 : 0.0;
                     const double a0 = tk - tX, a1 = a0 + dt, a2 = a1 + dt;
                     const double S0 = a0 * a0 * (a0 + 3 * tX) * (1.0 / 6), S1 = a1 * a1 * (a1 + 3 * tX) * (1.0 / 6),
                                  S2 = a2 * a2 * (a2 + 3 * tX) * (1.0 / 6);
                     const double al[3] = {a0, dt - 2 * a0, a0 - dt}, be[3] = {1.0, -2.0, 1.0};
-                    const double ga[3] = {early * (S0 - tail), early * (S1 - 3 * S0 - tail), early * (S2 - 3 * S1 + 3 * S0 - tail)};
+                    const double ga[3] = {S0 - tail, S1 - 3 * S0 - tail, S2 - 3 * S1 + 3 * S0 - tail};
                     const double wx[3] = {v[1] * y[2] - v[2] * y[1], v[2] * y[0] - v[0] * y[2], v[0] * y[1] - v[1] * y[0]};
                     double pM[3], pI[3], pW[3], pU[3];
 #pragma unroll
@@ -707,7 +724,7 @@ __global__ void __launch_bounds__(32 * kKWarps, 3) k_assemble_kernel(KArgs A) {
                             if (r2 > 0) run[e] += g;                    // r = 0: both fronts here at once, no constant remains
                         }
                 }
-                if (b > 0 && l >= A.lag0) {
+                if (l >= A.lag0) {
                     if (idle < 4 || l == A.lag0) {
                         double v[8];
 #pragma unroll
@@ -981,7 +998,13 @@ int launch_k_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_su
     // it 29 ms on the 2800-triangle bar (lags 40..49) against 14 by threads, rule
     // 3/1/3 25 against 34, 7/1/3 30 against 72.  On few pairs the threads do not
     // fill the chip (3/1/1: 448 triangles 1.4 against 2.0 ms, 80: 0.13 against 0.60).
-    const bool byThread = n_gh * n_sub * n_sing < 6 && pairs >= 1024LL * sms;
+    // On windows of few lags, as in ghc.cu: rule 3/1/3, lags from the middle of the
+    // run, 1 and 4 of them 3.8 and 14.5 ms by threads against 12.4 and 16.8 on the
+    // bar (12 lags 41.4 against 26.9), 0.20 and 0.64 against 0.33 and 0.46 on 448
+    // triangles; 7/4/3, 1 lag 29.8 against 33.0 and 1.26 against 0.68.
+    const int np = n_gh * n_sub * n_sing;
+    const bool byThread = (np < 6 && pairs >= 1024LL * sms) ||
+                          (pairs >= 128LL * sms && nlag * (np * (1 + 5.2 * sms / m.nt)) < 47 + 0.73 * np);
     if (byThread) {
         k_assemble_thread_kernel<<<(unsigned)((pairs + 127) / 128), 128, 0, s>>>(A);
         EBEM_CUDA_TRY(cudaGetLastError());

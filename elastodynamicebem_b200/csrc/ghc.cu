@@ -232,6 +232,11 @@ __global__ void __launch_bounds__(32 * kGHCWarps, 4) ghc_assemble_kernel(GHCArgs
         const int j = (int)((p <= 0xffffffffLL) ? (long long)((unsigned)p / (unsigned)A.N) : p / A.N);      // field (inner rule)
         const int i = (int)(p - (long long)j * A.N);                                                    // source (outer rule)
         if (i == j) continue;
+        // before the P front in every lag: nodes lie within 2/3 of the longest side from the centroid
+        const TriGeom &GS = A.geo[i], &GF = A.geo[j];
+        const double e0 = GS.ctr[0] - GF.ctr[0], e1 = GS.ctr[1] - GF.ctr[1], e2 = GS.ctr[2] - GF.ctr[2];
+        const double reach = (lend + 1) * dt * cP + 0.66667 * (GS.maxL + GF.maxL);
+        if (reach * reach * (1 + 1e-9) < e0 * e0 + e1 * e1 + e2 * e2) continue;
         double VS[3][3], VF[3][3];
         for (int v = 0; v < 3; v++)
             for (int c = 0; c < 3; c++) {
@@ -287,13 +292,25 @@ __global__ void __launch_bounds__(32 * kGHCWarps, 4) ghc_assemble_kernel(GHCArgs
             const int total = bins_sort(B, n, win.bins, lane);
             double cur[6] = {0, 0, 0, 0, 0, 0}, nxt[6] = {0, 0, 0, 0, 0, 0}, run[6] = {0, 0, 0, 0, 0, 0};
             double last = 0.0;                        // this lane's reduced entry of the lag before
-            int first = 0, idle = 0;                  // idle: bins without items up to this one
-            for (int b = 0; b < win.bins; b++) {
+            const double tail = 2 * dt2;
+            int first = B.off[0], idle = 0;           // idle: bins without items up to this one
+            for (int t = lane; t < first; t += 32) {  // bin 0: the constant only
+                const unsigned it = B.list[t];
+                const int np = (int)(it & 0x7fffffffu), q = (int)(((float)np + 0.5f) * iout), o = np - q * A.n_out;
+                const double x0 = ys[4 * q] - xs[4 * o], x1 = ys[4 * q + 1] - xs[4 * o + 1], x2 = ys[4 * q + 2] - xs[4 * o + 2];
+                const double r2 = x0 * x0 + x1 * x1 + x2 * x2, ir = q_rcp(q_sqrt(r2)), ir3 = ir * ir * ir;
+                const double w = xs[4 * o + 3] * ys[4 * q + 3], sw = it >> 31 ? -w : w;
+                const double fT = sw * 1.5 * ir3 * ir * ir, dT = -0.5 * sw * ir3;
+                const double xx[6] = {x0 * x0, x0 * x1, x0 * x2, x1 * x1, x1 * x2, x2 * x2};
+                if (r2 > 0)
+#pragma unroll
+                    for (int e = 0; e < 6; e++) run[e] += tail * (fT * xx[e] + ((e == 0 || e == 3 || e == 5) ? dT : 0.0));
+            }
+            for (int b = 1; b < win.bins; b++) {
                 const int k = win.kbase + b - 1, lastitem = B.off[b], items = lastitem - first;
                 if (items == 0 && first == 0) continue;                 // before the first arrival
                 idle = items ? 0 : idle + 1;
-                const double early = b == 0 ? 0.0 : 1.0;                // bin 0: the constant only
-                const double tk2 = (k * dt) * (k * dt), step = (2 * k + 1) * dt2, tail = 2 * dt2;
+                const double tk2 = (k * dt) * (k * dt), step = (2 * k + 1) * dt2;
                 for (int t = first + lane; t < lastitem; t += 32) {
                     const unsigned it = B.list[t];
                     const bool isS = it >> 31;
@@ -305,9 +322,9 @@ __global__ void __launch_bounds__(32 * kGHCWarps, 4) ghc_assemble_kernel(GHCArgs
                     const double Q = tk2 - r2 * ic2;
                     // entries 11, 12, 13, 22, 23, 33 of x x^T times f plus I times d
                     const double fT = sw * 1.5 * ir3 * ir * ir, dT = -0.5 * sw * ir3;
-                    const double fH = early * (sw * ir3 * ic2), dH = isS ? early * (w * ir * ic2) : 0.0;
+                    const double fH = sw * ir3 * ic2, dH = isS ? w * ir * ic2 : 0.0;
                     const double xx[6] = {x0 * x0, x0 * x1, x0 * x2, x1 * x1, x1 * x2, x2 * x2};
-                    const double e1 = early * (Q - tail), e2 = early * (step - Q - tail);
+                    const double e1 = Q - tail, e2 = step - Q - tail;
 #pragma unroll
                     for (int e = 0; e < 6; e++) {
                         const bool diag = e == 0 || e == 3 || e == 5;
@@ -318,7 +335,7 @@ __global__ void __launch_bounds__(32 * kGHCWarps, 4) ghc_assemble_kernel(GHCArgs
                     }
                 }
                 const int l = k - 1;
-                if (b > 0 && l >= A.lag0 && l <= lhi) {
+                if (l >= A.lag0 && l <= lhi) {
                     if (idle < 3 || l == A.lag0) {
                         double v[8];
 #pragma unroll
@@ -401,7 +418,14 @@ int launch_ghc_assemble(const MeshData& m, const PhysParams& P, int n_gh, int n_
     // against 3.5 and 13.7 against 9.6).  Below 48 pairs an SM and node pair
     // the threads do not fill the chip (3 node pairs: 80 triangles 0.15 ms
     // against 0.08, 252 triangles 0.28 against 0.42).
-    const bool byThread = np <= 24 && NN >= 48LL * sms * np;
+    // On windows of few lags the threads' time falls with the lags and the sort of
+    // the node pairs stays: 36 node pairs, lags from the middle of the run, 1 and 4
+    // of them 3.2 and 10.4 ms by threads against 12.6 and 16.9 on 2800 triangles
+    // (12 lags 28.5 against 27.0), 0.57 and 1.80 against 1.28 and 1.98 on 1280,
+    // 0.11 and 0.29 against 0.16 and 0.23 on 320; 84 node pairs, 1 lag 6.3 against
+    // 14.6, 1.10 against 1.46 and 0.19 against 0.18.
+    const bool byThread = (np <= 24 && NN >= 48LL * sms * np) ||
+                          (NN >= 256LL * sms && nlag * (np * (1 + 3.0 * sms / m.nt) - 20) < 190);
     if (byThread) {
         ghc_assemble_thread_kernel<<<(unsigned)((NN + 127) / 128), 128, 0, s>>>(A);
         e = cudaGetLastError();
