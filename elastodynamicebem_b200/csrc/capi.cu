@@ -81,6 +81,16 @@ cudaError_t pool_malloc(cudaMemPool_t* pools, unsigned long long keep, void** p,
     cudaMemPool_t pool = nullptr;
     if (e == cudaSuccess) e = device_pool(pools, dev, keep, &pool);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, s);
+    if (e == cudaErrorMemoryAllocation) {
+        // a pool does not reach what the other one holds for later calls
+        cudaGetLastError();
+        {
+            std::lock_guard<std::mutex> lock(g_pool_mu);
+            for (cudaMemPool_t other : {g_pool[dev], g_store_pool[dev]})
+                if (other && other != pool) cudaMemPoolTrimTo(other, 0);
+        }
+        e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, s);
+    }
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
