@@ -752,7 +752,13 @@ __global__ void __launch_bounds__(32 * kPPWarps, 4) pp_front_kernel(const TriGeo
         if (__ballot_sync(0xffffffffu, first < nu) == 0u) continue;
         FrontLane L;
         group_geometry(L, g < gn, &x, F, lane);
-        const unsigned circ = group_fields(S.W, L, lane);
+        const unsigned circ = group_fields(S.W, L, lane), split = __ballot_sync(0xffffffffu, L.split);
+        auto add_split = [&](double T[7], int gg, bool cP, bool cS, double rP, double rS, double t2) {
+            for (unsigned m = (split >> (3 * gg)) & 7u; m; m &= m - 1) {
+                const int slot = 3 * gg + __ffs(m) - 1;
+                if ((cP || rP > S.near[slot]) && !(cS || rS > S.near[slot])) group_foot(T, S.W, slot, t2);
+            }
+        };
         if (L.child) {
             S.near[lane] = L.live ? L.near : INFINITY;
             if (c == 0) {
@@ -780,6 +786,7 @@ __global__ void __launch_bounds__(32 * kPPWarps, 4) pp_front_kernel(const TriGeo
                     if (!ask) {
                         double T[7] = {0, 0, 0, 0, 0, 0, 0};
                         group_node(T, S.W, gg, cP, cS, (circ >> (3 * gg)) & 1u, rP, rS, tau * tau, k1, ks);
+                        if (cP && !cS) add_split(T, gg, cP, cS, rP, rS, tau * tau);
                         pp_store(Mbuf + (((size_t)pl * nu + ui) * N + j0 + gg) * 6, T, S.C[gg], ic4);
                     }
                 }
@@ -801,11 +808,13 @@ __global__ void __launch_bounds__(32 * kPPWarps, 4) pp_front_kernel(const TriGeo
                         }
                         double T[7] = {0, 0, 0, 0, 0, 0, 0};
                         group_node(T, S.W, cell.x, cP, cS, (circ >> (3 * cell.x)) & 1u, rP, rS, tau * tau, k1, ks);
+                        add_split(T, cell.x, cP, cS, rP, rS, tau * tau);
                         while (m) {
                             const int k = __ffs(m) - 1;
                             m &= m - 1;
                             const bool isP = k < 3;
-                            group_item(T, S.W, 3 * cell.x + (isP ? k : k - 3), isP, isP ? rP : rS, isP ? k1 : ks);
+                            const int slot = 3 * cell.x + (isP ? k : k - 3);
+                            group_item(T, S.W, slot, !((split >> slot) & 1u), isP, isP ? rP : rS, isP ? k1 : ks);
                         }
                         pp_store(Mbuf + (((size_t)pl * nu + cell.y) * N + j0 + cell.x) * 6, T, S.C[cell.x], ic4);
                     }

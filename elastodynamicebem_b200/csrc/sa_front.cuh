@@ -48,6 +48,10 @@
 // as x grows, which cancel between two ends on one side of the foot; they
 // are therefore kept as tails (integrals from |x| to infinity, Psi for J,
 // chi, K), and the constants enter only when the piece contains the foot.
+// They come with the weight t^2 in both fronts and opposite signs, t^2 / F on
+// children as thin as the outer rule's nodes lie to the sides; there they are
+// left out where the S front has passed the foot too (front_foot).  With them the
+// blocks were off by up to 12 times the rounding of what is left.
 //
 // The reference's thresholds are kept: a front crosses a side when rho^2 -
 // F^2 > 1e-6 (childTriangle.m:62, 75), |2 area| < 1e-6 skips a child, zeta <
@@ -134,8 +138,9 @@ EBEM_DI void front_end(double e[FC_NE], double F, double z, double iz, double r0
 // No branches: the piece runs from the lower end (the front's crossing or V2)
 // to the upper one (the crossing or V1), and the functions of the crossing
 // and of both vertices are always formed, the unused ones with weight 0.
+// foot: with the constants t^2 front_foot of a piece that contains the foot.
 template <class View>
-EBEM_DI void front_item(double H[7], const View& C, double r, bool isP) {
+EBEM_DI void front_item(double H[7], const View& C, double r, bool isP, bool foot = true) {
     const double F = C(FC_F), z = C(FC_Z), r02 = C(FC_R02), x1 = C(FC_X1), x2 = C(FC_X2), ir0 = C(FC_IR0);
     const double z2 = z * z, r2 = r * r, rp = r2 + z2, rm = r2 - z2;
     const double xr = q_sqrt(r2 - r02), rho = q_sqrt(rm);
@@ -171,11 +176,13 @@ EBEM_DI void front_item(double H[7], const View& C, double r, bool isP) {
     double ss = B - FL - hChi + xD, zz = hChi - rm * hPsi, S = FL + rm * hPsi;
     // twice the constants of the odd parts when the piece contains the foot
     const double in = ((mhi || x1 >= 0) && (mlo || x2 < 0)) ? 1.0 : 0.0;
-    const double J2 = in * C(FC_J2), y2 = in * 2 * r2 * (ir0 * ir0), b0 = rp * J2 - in * 2 * kPi * r;
+    const double tt = foot ? r2 : 0.0;
+    const double J2 = in * C(FC_J2), Jm = (tt - z2) * J2, y2 = in * 2 * tt * (ir0 * ir0), Fy = F * y2;
+    const double b0 = (tt + z2) * J2 - in * 2 * kPi * r;
     B += b0;
-    ss += b0 + F * y2;
-    zz += rm * J2 - F * y2;
-    H[0] = isP ? B : S - rm * J2;
+    ss += b0 + Fy;
+    zz += Jm - Fy;
+    H[0] = isP ? B : S - Jm;
     H[1] = B - xD;
     H[2] = hsc;
     H[3] = ss;
@@ -186,8 +193,9 @@ EBEM_DI void front_item(double H[7], const View& C, double r, bool isP) {
 
 // Whole side of one child: G = a + r^2 b of the same seven functions without
 // the V(rho) x (angle) terms (the scalar's b enters as +b for P, -b for S).
+// foot as in front_item.
 template <class View>
-EBEM_DI void front_full(double a[7], double b[7], const View& C) {
+EBEM_DI void front_full(double a[7], double b[7], const View& C, bool foot = true) {
     const double F = C(FC_F), z = C(FC_Z), x1 = C(FC_X1), x2 = C(FC_X2), z2 = z * z;
     double L = 0, J = 0, X1 = 0, XI = 0, CH = 0, sca = 0, scb = 0, ca = 0, cb = 0, sa = 0, sb = 0;
 #pragma unroll
@@ -207,20 +215,40 @@ EBEM_DI void front_full(double a[7], double b[7], const View& C) {
         sa += od * (ax * C(p + FE_IR) * ln);
         sb += od * C(p + FE_K);
     }
+    double JA = J;
     if (x1 >= 0 && x2 < 0) {
-        const double i2 = 2 * C(FC_IR0) * C(FC_IR0);
-        J += C(FC_J2);
-        CH += F * i2;
-        sb -= i2;
+        JA += C(FC_J2);
+        if (foot) {
+            const double i2 = 2 * C(FC_IR0) * C(FC_IR0);
+            J = JA;
+            CH += F * i2;
+            sb -= i2;
+        }
     }
-    const double A1 = F * L + z2 * J;
-    a[0] = A1;           b[0] = J;
-    a[1] = A1 - X1;      b[1] = J - XI;
-    a[2] = -sca;         b[2] = -scb;
-    a[3] = X1 + z2 * J;  b[3] = J + CH + XI;
-    a[4] = -ca;          b[4] = -cb;
-    a[5] = sa - L;       b[5] = -sb;
-    a[6] = -z2 * J;      b[6] = J - CH;
+    const double A1 = F * L + z2 * JA;
+    a[0] = A1;            b[0] = J;
+    a[1] = A1 - X1;       b[1] = J - XI;
+    a[2] = -sca;          b[2] = -scb;
+    a[3] = X1 + z2 * JA;  b[3] = J + CH + XI;
+    a[4] = -ca;           b[4] = -cb;
+    a[5] = sa - L;        b[5] = -sb;
+    a[6] = -z2 * JA;      b[6] = J - CH;
+}
+
+// The constants of a child whose side contains the foot, which a front adds t^2
+// times from where it passes the foot on: +K for P, -K for S, in the plane frame
+// (S, T11, T12, T22, T13, T23, T33) with the node's weight.
+template <class View>
+EBEM_DI void front_foot(double T[7], const View& C, double t2) {
+    const double w = t2 * C(FC_W), ux = C(FC_UX), uy = C(FC_UY), ir0 = C(FC_IR0);
+    const double wJ = w * C(FC_J2), wy = w * (2 * ir0 * ir0), wF = wy * C(FC_F), wz = wy * C(FC_ZS);
+    T[0] += wJ;
+    T[1] -= wJ + uy * uy * wF;
+    T[2] += ux * uy * wF;
+    T[3] -= wJ + ux * ux * wF;
+    T[4] -= uy * wz;
+    T[5] += ux * wz;
+    T[6] -= wJ - wF;
 }
 
 // Angle of the whole child and its moments (1, cc, sc, ss, c, s).
