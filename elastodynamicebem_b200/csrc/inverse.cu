@@ -20,8 +20,8 @@
 // blocks (of it, per ncu, block and cluster barriers and the release of the
 // remote stores about 40 %); 64 columns move A half as often as 32 (n = 2100:
 // 4.6 against 4.7 ms).  Against the library's LU and n triangular solves (one
-// marching step each): n = 258 0.90 -> 0.53 ms, 858 3.1 -> 1.6, 1440 5.2 -> 2.8,
-// 2100 9.3 -> 4.8, 3840 22.9 -> 15.5.
+// marching step each): n = 258 0.90 -> 0.52 ms, 858 3.1 -> 1.5, 1440 5.2 -> 2.7,
+// 2100 9.3 -> 4.7, 3840 22.9 -> 15.3.
 #include "ebem_internal.h"
 #include "sa_math.cuh"
 
@@ -131,17 +131,16 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(const double* __restr
     __shared__ double sr[kGJStep][kGJTileC];
     const int r0 = blockIdx.x * kGJTileR, c0 = blockIdx.y * kGJTileC;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    // The panel's products are summed by themselves and added to A once: its entries
+    // are rounded n / 64 times, not n times (n = 1500, a diagonal of size 1 beside small
+    // entries: solutions 2.0e-15 off -> below 9e-16).  A read after the products,
+    // 16 loads in flight, instead of before them also leaves the block a shorter
+    // start (n = 3840 15.56 -> 15.28 ms; one load at a time 20.4).
     double acc[8][4];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int r = r0 + tx + 16 * i;
-        const bool pivot = r < n && used[r] >= k0;         // of this panel: the row starts from 0
+    for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int c = c0 + ty + 16 * j;
-            acc[i][j] = (r < n && c < n && !pivot) ? A[(size_t)c * n + r] : 0.0;
-        }
-    }
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
     for (int b0 = 0; b0 < nb; b0 += kGJStep) {
         __syncthreads();
         for (int t = threadIdx.x; t < kGJStep * kGJTileR; t += 256) {
@@ -166,14 +165,36 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(const double* __restr
                 for (int j = 0; j < 4; j++) acc[i][j] = fma(x[i], y[j], acc[i][j]);
         }
     }
+    unsigned open = 0;                                 // rows but this panel's pivots, which start from 0
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int c = c0 + ty + 16 * j, b = c - k0;
-        if (c >= n) continue;
+    for (int i = 0; i < 8; i++) {
+        const int r = r0 + tx + 16 * i;
+        if (r < n && used[r] < k0) open |= 1u << i;
+    }
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int r = r0 + tx + 16 * i;
-            if (r < n) B[(size_t)c * n + r] = (b >= 0 && b < nb) ? Pn[(size_t)b * n + r] : acc[i][j];
+    for (int h = 0; h < 4; h += 2) {                   // 16 loads in flight
+        double base[2][8];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int c = c0 + ty + 16 * (h + j), b = c - k0;
+            const bool panel = b >= 0 && b < nb;
+            const double* from = panel ? Pn + (size_t)b * n : A + (size_t)c * n;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int r = r0 + tx + 16 * i;
+                base[j][i] = (c < n && r < n && (panel || (open >> i & 1u))) ? from[r] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int c = c0 + ty + 16 * (h + j), b = c - k0;
+            if (c >= n) continue;
+            const bool panel = b >= 0 && b < nb;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int r = r0 + tx + 16 * i;
+                if (r < n) B[(size_t)c * n + r] = panel ? base[j][i] : base[j][i] + acc[i][h + j];
+            }
         }
     }
 }
