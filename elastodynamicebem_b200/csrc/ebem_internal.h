@@ -285,6 +285,17 @@ constexpr int kHistBlock = 8;
 int launch_hist_block(const double* E1, int rows, int cols, int M, const double* rev, int nT, int n0, double* Y, int sm_count,
                       cudaStream_t s);
 
+// Instants t_q - k dt (k = 0 .. nh[q] = min(ceil(t_q / dt), nT) - 1; none for t_q <= 0)
+// of the post-processings, k dt rounded before the difference as the reference
+// forms them: the distinct ones in ascending order and, per (q, k), the index
+// among them at tab[q kmax + k] (march.cu).
+struct Instants {
+    std::vector<int> nh, tab;
+    std::vector<double> uniq;
+    int kmax = 1;
+};
+void form_instants(const double* times, int ntimes, double dt, int nT, Instants* out);
+
 // ---------------------------------------------------------------------------
 // learned quadrature selector (selector.cu)
 // features of samples[3 q + 0..2] = (source, field, lag)

@@ -879,40 +879,65 @@ __global__ void __launch_bounds__(1024) pp_inst_sum_kernel(const double* __restr
     }
 }
 
+void form_instants(const double* times, int ntimes, double dt, int nT, Instants* out) {
+    Instants& I = *out;
+    I.nh.assign(ntimes, -1);
+    I.kmax = 1;
+    size_t total = 0;
+    for (int q = 0; q < ntimes; q++) {
+        if (times[q] > 0) I.nh[q] = std::min((int)std::ceil(times[q] / dt) - 1, nT - 1);
+        I.kmax = std::max(I.kmax, I.nh[q] + 1);
+        total += I.nh[q] + 1;
+    }
+    auto instant = [&](int q, int k) {
+        volatile double a = (double)k * dt;        // rounded product, then the difference
+        return times[q] - a;
+    };
+    I.tab.assign((size_t)ntimes * I.kmax, 0);
+    // The n-th smallest instants of all times lie within one dt of each other: in
+    // ascending order as they are visited here unless times differ by whole steps
+    // (on the time grid), where the rounding of a step decides the order.
+    std::vector<std::pair<double, int>> runs;      // smallest instant of each time
+    for (int q = 0; q < ntimes; q++)
+        if (I.nh[q] >= 0) runs.emplace_back(instant(q, I.nh[q]), q);
+    std::sort(runs.begin(), runs.end());
+    I.uniq.clear();
+    I.uniq.reserve(total);
+    bool sorted = true;
+    for (int n = 0; n < I.kmax && sorted; n++)
+        for (const auto& r : runs) {
+            const int q = r.second, k = I.nh[q] - n;
+            if (k < 0) continue;
+            const double t = instant(q, k);
+            if (!I.uniq.empty() && !(t >= I.uniq.back())) {
+                sorted = false;
+                break;
+            }
+            if (I.uniq.empty() || t != I.uniq.back()) I.uniq.push_back(t);
+            I.tab[(size_t)q * I.kmax + k] = (int)I.uniq.size() - 1;
+        }
+    if (sorted) return;
+    I.uniq.clear();
+    for (int q = 0; q < ntimes; q++)
+        for (int k = 0; k <= I.nh[q]; k++) I.uniq.push_back(instant(q, k));
+    const std::vector<double> taus(I.uniq);
+    std::sort(I.uniq.begin(), I.uniq.end());
+    I.uniq.erase(std::unique(I.uniq.begin(), I.uniq.end()), I.uniq.end());
+    size_t c = 0;
+    for (int q = 0; q < ntimes; q++)
+        for (int k = 0; k <= I.nh[q]; k++)
+            I.tab[(size_t)q * I.kmax + k] = (int)(std::lower_bound(I.uniq.begin(), I.uniq.end(), taus[c++]) - I.uniq.begin());
+}
+
 int launch_pp_sa(const MeshData& m, const PhysParams& P, const double* d_phi, const double* d_pts, int npts,
                        const double* h_times, int ntimes, double* d_u, cudaStream_t s) {
-    std::vector<int> nh(ntimes);
-    int kmax = 1;
-    std::vector<double> taus;
-    for (int q = 0; q < ntimes; q++) {
-        const double t = h_times[q];
-        int n = -1;
-        if (t > 0) {
-            n = (int)std::ceil(t / P.dt) - 1;
-            if (n > P.nT - 1) n = P.nT - 1;
-        }
-        nh[q] = n;
-        kmax = std::max(kmax, n + 1);
-        for (int k = 0; k <= n; k++) {
-            volatile double a = (double)k * P.dt;      // rounded product, then the difference
-            taus.push_back(t - a);
-        }
-    }
-    std::vector<double> uniq(taus);
-    std::sort(uniq.begin(), uniq.end());
-    uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
-    const int nu = (int)uniq.size();
+    Instants I;
+    form_instants(h_times, ntimes, P.dt, P.nT, &I);
+    const int nu = (int)I.uniq.size(), kmax = I.kmax;
     if (nu == 0) {
         // no instant: u = 0
         EBEM_CUDA_TRY(cudaMemsetAsync(d_u, 0, sizeof(double) * 3 * (size_t)npts * ntimes, s));
         return EBEM_OK;
-    }
-    std::vector<int> tab((size_t)ntimes * kmax, 0);
-    {
-        size_t c = 0;
-        for (int q = 0; q < ntimes; q++)
-            for (int k = 0; k <= nh[q]; k++)
-                tab[(size_t)q * kmax + k] = (int)(std::lower_bound(uniq.begin(), uniq.end(), taus[c++]) - uniq.begin());
     }
     const size_t per_point = (size_t)nu * m.nt * 6 * sizeof(double);
     auto by_halves = [&]() {
@@ -928,9 +953,9 @@ int launch_pp_sa(const MeshData& m, const PhysParams& P, const double* d_phi, co
     int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)npts, ((size_t)1 << 30) / per_point));
     // the tables in one upload: instants, index table, nHat
     HostPack pk;
-    const size_t o_taus = pk.add(uniq.data(), nu * sizeof(double));
-    const size_t o_tab = pk.add(tab.data(), tab.size() * sizeof(int));
-    const size_t o_nh = pk.add(nh.data(), ntimes * sizeof(int));
+    const size_t o_taus = pk.add(I.uniq.data(), nu * sizeof(double));
+    const size_t o_tab = pk.add(I.tab.data(), I.tab.size() * sizeof(int));
+    const size_t o_nh = pk.add(I.nh.data(), ntimes * sizeof(int));
     unsigned char* d_pack = nullptr;
     double* Mbuf = nullptr;
     if (pk.upload(&d_pack, s) != cudaSuccess) {

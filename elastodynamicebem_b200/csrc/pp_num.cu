@@ -221,36 +221,10 @@ int launch_pp_num(const MeshData& m, const PhysParams& P, int n_sub, int n_sing,
         return fail(EBEM_ERR_INVALID, "the reference's point post-processing reads node 3 * subregion + l "
                                       "(kernelSP.cu:41), past the node table for this rule; pass "
                                       "EBEM_FIX_REFERENCE_DEFECTS to read node subregion * n_sing + l");
-    // instants t_q - k dt, formed as the reference forms them, deduplicated
-    std::vector<int> nh(ntimes);
-    int kmax = 1;
-    std::vector<double> taus;
-    for (int q = 0; q < ntimes; q++) {
-        const double t = h_times[q];
-        int n = -1;
-        if (t > 0) {
-            n = (int)std::ceil(t / P.dt) - 1;
-            if (n > P.nT - 1) n = P.nT - 1;
-        }
-        nh[q] = n;
-        kmax = std::max(kmax, n + 1);
-        for (int k = 0; k <= n; k++) {
-            volatile double a = (double)k * P.dt;      // rounded product, then the difference
-            taus.push_back(t - a);
-        }
-    }
-    std::vector<double> uniq(taus);
-    std::sort(uniq.begin(), uniq.end());
-    uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
-    const int nu = std::max(1, (int)uniq.size());
-    if (uniq.empty()) uniq.push_back(0.0);
-    std::vector<int> tab((size_t)ntimes * kmax, 0);
-    {
-        size_t c = 0;
-        for (int q = 0; q < ntimes; q++)
-            for (int k = 0; k <= nh[q]; k++)
-                tab[(size_t)q * kmax + k] = (int)(std::lower_bound(uniq.begin(), uniq.end(), taus[c++]) - uniq.begin());
-    }
+    Instants I;
+    form_instants(h_times, ntimes, P.dt, P.nT, &I);
+    if (I.uniq.empty()) I.uniq.push_back(0.0);
+    const int nu = (int)I.uniq.size(), kmax = I.kmax;
     std::vector<double> nodes((size_t)3 * n_sub * n_sing), w(n_sing);
     if (gh_composite(n_sing, n_sub, nodes.data(), w.data()))
         return fail(EBEM_ERR_INVALID, "inner rule: n_sub in {1,4,16,64}, n_sing in {1,3,7,12,19}");
@@ -258,12 +232,12 @@ int launch_pp_num(const MeshData& m, const PhysParams& P, int n_sub, int n_sing,
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)npts, ((size_t)1 << 30) / per_point));
     // the tables in one upload: instants, rule nodes and weights, index table, nHat
     HostPack pk;
-    const size_t o_taus = pk.add(uniq.data(), nu * sizeof(double));
+    const size_t o_taus = pk.add(I.uniq.data(), nu * sizeof(double));
     std::vector<double> rule(nodes);                        // the nodes, then the weights
     rule.insert(rule.end(), w.begin(), w.end());
     const size_t o_nodes = pk.add(rule.data(), rule.size() * sizeof(double));
-    const size_t o_tab = pk.add(tab.data(), tab.size() * sizeof(int));
-    const size_t o_nh = pk.add(nh.data(), ntimes * sizeof(int));
+    const size_t o_tab = pk.add(I.tab.data(), I.tab.size() * sizeof(int));
+    const size_t o_nh = pk.add(I.nh.data(), ntimes * sizeof(int));
     unsigned char* d_pack = nullptr;
     double* Mbuf = nullptr;
     cudaError_t e = pk.upload(&d_pack, s);
