@@ -37,6 +37,7 @@
 #include "ebem_internal.h"
 
 #include <algorithm>
+#include <cmath>
 
 namespace ebem {
 
@@ -88,9 +89,18 @@ __global__ void __launch_bounds__(128, 6) pp_num_level_kernel(const double* __re
     const bool live = idx <= last;
     if (LANES == 1 && !live) return;
     idx = live ? idx : last;                       // whole warps take part in the sums
-    const int m = (int)(idx % N);
-    const long long rr = idx / N;
-    const int ui = (int)(rr % nu), pl = (int)(rr / nu);
+    int m, ui, pl;
+    if (last <= 0xffffffffLL) {                    // 32-bit quotients: the 64-bit ones take as long as a node
+        const unsigned rr = (unsigned)idx / (unsigned)N;
+        m = (int)((unsigned)idx - rr * (unsigned)N);
+        pl = (int)(rr / (unsigned)nu);
+        ui = (int)(rr - (unsigned)pl * (unsigned)nu);
+    } else {
+        const long long rr = idx / N;
+        m = (int)(idx - rr * N);
+        pl = (int)(rr / nu);
+        ui = (int)(rr - (long long)pl * nu);
+    }
     const int p = p0 + pl;
     const double x[3] = {pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]};
     const double tau = taus[ui];
@@ -256,10 +266,15 @@ int launch_pp_num(const MeshData& m, const PhysParams& P, int n_sub, int n_sing,
     for (int p0 = 0; p0 < npts && e == cudaSuccess; p0 += chunk) {
         const int np = std::min(chunk, npts - p0);
         const long long lv = (long long)m.nt * np * nu;
-        // 8 lanes an item up to about three waves of a thread each: 80 triangles,
-        // 64 points, 40 instants (205 k items) 189 us against 217, 320 triangles
-        // (819 k) 404 against 360
-        const bool split = lv < 2048LL * sms;
+        // 8 lanes an item where a thread each leaves the chip idle, the fewer nodes the
+        // sooner not: every lane finds its item and triangle for itself.  Equal at about
+        // 250 items an SM with 12 nodes, 800 with 28, 1900 with 48 and 5000 with 112, some
+        // 5 nn^1.5 (not tried beyond 5000): sphere of 320 triangles, 4 points at 10 times,
+        // 690 items an SM: 76 us by threads against 89 by lanes, 95 and 91, 118 and 91, 188
+        // and 99.  Where no front has arrived yet lanes only cost (1280 triangles, 1 point
+        // at 40 times, 48 nodes: 105 us against 142; with fronts there 205 against 181).
+        const int nn = n_sub * n_sing;
+        const bool split = lv < (long long)(std::min(5.0 * nn * std::sqrt((double)nn), 5000.0) * sms);
         const auto level = split ? pp_num_level_kernel<8> : pp_num_level_kernel<1>;
         level<<<(unsigned)(((split ? 8 : 1) * lv + 127) / 128), 128, shmem, s>>>(
             m.d_coords, m.d_tris, m.d_geo, m.nt, d_pts, p0, np, nu, d_taus, d_rule, d_rule + nodes.size(), n_sub,
