@@ -360,129 +360,180 @@ __device__ __forceinline__ void mlp_class2(const float* __restrict__ w, const fl
 // for lag l = lag0 + q.  A lag that a front sweeps takes the maximal rule;
 // any other takes the class of the largest probability, or the maximal rule
 // when that probability is below the threshold; 0 outside the pair's
-// non-null lags (nothing to assemble there).  A block walks the lags of 128
-// pairs, one thread each, and queues those that need the network; 256 queued
-// lags are evaluated at a time, two per thread.  (One thread evaluating the
-// lags of its own pair kept its hidden layers in local memory and ran with
-// the lanes whose lag a front sweeps idle: 1024-triangle graded screen, 80
-// lags, 9.8 M lags for the network: 19.2 ms, now 3.5 ms, of which 0.7 ms without
-// the network; the network's multiply-adds alone take 1.4 ms of the FP32 pipes.)  Classes are staged in
-// shared memory (stage bytes, a whole number of lags for all pairs) and
-// written in runs.  Per-class counts of the non-null lags.
+// non-null lags (nothing to assemble there).  Two kernels:
+//
+// sweep_kernel, a thread per pair: every lag but those for the network, whose
+// byte is kAsk; the number of these and of the swept lags per group of 32
+// consecutive pairs in lags.
+// Classes are staged in shared memory (stage_lags per pair) and written in runs.
+//
+// network_kernel, a warp per group that has any: the warp queues the lags marked
+// kAsk and evaluates 64 at a time, two per lane.  The weights (21 KB) are loaded
+// once per resident block, of which 254 registers a thread allow 2 an SM; the
+// features of all pairs with a lag to evaluate in the next 32 are formed together.
+//
+// One kernel for both, 128 pairs a block and the weights loaded by each, had its
+// pairs and lags walked by 8 warps an SM.  Sphere of 1280 triangles, one lag 0.37 ms
+// (a thread per pair with the network in local memory 0.13), now 0.07; 40 lags 1.40
+// (0.67), now 0.32; graded screen of 1024 triangles, 80 lags, 9.8 M lags for the
+// network 3.40 (19.2), now 3.30, of which the network's multiply-adds alone take 1.4
+// of the FP32 pipes.
 static_assert(kOffW1 % 4 == 0 && kOffW2 % 4 == 0 && kOffB1 % 2 == 0 && kOffB2 % 2 == 0 && kOffW3 % 2 == 0 && kH % 8 == 0,
               "weights are read as float4 and float2");
-constexpr int kInferPairs = 128, kInferQueue = 3 * kInferPairs;
-__global__ void __launch_bounds__(kInferPairs) infer_kernel(const float* __restrict__ params, const TriGeom* __restrict__ geo,
-                                                            int N, double velP, double velS, double dt, int lag0, int nlag,
-                                                            int stage_lags, float threshold,
-                                                            unsigned char* __restrict__ cls,
-                                                            unsigned long long* __restrict__ counts) {
-    extern __shared__ unsigned char stage[];       // [stage_lags][kInferPairs]
-    __shared__ __align__(16) float w[kParams];
-    __shared__ unsigned long long cnt[kC];
-    __shared__ int2 queue[kInferQueue];            // (pair of the block, lag offset)
-    __shared__ int queued;
-    __shared__ float pf[kF][kInferPairs];          // the pairs' features, and their d, h_j, r_min, r_max
-    __shared__ double pd[4][kInferPairs];
+constexpr unsigned char kAsk = 0xff;
+constexpr int kSweepPairs = 256, kSweepLags = 96;
+
+__global__ void __launch_bounds__(kSweepPairs) sweep_kernel(const TriGeom* __restrict__ geo, int N, double velP, double velS,
+                                                            double dt, int lag0, int nlag, unsigned char* __restrict__ cls,
+                                                            int2* __restrict__ lags, unsigned long long* __restrict__ counts) {
+    extern __shared__ __align__(16) unsigned char stage[];       // [kSweepPairs][nq]
     const int tid = (int)threadIdx.x;
-    // the hidden layers' weights transposed, the rest where the parameters have them
-    for (int k = tid; k < kParams; k += kInferPairs) {
-        const float v = params[k];
-        if (k < kOffB1) w[(k % kF) * kH + k / kF] = v;
-        else if (k >= kOffW2 && k < kOffB2) w[kOffW2 + ((k - kOffW2) % kH) * kH + (k - kOffW2) / kH] = v;
-        else w[k] = v;
-    }
-    if (tid < kC) cnt[tid] = 0;
-    if (tid == 0) queued = 0;
-    const long long p0 = (long long)blockIdx.x * kInferPairs, p = p0 + tid, NN = (long long)N * N;
-    const int pairs = (int)min((long long)kInferPairs, NN - p0);
-    int llo = -1, lhi = -2;
+    const long long NN = (long long)N * N, p0 = (long long)blockIdx.x * kSweepPairs, p = p0 + tid;
+    const int pairs = (int)min((long long)kSweepPairs, NN - p0);
+    if (blockIdx.x == 0 && tid < kC) counts[tid] = 0;            // for network_kernel
+    int llo = -1, lhi = -2, mine = 0, swept = 0;
     double lo = 0.0, hi = 0.0;                     // the window that a front sweeps (front_sweeps)
     if (p < NN) {
-        const TriGeom &Ti = geo[p % N], &Tj = geo[p / N];
+        const int j = (int)(NN <= 0xffffffffLL ? (long long)((unsigned)p / (unsigned)N) : p / N), i = (int)(p - (long long)j * N);
+        const TriGeom &Ti = geo[i], &Tj = geo[j];
         pair_band(Tj, Ti, velP, velS, dt, lag0, nlag, &llo, &lhi);
         sweep_window(Ti, Tj, lo, hi);
-        PairFeat q;
-        pair_features(q, Ti, Tj, velS, dt);
-#pragma unroll
-        for (int k = 0; k < kF; k++)
-            if (k < 7 || k > 10) pf[k][tid] = q.f[k];
-        pd[0][tid] = q.d;
-        pd[1][tid] = q.hj;
-        pd[2][tid] = q.rmin;
-        pd[3][tid] = q.rmax;
     }
-    unsigned c_loc[kC] = {0, 0, 0, 0};
-    for (int q0 = 0; q0 < nlag; q0 += stage_lags) {
-        const int nq = min(stage_lags, nlag - q0);
+    for (int q0 = 0; q0 < nlag; q0 += kSweepLags) {
+        const int nq = min(kSweepLags, nlag - q0);
         __syncthreads();
-        for (int q = 0; q <= nq; q++) {            // a step past the last lag empties the queue
-            const int l = lag0 + q0 + q;
-            bool ask = false;
-            if (q < nq && p < NN) {
-                int c = 0;
+        if (p < NN)
+            for (int q = 0; q < nq; q++) {
+                const int l = lag0 + q0 + q;
+                unsigned char c = 0;
                 if (llo >= 0 && l >= llo && l <= lhi) {
-                    if (window_swept(lo, hi, l, velP, velS, dt)) {
-                        c = kC - 1;
-                        c_loc[kC - 1]++;
-                    } else {
-                        ask = true;
-                    }
+                    const bool s = window_swept(lo, hi, l, velP, velS, dt);
+                    c = s ? (unsigned char)(kC - 1) : kAsk;
+                    swept += s;
+                    mine += !s;
                 }
-                stage[q * kInferPairs + tid] = (unsigned char)c;
+                stage[tid * nq + q] = c;
             }
-            const unsigned asking = __ballot_sync(0xffffffffu, ask);
-            if (asking) {
-                int at = 0;
-                if ((tid & 31) == 0) at = atomicAdd(&queued, __popc(asking));
-                at = __shfl_sync(0xffffffffu, at, 0) + __popc(asking & ((1u << (tid & 31)) - 1u));
-                if (ask) queue[at] = make_int2(tid, q);
+        __syncthreads();
+        unsigned char* out = cls + p0 * nlag + q0;
+        if (nq == nlag) {
+            // one run of the output, in words where the buffer allows
+            const int bytes = pairs * nq, words = (reinterpret_cast<size_t>(out) & 3) == 0 ? bytes / 4 : 0;
+            for (int k = tid; k < words; k += kSweepPairs)
+                reinterpret_cast<unsigned*>(out)[k] = reinterpret_cast<const unsigned*>(stage)[k];
+            for (int k = 4 * words + tid; k < bytes; k += kSweepPairs) out[k] = stage[k];
+        } else {
+            for (int k = tid; k < pairs * nq; k += kSweepPairs) {
+                const int pr = k / nq, q = k - pr * nq;
+                out[(long long)pr * nlag + q] = stage[k];
             }
-            __syncthreads();
-            int have = queued;
-            __syncthreads();                       // no one queues before everyone has read
-            // at most 255 left over before a step's 128
-            while (have >= 2 * kInferPairs || (q == nq && have > 0)) {
-                const int n = min(have, 2 * kInferPairs);
-                if (tid < n) {
-                    float x[2][kF];
-                    int c[2];
-                    int2 it[2];
-#pragma unroll
-                    for (int t = 0; t < 2; t++) {
-                        it[t] = queue[min(tid + t * kInferPairs, n - 1)];
-                        const int pr = it[t].x;
-#pragma unroll
-                        for (int k = 0; k < kF; k++) x[t][k] = pf[k][pr];
-                        time_features(x[t], pd[0][pr], pd[1][pr], pd[2][pr], pd[3][pr], lag0 + q0 + it[t].y, velP, velS, dt);
-                    }
-                    mlp_class2(w, w + kOffW1, w + kOffW2, x, threshold, c);
-#pragma unroll
-                    for (int t = 0; t < 2; t++) {
-                        if (tid + t * kInferPairs >= n) continue;
-                        stage[it[t].y * kInferPairs + it[t].x] = (unsigned char)c[t];
-#pragma unroll
-                        for (int o = 0; o < kC; o++) c_loc[o] += (c[t] == o);
-                    }
-                }
-                const int2 rest = queue[2 * kInferPairs + tid];
-                __syncthreads();
-                have -= n;
-                if (tid < have) queue[tid] = rest;
-                if (tid == 0) queued = have;
-                __syncthreads();
-            }
-        }
-        for (int k = tid; k < pairs * nq; k += kInferPairs) {
-            const int pr = k / nq, q = k - pr * nq;
-            cls[(p0 + pr) * nlag + q0 + q] = stage[q * kInferPairs + pr];
         }
     }
-#pragma unroll
-    for (int o = 0; o < kC; o++)
-        if (c_loc[o]) atomicAdd(&cnt[o], (unsigned long long)c_loc[o]);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    swept = __reduce_add_sync(0xffffffffu, swept);
+    if ((tid & 31) == 0 && p < NN) lags[p >> 5] = make_int2(mine, swept);
+}
+
+constexpr int kNetWarps = 4, kNetQueue = 96;       // queue: at most 63 left over before a step's 32
+__global__ void __launch_bounds__(32 * kNetWarps) network_kernel(const float* __restrict__ params, const TriGeom* __restrict__ geo,
+                                                                 int N, double velP, double velS, double dt, int lag0,
+                                                                 int nlag, float threshold, const int2* __restrict__ lags,
+                                                                 unsigned char* __restrict__ cls,
+                                                                 unsigned long long* __restrict__ counts) {
+    __shared__ __align__(16) float w[kParams];
+    __shared__ int2 queues[kNetWarps][kNetQueue];  // (pair of the group, lag offset)
+    __shared__ float pfs[kNetWarps][kF][32];       // the pairs' features, and their d, h_j, r_min, r_max
+    __shared__ double pds[kNetWarps][4][32];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    // the hidden layers' weights transposed, the rest where the parameters have them
+    for (int k = threadIdx.x; k < kParams; k += 32 * kNetWarps) {
+        int from = k;
+        if (k < kOffB1) from = (k % kH) * kF + k / kH;
+        else if (k >= kOffW2 && k < kOffB2) from = kOffW2 + ((k - kOffW2) % kH) * kH + (k - kOffW2) / kH;
+        w[k] = params[from];
+    }
     __syncthreads();
-    if (tid < kC && cnt[tid]) atomicAdd(counts + tid, cnt[tid]);
+    int2* queue = queues[wib];
+    float(*pf)[32] = pfs[wib];
+    double(*pd)[32] = pds[wib];
+    const long long NN = (long long)N * N, groups = (NN + 31) / 32, nwarps = (long long)gridDim.x * kNetWarps;
+    unsigned c_loc[kC] = {0, 0, 0, 0};
+    for (long long g = (long long)blockIdx.x * kNetWarps + wib; g < groups; g += nwarps) {
+        const int2 of = lags[g];
+        int left = of.x;
+        c_loc[kC - 1] += lane == 0 ? of.y : 0;
+        if (left == 0) continue;
+        const long long p = 32 * g + lane;
+        unsigned char* mine = cls + p * nlag;
+        bool known = false;
+        int queued = 0;
+        for (int q0 = 0; q0 < nlag && left; q0 += 32) {
+            // the lane's pair: lags of this run that ask
+            unsigned ask = 0;
+            if (p < NN) {
+                const int nq = min(32, nlag - q0);
+#pragma unroll 8
+                for (int e = 0; e < nq; e++) ask |= (mine[q0 + e] == kAsk ? 1u : 0u) << e;
+            }
+            if (ask && !known) {
+                PairFeat f;
+                const TriGeom &Ti = geo[p % N], &Tj = geo[p / N];
+                pair_features(f, Ti, Tj, velS, dt);
+#pragma unroll
+                for (int k = 0; k < kF; k++)
+                    if (k < 7 || k > 10) pf[k][lane] = f.f[k];
+                pd[0][lane] = f.d;
+                pd[1][lane] = f.hj;
+                pd[2][lane] = f.rmin;
+                pd[3][lane] = f.rmax;
+                known = true;
+            }
+            for (unsigned any = __reduce_or_sync(0xffffffffu, ask); any; any &= any - 1) {
+                const int e = __ffs(any) - 1;
+                const unsigned asking = __ballot_sync(0xffffffffu, (ask >> e) & 1u);
+                if ((ask >> e) & 1u) queue[queued + __popc(asking & ((1u << lane) - 1u))] = make_int2(lane, q0 + e);
+                queued += __popc(asking);
+                left -= __popc(asking);
+                __syncwarp();
+                // 64 at a time, and what is left after the group's last
+                while (queued >= 64 || (queued && !left)) {
+                    const int n = min(queued, 64);
+                    if (lane < n) {
+                        float x[2][kF];
+                        int c[2];
+                        int2 it[2];
+#pragma unroll
+                        for (int t = 0; t < 2; t++) {
+                            it[t] = queue[min(lane + 32 * t, n - 1)];
+                            const int pr = it[t].x;
+#pragma unroll
+                            for (int k = 0; k < kF; k++) x[t][k] = pf[k][pr];
+                            time_features(x[t], pd[0][pr], pd[1][pr], pd[2][pr], pd[3][pr], lag0 + it[t].y, velP, velS, dt);
+                        }
+                        mlp_class2(w, w + kOffW1, w + kOffW2, x, threshold, c);
+#pragma unroll
+                        for (int t = 0; t < 2; t++) {
+                            if (lane + 32 * t >= n) continue;
+                            cls[(32 * g + it[t].x) * nlag + it[t].y] = (unsigned char)c[t];
+#pragma unroll
+                            for (int o = 0; o < kC; o++) c_loc[o] += (c[t] == o);
+                        }
+                    }
+                    const int2 rest = queue[64 + lane];
+                    __syncwarp();
+                    queued -= n;
+                    if (lane < queued) queue[lane] = rest;
+                    __syncwarp();
+                }
+            }
+        }
+        __syncwarp();                              // the features of the next group
+    }
+#pragma unroll
+    for (int o = 0; o < kC; o++) {
+        const unsigned v = __reduce_add_sync(0xffffffffu, c_loc[o]);
+        if (lane == 0 && v) atomicAdd(counts + o, (unsigned long long)v);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -586,17 +637,23 @@ int selector_train(float* d_params, const float* d_feats, const int* d_labels, l
 
 int selector_infer(const float* d_params, const MeshData& m, const PhysParams& P, float threshold, int lag0, int nlag,
                    unsigned char* d_cls, long long* h_counts, cudaStream_t s) {
-    unsigned long long* d_cnt = nullptr;
-    if (ws_malloc(&d_cnt, sizeof(unsigned long long) * kC, s) != cudaSuccess)
+    const long long NN = (long long)m.nt * m.nt, groups = (NN + 31) / 32;
+    unsigned long long* d_cnt = nullptr;           // counts per class, then the lags of each group
+    if (ws_malloc(&d_cnt, sizeof(unsigned long long) * kC + sizeof(int2) * groups, s) != cudaSuccess)
         return fail(EBEM_ERR_NOMEM, "inference workspace allocation failed");
     int rc = EBEM_OK;
-    cudaError_t e = cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long) * kC, s);
-    const long long NN = (long long)m.nt * m.nt;
-    if (e == cudaSuccess) {
-        // at most 12 KB of staged classes: with the weights, the queue and the features within the default 48 KB
-        const int stage_lags = std::min(nlag, 96);
-        infer_kernel<<<(unsigned)((NN + kInferPairs - 1) / kInferPairs), kInferPairs, (size_t)stage_lags * kInferPairs, s>>>(
-            d_params, m.d_geo, m.nt, P.velP, P.velS, P.dt, lag0, nlag, stage_lags, threshold, d_cls, d_cnt);
+    int2* d_lags = reinterpret_cast<int2*>(d_cnt + kC);
+    cudaError_t e = cudaSuccess;
+    {
+        // at most 24 KB of staged classes
+        const size_t smem = (size_t)std::min(nlag, kSweepLags) * kSweepPairs;
+        sweep_kernel<<<(unsigned)((NN + kSweepPairs - 1) / kSweepPairs), kSweepPairs, smem, s>>>(
+            m.d_geo, m.nt, P.velP, P.velS, P.dt, lag0, nlag, d_cls, d_lags, d_cnt);
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m.device);
+        const unsigned blocks = (unsigned)std::min<long long>((groups + kNetWarps - 1) / kNetWarps, 2LL * sms);
+        network_kernel<<<blocks, 32 * kNetWarps, 0, s>>>(d_params, m.d_geo, m.nt, P.velP, P.velS, P.dt, lag0, nlag,
+                                                         threshold, d_lags, d_cls, d_cnt);
         e = cudaGetLastError();
     }
     unsigned long long hc[kC] = {0, 0, 0, 0};
