@@ -169,10 +169,10 @@ def cpu_baseline(workload, target_s: float = 12.0, nthreads: int = 0):
 
 
 def forms(core, problem, torch, w, dm, L, plain_rate):
-    """The assembly forms against the plain FP64 assembly: mixed precision on
-    the benchmark workload (speed and error of blocks, density, displacement)
-    and the batched persistent launch on 64 instances of uneven size (against
-    one launch per instance)."""
+    """The assembly forms against the plain FP64 assembly: the mixed mode on the
+    benchmark workload (whose blocks have to be the FP64 ones), the selector, and
+    the batched persistent launch on 64 instances of uneven size (against one
+    launch per instance)."""
     def timed(fn, reps=3):
         fn()
         torch.cuda.synchronize()
@@ -187,32 +187,24 @@ def forms(core, problem, torch, w, dm, L, plain_rate):
     out = {}
 
     def mixed_form(n_gh):
-        # the sphere of 1280 triangles with outer rule n_gh: assembly times,
-        # errors of blocks, density and displacement (256 exterior points x 40
-        # times) of the mixed form against FP64; E_0's asymmetry and the
+        # the sphere of 1280 triangles with outer rule n_gh: assembly time and
+        # whether the mixed mode gives the same blocks; E_0's asymmetry and the
         # density of the Cholesky factorisation of its symmetric part against LU
         buf64 = torch.empty((L, n3, n3), dtype=torch.float64, device="cuda")
-        buf32 = torch.empty_like(buf64)
         t64 = timed(lambda: core.assemble_sa(dm, w.params, n_gh, 0, L, out=buf64))
-        t32 = timed(lambda: core.assemble_sa(dm, w.params, n_gh, 0, L, out=buf32, prec=core.PREC_MIXED))
-        e_rel = float((buf32 - buf64).norm() / buf64.norm())
+        buf32 = torch.empty_like(buf64)
+        core.assemble_sa(dm, w.params, n_gh, 0, L, out=buf32, prec=core.PREC_MIXED)
+        same = bool(torch.equal(buf32, buf64))
         del buf32
         E0 = buf64[0]
         asym = float((E0 - E0.t()).norm() / E0.norm())
         b = core.rhs(dm, w.params, n_gh, w.datum)
         phi_ch = core.march(buf64.transpose(1, 2), b, factor=core.FACTOR_CHOLESKY)
         phi64, _ = core.timemarch_sa(dm, w.params, n_gh, w.datum)
-        phi32, _ = core.timemarch_sa(dm, w.params, n_gh, w.datum, prec=core.PREC_MIXED)
-        u64 = core.pp_sa(dm, w.params, phi64, w.points, w.times)
-        u32 = core.pp_sa(dm, w.params, phi32, w.points, w.times)
-        res = {"assembly_ms": t32, "fp64_assembly_ms": t64, "speedup": t64 / t32, "blocks_rel_err": e_rel,
-               "density_rel_err": float((phi32 - phi64).norm() / phi64.norm()),
-               "displacement_rel_err": float((u32 - u64).norm() / u64.norm()),
-               "points": int(len(w.points)), "times": int(len(w.times)),
-               "e0_asymmetry": asym,
+        res = {"assembly_ms": t64, "blocks_equal_fp64": same, "e0_asymmetry": asym,
                "cholesky_vs_lu_density_rel": float((phi_ch - phi64).norm() / phi64.norm()),
                "scope": "the FP64 closed form: no quadrature node is left for FP32"}
-        del buf64, phi64, phi32, phi_ch
+        del buf64, phi64, phi_ch
         torch.cuda.empty_cache()
         return res
 
@@ -228,19 +220,17 @@ def forms(core, problem, torch, w, dm, L, plain_rate):
     plan = core.BatchPlan(dms, prms, 7, nlag=nlag, prec=core.PREC_FP64)
     t_batch = timed(lambda: plan.assemble(outs))
     t_seq = timed(lambda: [core.assemble_sa(d, p, 7, 0, l, out=o) for d, p, l, o in zip(dms, prms, nlag, outs)])
-    plan32 = core.BatchPlan(dms, prms, 7, nlag=nlag, prec=core.PREC_MIXED)
-    t_b32 = timed(lambda: plan32.assemble(outs))
     info = plan.info()
     out["batched"] = {"instances": len(inst), "N_range": [min(d.N for d in dms), max(d.N for d in dms)],
                       "lags_per_instance": "all (L of each instance)",
                       "output_gb": sum(9 * d.N ** 2 * l * 8 for d, l in zip(dms, nlag)) / 1e9,
                       "pair_integrals": int(sum(counts)),
                       "batch_ms": t_batch, "one_launch_per_instance_ms": t_seq, "speedup": t_seq / t_batch,
-                      "batch_mixed_ms": t_b32, "pair_integrals_per_s": sum(counts) / t_batch * 1e3,
+                      "pair_integrals_per_s": sum(counts) / t_batch * 1e3,
                       "schedule": ("persistent launch over all instances" if info["warps_per_block"]
                                    else "one two-pass assembly per instance"),
                       "tile": {"warps_per_block": info["warps_per_block"], "pairs_per_grab": info["pairs_per_grab"]}}
-    plan.close(); plan32.close()
+    plan.close()
     del outs
     torch.cuda.empty_cache()
     return out
@@ -249,8 +239,8 @@ def forms(core, problem, torch, w, dm, L, plain_rate):
 def selector_form(core, torch, w, dm, L, timed):
     """The learned selector on the benchmark sphere: trained on 200k (pair,
     lag) samples of the configuration 1-4 meshes, then the selected assembly
-    (FP64, and with the mixed form) against the plain assembly on the maximal
-    rule, with the density and displacement errors against the latter."""
+    against the plain assembly on the maximal rule, with the density and
+    displacement errors against the latter."""
     from elastodynamicebem_b200 import selector as S
     t0 = time.perf_counter()
     X, Y = S.training_set(200_000)
@@ -269,17 +259,15 @@ def selector_form(core, torch, w, dm, L, timed):
     cls, counts = core.selector_infer(params, dm, p, S.THRESHOLD, 0, L)
     res = {"rules": [list(r) for r in S.RULES], "train_samples": int(X.shape[0]), "train_s": t_train,
            "final_loss": float(losses[-1]), "lags_per_class": counts, "max_rule_ms": t_max, "inference_ms": t_inf}
-    for name, prec in (("fp64", core.PREC_FP64), ("mixed", core.PREC_MIXED)):
-        t = timed(lambda: core.assemble_sa_selected(dm, p, cls, S.RULES, 0, L, out=buf, prec=prec), reps=1)
-        E, _ = core.assemble_sa_selected(dm, p, cls, S.RULES, 0, L, out=buf, prec=prec)
-        phi = core.march(E, b)
-        u = core.pp_sa(dm, p, phi, w.points, w.times)
-        res[name] = {"assembly_ms": t, "speedup_vs_max_rule": t_max / t,
-                     "density_rel_err": float((phi - phi_max).norm() / phi_max.norm()),
-                     "displacement_rel_err": float((u - u_max).norm() / u_max.norm())}
+    t = timed(lambda: core.assemble_sa_selected(dm, p, cls, S.RULES, 0, L, out=buf), reps=1)
+    E, _ = core.assemble_sa_selected(dm, p, cls, S.RULES, 0, L, out=buf)
+    phi = core.march(E, b)
+    u = core.pp_sa(dm, p, phi, w.points, w.times)
+    res["fp64"] = {"assembly_ms": t, "speedup_vs_max_rule": t_max / t,
+                   "density_rel_err": float((phi - phi_max).norm() / phi_max.norm()),
+                   "displacement_rel_err": float((u - u_max).norm() / u_max.norm())}
     res["scope"] = ("selector classes per (pair, lag) among the rules, lags a wavefront sweeps on the maximal "
-                    "rule; the batched launch takes one rule per plan, so selector + mixed is the combination "
-                    "measured on this mesh")
+                    "rule; the batched launch takes one rule per plan")
     del buf, E, phi_max, cls
     torch.cuda.empty_cache()
     return res
@@ -344,7 +332,7 @@ def main():
     ap.add_argument("--e2e-steps", type=int, default=3)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-peak", action="store_true", help="skip the DGEMM peak measurement")
-    ap.add_argument("--no-forms", action="store_true", help="skip the mixed-precision and batched measurements")
+    ap.add_argument("--no-forms", action="store_true", help="skip the mixed-mode, selector and batched measurements")
     ap.add_argument("--reference-sample-s", type=float, default=8.0,
                     help="seconds of host-core work per step of --impl reference")
     ap.add_argument("--workload", default="sphere1280", choices=["sphere1280", "sphere320"],

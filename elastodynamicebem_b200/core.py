@@ -155,7 +155,7 @@ FACTOR_CHOLESKY = 1
 def march(E: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, stream=None, factor: int = FACTOR_LU):
     """Density phi (nT, 3N) from the blocks E (L, 3N, 3N storage of
     assemble_sa, i.e. E[l] transposed view) and the right-hand side b (nT, 3N);
-    E_0 factored by LU (the reference's) or Cholesky of its symmetric part."""
+    E_0 inverted with partial pivoting (the reference's lu) or by Cholesky of its symmetric part."""
     Eraw = E.transpose(1, 2).contiguous()      # column-major blocks of the C ABI (no copy for assemble_sa's view)
     L, n3 = Eraw.shape[0], Eraw.shape[1]
     nT = b.shape[0]
@@ -214,8 +214,8 @@ class BandedOperator:
 
 
 class DeviceLU:
-    """LU factors of the device matrix A[row, col] (ebem_lu_create), kept on
-    the device; ``solve`` overwrites contiguous device right-hand sides (one
+    """The device matrix A[row, col] prepared for repeated solves
+    (ebem_lu_create: its inverse, kept on the device); ``solve`` overwrites contiguous device right-hand sides (one
     per row of ``b``) with A^{-1} b."""
 
     def __init__(self, A: torch.Tensor, stream=None):

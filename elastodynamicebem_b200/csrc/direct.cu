@@ -17,14 +17,14 @@
 //                    DIR/BEMenerg_dir_timeMarchingD.m:272-296, DIR/BEMenerg_dir_calcBetaVgpu.m,
 //                    DIR/BEMenerg_dir_calcBetaKgpu.m
 //
-// B200 design (not the reference's): one thread per (row triangle, vertex)
-// pair walks the time levels once (level reuse, a 4-level window for the
-// third difference of K, 3 levels for V and P) and visits only the
-// triangles that contain the vertex (an adjacency list; the reference scans
+// B200 design (not the reference's): a warp per (row triangle, vertex) pair of K
+// and per (evaluation, vertex) of the traction part sorts its node pairs by
+// the level of a front's arrival and evaluates each once per front; it visits only
+// the triangles that contain the vertex (an adjacency list; the reference scans
 // all N triangles per block).  Post-processing is contracted with the data
-// in the kernel (each instant evaluated once, no nHat x N matrices), with
-// the reference's matrices available for verification.  The DN system is
-// factorised once (QR), the reference re-solves densely every step.
+// in the kernel (no nHat x N matrices), with the reference's matrices available
+// for verification.  The DN system is factorised once (QR), the reference
+// re-solves densely every step.
 #include "ebem_internal.h"
 
 #include <cublas_v2.h>
@@ -1060,7 +1060,8 @@ int launch_v_diag(const MeshData& m, const PhysParams& P, int n_gh, int n_diag, 
 }
 
 // ---------------------------------------------------------------------------
-// post-processing: one thread per (triangle or vertex, evaluation (t, x))
+// post-processing: the G part a thread per (triangle, evaluation (t, x), chunk of
+// slices), the P part a warp per (vertex, evaluation, chunk of slices)
 
 struct PPArgs {
     const DirTri* tri;
@@ -1102,9 +1103,8 @@ __device__ __forceinline__ void warp_add3(double* dst, double v0, double v1, dou
 // Block (x-tile, evaluation, chunk c) takes the slices n in
 // [c kchunk + 1, (c + 1) kchunk] and evaluates G at the levels n_lo - 1 .. n_hi
 // (one level more than its slices), so that short meshes still fill the GPU.
-// kernelG / kernelP evaluations capped at 128 registers (4 blocks per SM):
-// 16 points x 4 times on the 448-triangle bar 3.51 -> 3.23 ms (80 registers:
-// 3.63 ms, the spills then cost more than the occupancy gains).
+// 128 registers (4 blocks per SM); 16 points x 4 times on the 448-triangle bar,
+// G and P together, 0.46 ms, and 0.44 with 2 or 6 blocks.
 __global__ void __launch_bounds__(128, 4) pp_g_kernel(PPArgs A, int kchunk) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int ev = blockIdx.y;                          // evaluation index q * npts + ip
@@ -1181,7 +1181,9 @@ __global__ void __launch_bounds__(128, 4) pp_g_kernel(PPArgs A, int kchunk) {
 //       S  mu (-6, -6, -6, 30 ir^2) ir^5,          S  minus P's.
 // Evaluating the kernel at every level (thread per vertex) was bound by FP64 latency, most of
 // it at levels past both fronts, where the second difference vanishes: 16 points
-// x 4 times on the 448-triangle bar 2.62 -> 0.17 ms.
+// x 4 times on the 448-triangle bar 2.62 -> 0.17 ms.  Of the 3 blocks an SM that
+// the registers allow, shared memory (76 864 bytes a block, the bins sized for
+// kBinChunk node pairs) admits 2.
 constexpr int kPPWarps = 4, kPPSlices = 64, kPPNodes = 128, kPPNode = 8;
 
 inline __host__ __device__ size_t pp_warp_bytes() {

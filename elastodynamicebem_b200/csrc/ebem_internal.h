@@ -192,10 +192,10 @@ int launch_rhs(const MeshData& m, const PhysParams& P, int n_gh, int datum, doub
 // EBEM_FACTOR_CHOLESKY (of the symmetric part (E_0 + E_0^T) / 2).
 int march_device(const double* dE, int n3, int L, const double* drhs, int nT, double* dphi, cudaStream_t s,
                  int factor = EBEM_FACTOR_LU);
-// A square system solved many times: A^{-1} formed once from the LU factors
-// (partial pivoting), so that each solve is one matrix-vector (or matrix)
-// product instead of a row-interchange pass and two triangular solves, which
-// for one right-hand side are latency-bound.  `pooled` plans (the marching's
+// A square system solved many times: A^{-1} formed once (inverse.cu up to 4096
+// rows, from the LU factors beyond; partial pivoting), so that each solve is one
+// matrix-vector (or matrix) product instead of a row-interchange pass and two
+// triangular solves, which for one right-hand side are latency-bound.  `pooled` plans (the marching's
 // own) keep the inverse in the workspace pool, released on `st`.
 struct LuPlan {
     int n = 0;

@@ -515,8 +515,8 @@ int march_device(const double* dE, int n3, int L, const double* drhs, int nT, do
 // A^{-1} of one matrix kept on the device (the E_0 solve of the marching,
 // also for callers that drive the steps themselves): Gauss-Jordan elimination
 // with partial pivoting; past its size, or where the device has no room for
-// its cluster or buffers, LU (getrf) and getrs on the identity, whose n right-hand sides run as
-// matrix-matrix triangular solves.
+// its cluster or buffers, LU (getrf) and getrs on the identity, whose n
+// right-hand sides run as matrix-matrix triangular solves.
 __global__ void set_identity_kernel(double* __restrict__ a, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[(size_t)i * n + i] = 1.0;

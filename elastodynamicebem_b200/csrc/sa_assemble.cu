@@ -16,9 +16,9 @@
 // (source i, field j) pair.  F(t_k), the combined kernel integral at one
 // instant, depends on k only, so each level is evaluated once and E_l =
 // F_{l+1} - 2 F_l + F_{l-1} is formed from three levels (the reference
-// evaluates every instant three times, once per lag that uses it).  Dense
-// outputs store the levels and write the blocks in a second, coalesced pass
-// (sa_twopass.cu); the other modes write the blocks directly.
+// evaluates every instant three times, once per lag that uses it).  For dense
+// outputs the blocks are kept as records and written in a second, coalesced pass
+// (sa_twopass.cu); the other modes write them directly.
 #include "ebem_internal.h"
 
 #include <algorithm>

@@ -10,9 +10,9 @@
 // correction for 1/x and sqrt(x); log x = e ln 2 + 2 atanh((m - 1)/(m + 1)),
 // x = m 2^e with m in [sqrt(1/2), sqrt 2); arctangent by the half-angle
 // breakpoints tan(pi/8), tan(3 pi/8).  The two series are interpolated at
-// Chebyshev nodes over the reduced range (relative error 1.3e-18 and 1.2e-18
-// before rounding; tests/test_front_cpu.py checks them against the host's
-// long double functions).
+// Chebyshev nodes over the reduced range (relative error 2.3e-18 and 3.1e-18
+// before rounding; tests/test_front_cpu.py and, on the device,
+// tests/test_math_gpu.py check the functions against the host's long double ones).
 #pragma once
 
 #include "sa_device.cuh"

@@ -68,13 +68,14 @@ const char* ebem_last_error(void);
  * library keeps for each device; up to 2 GiB per device stay reserved between
  * calls so that repeated calls neither allocate nor synchronise the device.
  * The storage of banded operators and the node tables of meshes come from a
- * second pool, which keeps up to 1 GiB of what destroyed handles held.
+ * second pool, which keeps up to 1 GiB of what destroyed handles held; a call
+ * whose workspace does not fit gets that memory too.
  * ebem_release_workspace returns every device's reserved workspace memory
  * that no call in flight uses (after the calls in flight have finished). */
 int ebem_release_workspace(void);
 
 /* Bytes the workspace pool of `device` holds reserved and in use (both 0
- * when the library has not used that device).  No counterpart in the
+ * when the library has not used that device; the second pool is not counted).  No counterpart in the
  * reference. */
 int ebem_workspace_info(int device, unsigned long long* reserved, unsigned long long* used);
 
@@ -93,7 +94,7 @@ int ebem_profile_read(double* ms, long long* launches, int reset);
 /* Release everything the library keeps for `device` between calls, before
  * its CUDA context is reset (cudaDeviceReset, or the reset(gpuDevice) that
  * f/BEMenerg_indir/BEMenerg_core/BEMenerg_coreGPU/BEMenerg_coreGPU_timeMarching.m:7,170
- * runs at entry and exit): waits for the device, destroys the workspace pool
+ * runs at entry and exit): waits for the device, destroys both of its pools
  * and the calling thread's cuSOLVER / cuBLAS handles, and forgets the device
  * address of the allocation-free assembly's scratch array.  Handles of other
  * host threads are abandoned (not destroyed) at their next use.  Later calls
@@ -263,8 +264,8 @@ int ebem_batch_destroy(ebem_batch* batch);
  * ebem_assemble_sa_selected assembles every lag of every pair with the rule
  * of its class, rules[2 c], rules[2 c + 1] (host, nclass pairs) for class c
  * (E as ebem_assemble_sa, device, every entry written); counts (host, nclass
- * entries, may be NULL) receives the non-null lags per class.  With every
- * class byte 0 it is the plain assembly with rule (rules[0], rules[1]). */
+ * entries, may be NULL) receives the non-null lags per class.  A class byte of
+ * nclass or more names no rule: its block is zero.  With every class byte 0 it is the plain assembly with rule (rules[0], rules[1]). */
 #define EBEM_SELECTOR_FEATURES 12
 #define EBEM_SELECTOR_CLASSES 4
 #define EBEM_SELECTOR_PARAMS 5252
@@ -301,7 +302,10 @@ int ebem_assemble_sa_ex(const ebem_mesh* mesh, const ebem_problem* prob, int n_g
  * (kernel: .../CUDAkernels/kernelGHC.cu:5; the same kernel is kernelV.cu of
  * f/BEMenerg_dir).  sa_diagonal = 1 also writes the diagonal blocks with the
  * semi-analytic result, as BEMenerg_coreGPU_timeMarching.m:101-131 inserts
- * its CPU semi-analytic diagonal.  E: host or device, 9 N^2 nlag doubles. */
+ * its CPU semi-analytic diagonal.  E: host or device, 9 N^2 nlag doubles.
+ * A lag's values agree between windows (lag0, nlag) to rounding, not bit for bit:
+ * what arrived before the window is summed by itself, and short windows may take
+ * another kernel. */
 int ebem_assemble_ghc(const ebem_mesh* mesh, const ebem_problem* prob, int n_gh, int n_sub, int n_sing, int lag0,
                       int nlag, double* E, int sa_diagonal, void* stream);
 
@@ -318,8 +322,7 @@ int ebem_assemble_ghc(const ebem_mesh* mesh, const ebem_problem* prob, int n_gh,
  * rhs: 3N x nT column-major, host or device. */
 int ebem_rhs(const ebem_mesh* mesh, const ebem_problem* prob, int n_gh, int datum, double* rhs, void* stream);
 
-/* Time marching: LU of E_0 once (and from it E_0^{-1}, as ebem_lu_create
- * does), then phi_n = E_0^{-1}(b_n - sum_{l=1}^{min(n,L-1)} E_l phi_{n-l}).
+/* Time marching: E_0^{-1} once (as ebem_lu_create forms it), then phi_n = E_0^{-1}(b_n - sum_{l=1}^{min(n,L-1)} E_l phi_{n-l}).
  * Replaces the marching loop of
  * f/BEMenerg_indir/BEMenerg_core/BEMenerg_coreGPU/BEMenerg_coreGPU_timeMarching.m:151-169
  * (and of BEMenerg_coreSA_timeMarching.m:46-113).  E: n3 x n3 x L (the
@@ -346,9 +349,10 @@ int ebem_march_ex(const double* E, int n3, int L, const double* rhs, int nT, dou
  * ebem_lu_create: the factorisation of the device matrix A (column-major
  * n x n) for repeated solves; replaces [L, U, P] = lu(sparse(matrix)) of
  * f/BEMenerg_indir/BEMenerg_core/BEMenerg_coreSA/BEMenerg_coreSA_timeMarching.m:46
- * (BEMenerg_coreGPU_timeMarching.m:153).  LU with partial pivoting, from
- * which A^{-1} is formed once and kept on the device (n^2 doubles), so that
- * a solve is one matrix-vector product rather than two triangular solves of
+ * (BEMenerg_coreGPU_timeMarching.m:153).  A^{-1} is formed once, by Gauss-Jordan
+ * elimination with partial pivoting up to n = 4096 and from LU factors beyond (or
+ * where the device has no room for the elimination), and kept on the device (n^2
+ * doubles), so that a solve is one matrix-vector product rather than two triangular solves of
  * one right-hand side.  Returns EBEM_ERR_SINGULAR on a zero pivot.
  * ebem_lu_solve overwrites the device columns b (n x nrhs) with A^{-1} b
  * (U\(L\(P*b)) of :59, equal to rounding: the two differ by about
@@ -376,7 +380,7 @@ int ebem_march_ex(const double* E, int n3, int L, const double* rhs, int nT, dou
  * ebem_banded_info: triangles, L, non-null pair-lags and device bytes held.
  * ebem_banded_to_dense: E_lag0..E_{lag0+nlag-1} in the layout of
  * ebem_assemble_sa (host or device).
- * ebem_banded_march: the marching of ebem_march (LU of E_0 once, history
+ * ebem_banded_march: the marching of ebem_march (E_0^{-1} once, history
  * sum_{l>=1} E_l phi_{n-l} per step) on the banded blocks; rhs and phi
  * 3N x nT, host or device.
  * No counterpart in the reference beyond the dense equivalents cited. */
@@ -466,7 +470,8 @@ int ebem_num_blocks_dir(const ebem_mesh* mesh, const ebem_problem* prob, int* lv
  * BEMenerg_dir_timeMarchingN.m:186-206, clamp |x| <= 1e-14, / 4 pi dt) plus,
  * when n_diag > 0, the same-triangle parts of BEMenerg_dir_calcSubBlockSingK.m
  * (BEMenerg_dir_timeMarchingN.m:208-264).  Lags >= L_K stay zero.
- * accumulate = 0 zeroes the output first. */
+ * accumulate = 0 zeroes the output first.  Windows agree to rounding, as in
+ * ebem_assemble_ghc. */
 int ebem_assemble_k(const ebem_mesh* mesh, const ebem_problem* prob, int n_gh, int n_sub, int n_sing, int n_diag,
                     int lag0, int nlag, int flags, double* K, int accumulate, void* stream);
 
