@@ -38,15 +38,15 @@ UNIT = "pair-integrals/s"
 FLOPS_PER_PAIR_INTEGRAL = 19_232.0
 
 # FP64 operations the level pass executes: ncu's counters on the sphere N=320
-# case (2,478,740 pair-integrals, 2 launches), 2 dfma + dadd + dmul = 6.885e9.  It
+# case (2,478,740 pair-integrals, 2 launches), 2 dfma + dadd + dmul = 6.910e9.  It
 # evaluates closed forms per front, so the census above is not what it does; the
 # roofline takes these.
-EXECUTED_FLOPS_PER_PAIR_INTEGRAL = 6_884_643_120 / 2_478_740
+EXECUTED_FLOPS_PER_PAIR_INTEGRAL = 6_909_741_440 / 2_478_740
 
-# DRAM bytes (read + write) of the level pass in the same capture: 12.16 MB read
-# + 46.64 MB written.  Its block records stay in L2 for the most part; a launch's
+# DRAM bytes (read + write) of the level pass in the same capture: 11.89 MB read
+# + 46.52 MB written.  Its block records stay in L2 for the most part; a launch's
 # traffic is scaled by the pair-integrals it processes.
-NCU_LEVEL_PASS_BYTES_N320 = 12.162560e6 + 46.642688e6
+NCU_LEVEL_PASS_BYTES_N320 = 11.891456e6 + 46.523136e6
 NCU_LEVEL_PASS_UNITS_N320 = 2_478_740
 
 
